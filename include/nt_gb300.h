@@ -122,6 +122,26 @@ int ntg_gemm(void* stream, const float* a, const float* b, float* c, int64_t m, 
              int64_t k, int32_t accumulate);
 /* Per-row sum(x^2)/D -> cov [N] (requirements.py:518-526, 572-582). */
 int ntg_cov_diag(void* stream, const float* x, int64_t n, int64_t d, float* cov);
+/* ntg_gram and, with cov1 (then cov2 too), ntg_cov_diag of both inputs. Without them the
+ * variances are those on nngp's diagonal (x1 == x2). */
+int ntg_flat_input(void* stream, const float* x1, const float* x2, int64_t n1, int64_t n2,
+                   int64_t d, float* nngp, float* cov1, float* cov2, int32_t precision,
+                   void* workspace, size_t workspace_bytes);
+/* A run of layers on flat kernels: each an affine rule (has_affine), then an activation
+ * (kind NTG_ACT_NONE: none). nngp, ntk [N1, N2] (in_t NULL: zero; out_t NULL: not wanted;
+ * outputs distinct from inputs) and the variances of both sides before the run at
+ * var1[i * s1], var2[j * s2], which leave through cov1 [N1], cov2 [N2] (NULL: not wanted).
+ * The same results as one ntg_affine_act per layer and tensor. */
+enum { NTG_FLAT_MAX_LAYERS = 32 };
+typedef struct {
+  int32_t has_affine;
+  ntg_affine_t aff;
+  ntg_act_t act;
+} ntg_flat_layer_t;
+int ntg_flat_rules(void* stream, const float* in_q, const float* in_t, int64_t n1, int64_t n2,
+                   const float* var1, int64_t s1, const float* var2, int64_t s2,
+                   int32_t n_layers, const ntg_flat_layer_t* layers, float* out_q, float* out_t,
+                   float* cov1, float* cov2);
 /* Image inputs x1 [N1, A, C, K], x2 [N2, A, C, K] (NHWC, K channels) ->
  * full-spatial nngp [N1, N2, A, A, C, C] = sum_k x1 x2 / K
  * (requirements.py:542-553). With x2 == x1 and pairs == 0 writes the

@@ -21,6 +21,7 @@ NTG_ACT_SIN, NTG_ACT_RBF, NTG_ACT_GELU = 3, 4, 5
 NTG_PAD_ZERO, NTG_PAD_CIRCULAR = 0, 1
 NTG_TUNE_STENCIL_RING = 0
 CHAIN_MAX_SEG, CHAIN_MAX_LAYERS = 4, 16
+FLAT_MAX_LAYERS = 32
 
 ERRORS = {
     1: 'invalid argument', 2: 'CUDA error', 3: 'unsupported', 4: 'not positive definite',
@@ -36,6 +37,10 @@ class Act(C.Structure):
 class Affine(C.Structure):
     _fields_ = [('w2', C.c_float), ('b2', C.c_float), ('ntk_w2', C.c_float),
                 ('ntk_nn', C.c_float), ('ntk_c', C.c_float), ('nn_scaled', C.c_int32)]
+
+
+class FlatLayer(C.Structure):
+    _fields_ = [('has_affine', C.c_int32), ('aff', Affine), ('act', Act)]
 
 
 class Var(C.Structure):
@@ -63,6 +68,9 @@ SIGNATURES = {
     'ntg_gram_workspace_bytes': ([_I64, _I64, _I64], C.c_size_t),
     'ntg_gemm': ([_P, _P, _P, _P, _I64, _I64, _I64, _I32], C.c_int),
     'ntg_cov_diag': ([_P, _P, _I64, _I64, _P], C.c_int),
+    'ntg_flat_input': ([_P, _P, _P, _I64, _I64, _I64, _P, _P, _P, _I32, _P, C.c_size_t], C.c_int),
+    'ntg_flat_rules': ([_P, _P, _P, _I64, _I64, _P, _I64, _P, _I64, _I32, C.POINTER(FlatLayer),
+                        _P, _P, _P, _P], C.c_int),
     'ntg_input_fs': ([_P, _P, _P, _I64, _I64, _I64, _I64, _I64, _I32, _P], C.c_int),
     'ntg_input_ds': ([_P, _P, _P, _I64, _I64, _I64, _I64, _P], C.c_int),
     'ntg_conv_fs': ([_P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I32, _I32, _I32, _I32,

@@ -75,6 +75,54 @@ def gram(x1: torch.Tensor, x2: torch.Tensor, precision: int = 0) -> torch.Tensor
     return out
 
 
+def flat_input(x1: torch.Tensor, x2: Optional[torch.Tensor], precision: int = 0):
+    """nngp, cov1, cov2 of flat inputs in one call (x2 None: cov1 is nngp's diagonal, so that a
+    self pair has var1 * var2 - nngp^2 == 0 exactly, and cov2 None)."""
+    xb = x1 if x2 is None else x2
+    n1, n2, d = x1.shape[0], xb.shape[0], x1.shape[1]
+    out = torch.empty((n1, n2), device=x1.device, dtype=torch.float32)
+    ws, nbytes = None, 0
+    if precision == 1:
+        nbytes = int(L.load().ntg_gram_workspace_bytes(n1, n2, d))
+        ws = torch.empty((nbytes,), device=x1.device, dtype=torch.uint8)
+    cov1 = cov2 = None
+    if x2 is not None:
+        cov1 = torch.empty((n1,), device=x1.device, dtype=torch.float32)
+        cov2 = torch.empty((n2,), device=x1.device, dtype=torch.float32)
+    L.call('ntg_flat_input', L.stream(), L.ptr(x1), L.ptr(xb), n1, n2, d, L.ptr(out), L.ptr(cov1),
+           L.ptr(cov2), precision, None if ws is None else ws.data_ptr(), nbytes)
+    return out, torch.diagonal(out) if x2 is None else cov1, cov2
+
+
+def _strided(c: torch.Tensor, n: int) -> torch.Tensor:
+    """c as n float32 device values with a positive stride."""
+    if not c.is_cuda or c.dtype != torch.float32 or tuple(c.shape) != (n,):
+        raise ValueError('nt_gb300 kernels take one float32 CUDA variance per sample')
+    return c if c.stride(0) > 0 else c.contiguous()
+
+
+def flat_rules(q, t, c1, c2, layers, want_t: bool):
+    """A run of (affine | None, activation) layers on flat kernels q, t [N1, N2] (t None: zero)
+    and c1 [N1], c2 [N2] or None, which may be strided: (q, t, c1, c2) after it."""
+    n1, n2 = q.shape
+    v1 = _strided(c1, n1)
+    if c2 is None and n2 > n1:
+        raise ValueError('a kernel of two inputs needs the variances of both')
+    v2 = v1 if c2 is None else _strided(c2, n2)
+    dev = q.device
+    out_q = torch.empty((n1, n2), device=dev, dtype=torch.float32)
+    out_t = torch.empty((n1, n2), device=dev, dtype=torch.float32) if want_t else None
+    o1 = torch.empty((n1,), device=dev, dtype=torch.float32)
+    o2 = None if c2 is None else torch.empty((n2,), device=dev, dtype=torch.float32)
+    arr = (L.FlatLayer * len(layers))(*[
+        L.FlatLayer(int(a is not None), IDENTITY_AFFINE if a is None else a, act)
+        for a, act in layers])
+    L.call('ntg_flat_rules', L.stream(), L.ptr(q), L.ptr(t), n1, n2, v1.data_ptr(),
+           max(v1.stride(0), 1), v2.data_ptr(), max(v2.stride(0), 1), len(layers), arr,
+           L.ptr(out_q), L.ptr(out_t), L.ptr(o1), L.ptr(o2))
+    return out_q, out_t, o1, o2
+
+
 def cov_diag(x: torch.Tensor) -> torch.Tensor:
     out = torch.empty((x.shape[0],), device=x.device, dtype=torch.float32)
     L.call('ntg_cov_diag', L.stream(), L.ptr(x), x.shape[0], x.shape[1], L.ptr(out))

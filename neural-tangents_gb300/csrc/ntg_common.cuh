@@ -110,7 +110,7 @@ __device__ __forceinline__ float atan_unit(float t) {
   p = fmaf(p, z, 0.19946566f);
   p = fmaf(p, z, -0.3332986f);
   p = fmaf(p, z, 0.99999934f);
-  return p * t;
+  return __fmul_rn(p, t);
 }
 
 // atan2(y, x) for x >= 0 (angle in [-pi/2, pi/2]); atan2(0, 0) = 0.
@@ -118,7 +118,7 @@ __device__ __forceinline__ float atan2_xpos(float y, float x) {
   const float ay = fabsf(y);
   const float mx = fmaxf(ay, x), mn = fminf(ay, x);
   float th = atan_unit(mn * rcp_approx(mx));
-  th = (ay > x) ? (0.5f * kPi - th) : th;
+  th = (ay > x) ? __fsub_rn(0.5f * kPi, th) : th;
   th = (mx == 0.f) ? 0.f : th;
   return copysignf(th, y);
 }
@@ -198,34 +198,37 @@ __device__ __forceinline__ ActC act_consts(const ntg_act_t& act) {
 }
 
 // Sin / Rbf / Gelu rules. Kernels instantiate act_apply<false> to leave them out:
-// compiled into the fused chain kernel, their library calls slow its ReLU path.
+// compiled into the fused chain kernel, their library calls slow its ReLU path. Each
+// product and sum is rounded as written (no contraction left to the compiler), so that
+// every kernel that inlines a rule gives the same bits.
 __device__ __forceinline__ void act_apply_rare(const ActC& c, float& q, float& t, float v1,
                                             float v2) {
   if (c.kind == NTG_ACT_SIN) {
     // elementwise.py:303-311: s1 = exp(b^2 (q - sum / 2)), s2 = exp(b^2 (-q - sum / 2)) cos 2c
-    const float sum = v1 + v2;
-    const float s1 = expf(c.b2 * fmaf(-0.5f, sum, q));
-    const float s2 = expf(c.b2 * fmaf(-0.5f, sum, -q)) * c.c2;
-    t = t * (c.a2 * c.b2 * (s1 + s2));
-    q = c.a2 * (s1 - s2);
+    const float sum = __fadd_rn(v1, v2);
+    const float s1 = expf(__fmul_rn(c.b2, fmaf(-0.5f, sum, q)));
+    const float e2 = expf(__fmul_rn(c.b2, fmaf(-0.5f, sum, -q)));
+    t = __fmul_rn(t, __fmul_rn(__fmul_rn(c.a2, c.b2), fmaf(e2, c.c2, s1)));
+    q = __fmul_rn(c.a2, fmaf(-e2, c.c2, s1));
   } else if (c.kind == NTG_ACT_RBF) {
     // elementwise.py:380-384: q' = exp(gamma (2 q - sum)), ntk' = ntk 2 gamma q'
-    const float qo = expf(c.a2 * fmaf(2.f, q, -(v1 + v2)));
-    t = t * (2.f * c.a2 * qo);
+    const float qo = expf(__fmul_rn(c.a2, fmaf(2.f, q, -__fadd_rn(v1, v2))));
+    t = __fmul_rn(t, __fmul_rn(__fmul_rn(2.f, c.a2), qo));
     q = qo;
   } else if (c.kind == NTG_ACT_GELU) {
     // elementwise.py:230-250 with prod = v1 v2, prod + 1 = (v1 + 1)(v2 + 1)
-    const float prod = v1 * v2;
-    const float pp1 = (v1 + 1.f) * (v2 + 1.f);
-    const float d2 = pp1 - q * q;
+    const float prod = __fmul_rn(v1, v2);
+    const float pp1 = __fmul_rn(__fadd_rn(v1, 1.f), __fadd_rn(v2, 1.f));
+    const float d2 = fmaf(-q, q, pp1);
     const float dl = sqrtf(fmaxf(d2, 0.f));
     const float ang = atan2_xpos(q, dl);
-    float qo = (q * q + prod * d2) / (pp1 * dl);
-    qo = (qo + q * ang) / (2.f * kPi);
+    float qo = __fdiv_rn(fmaf(prod, d2, __fmul_rn(q, q)), __fmul_rn(pp1, dl));
+    qo = __fdiv_rn(fmaf(q, ang, qo), 2.f * kPi);
     qo = fmaf(0.25f, q, qo);
-    float first = 1.f / d2 + (1.f - prod) / pp1 + 1.f;
-    first *= q / dl / (2.f * kPi);
-    t = t * (first + (0.25f + ang / (2.f * kPi)));
+    float first = __fadd_rn(__fadd_rn(__fdiv_rn(1.f, d2), __fdiv_rn(__fsub_rn(1.f, prod), pp1)),
+                            1.f);
+    first = __fmul_rn(first, __fdiv_rn(__fdiv_rn(q, dl), 2.f * kPi));
+    t = __fmul_rn(t, __fadd_rn(first, __fadd_rn(0.25f, __fdiv_rn(ang, 2.f * kPi))));
     q = qo;
   }
 }

@@ -22,6 +22,7 @@ __device__ __forceinline__ void tri_tile(int64_t t, int64_t& ti, int64_t& tj) {
 // 16-byte words. Bound by FP32 issue: two columns are one packed fma.rn.f32x2 (each lane
 // rounds as fmaf does), and the next 16-deep slice is loaded into registers while the
 // current one is multiplied, so a slice costs one barrier and no exposed load latency.
+// X X^T of [4096, 3072]: 1213 us (scalar fmaf, single buffer: 1383 us).
 // SYM (x1 == x2): the tiles on or below the diagonal only, each off-diagonal one also
 // stored transposed: fmaf(a, b, c) == fmaf(b, a, c), so the mirror is exactly the value
 // the tile (j, i) would hold. VEC: d a multiple of 4 and both inputs 16-byte aligned.
@@ -195,7 +196,8 @@ __device__ __forceinline__ void stage_rows(float* dst, const float* x, int64_t n
 // Small Grams, which a 128-wide tile would leave on a few SMs: T x T output tile per CTA,
 // each thread RU x RV outputs (rows ty + TY u, columns tx + 16 v) from
 // k-contiguous shared rows read as 16-byte words, slices streamed by a 4-stage cp.async
-// ring (one barrier per slice). The k order is that of gram_simt_kernel.
+// ring (one barrier per slice). The k order is that of gram_simt_kernel. Bound by the
+// chain of D / BK slices per tile: 256 x 256 x 784 takes 12.4 us (128-wide tiles: 102 us).
 // ---------------------------------------------------------------------------
 template <int T, int BK, int RU, int RV, bool SYM, bool VEC>
 __global__ void __launch_bounds__(16 * (T / RU))
@@ -264,8 +266,8 @@ __global__ void __launch_bounds__(16 * (T / RU))
 
 // Per-row sum(x^2) / D, the Gram's chain along the diagonal: 32 rows per CTA streamed
 // through a 4-stage cp.async ring by 128 threads, one lane of warp 0 per row running its
-// chain (bound by the 4-cycle dependent fmaf: D = 3072 takes 6 us; a thread per row
-// reading global memory took 207 us for 4001 rows). Blocks past the first input's rows
+// chain (bound by the 4-cycle dependent fmaf: 4001 + 1999 rows of D = 3072 take 24 us; a
+// thread per row reading global memory took 414 us). Blocks past the first input's rows
 // take the second's (n2 == 0: none).
 template <bool VEC>
 __global__ void __launch_bounds__(128)
@@ -305,6 +307,106 @@ __global__ void __launch_bounds__(128)
   }
   if (threadIdx.x < 32 && r0 + threadIdx.x < n)
     (second ? cov2 : cov1)[r0 + threadIdx.x] = acc * inv_d;
+}
+
+// ---------------------------------------------------------------------------
+// A run of Dense / activation rules on flat kernels in one pass: nngp and ntk are read
+// once and written once however many layers the run has, and the per-sample kernels
+// follow along. A CTA takes a 32 x 64 tile: 96 threads first run the variances of its
+// rows and columns through the layers (the activation rule on a sample with itself, as
+// affine_act_kernel evaluates it on a per-sample kernel) and leave each layer's
+// pre-activation variance and its square root in shared memory; then every thread runs
+// 8 entries (rows 4 warp + u, columns lane + 32 h) through them. Same operations per entry and per variance as one affine_act_kernel per
+// layer, so the results are those bit for bit. Bound by FP32 issue for a large kernel, by
+// the launch for a small one: three Erf layers of 4001 x 1999 take 65 us (18 launches,
+// seven of them over nngp and ntk: 337 us), two ReLU layers of 256 x 256 4.1 us (29 us).
+// ---------------------------------------------------------------------------
+constexpr int kFlatRows = 32, kFlatCols = 64, kFlatSamples = kFlatRows + kFlatCols;
+
+struct FlatRun {
+  int n;
+  ntg_flat_layer_t layer[NTG_FLAT_MAX_LAYERS];
+};
+
+// RELU: no activation or the ABRelu family without do_stabilize in every layer.
+template <bool RELU>
+__global__ void __launch_bounds__(256)
+    flat_rules_kernel(const __grid_constant__ FlatRun run, const float* in_q, const float* in_t,
+                      int64_t n1, int64_t n2, const float* var1, int64_t s1, const float* var2,
+                      int64_t s2, float* out_q, float* out_t, float* cov1, float* cov2) {
+  extern __shared__ float fv[];  // [layer][v | sqrt v][row or column]
+  const int64_t ntx = (n2 + kFlatCols - 1) / kFlatCols;
+  const int64_t by = blockIdx.x / ntx, bx = blockIdx.x - by * ntx;
+  const int64_t r0 = by * kFlatRows, c0 = bx * kFlatCols;
+  const int tid = threadIdx.x;
+  if (tid < kFlatSamples) {
+    const bool row = tid < kFlatRows;
+    const int64_t i = row ? r0 + tid : c0 + tid - kFlatRows;
+    const bool in = i < (row ? n1 : n2);
+    float v = in ? (row ? var1[i * s1] : var2[i * s2]) : 0.f;
+    for (int l = 0; l < run.n; ++l) {
+      const ntg_flat_layer_t& ly = run.layer[l];
+      if (ly.has_affine) v = fmaf(ly.aff.w2, v, ly.aff.b2);
+      if (ly.act.kind != NTG_ACT_NONE) {
+        const float s = sqrt_var(v);
+        fv[(2 * l) * kFlatSamples + tid] = v;
+        fv[(2 * l + 1) * kFlatSamples + tid] = s;
+        const ActC ac = act_consts(ly.act);
+        float t = 0.f;
+        const float vi = v;
+        act_apply<!RELU, !RELU>(ac, v, t, vi, vi, s, s);
+      }
+    }
+    if (in && row && bx == 0 && cov1) cov1[i] = v;
+    if (in && !row && by == 0 && cov2) cov2[i] = v;
+  }
+  __syncthreads();
+  const int lane = tid & 31, w = 4 * (tid >> 5);
+  float q[2][4], t[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t i = r0 + w + u, j = c0 + lane + 32 * h;
+      const bool in = i < n1 && j < n2;
+      q[h][u] = in ? in_q[i * n2 + j] : 0.f;
+      t[h][u] = in && in_t ? in_t[i * n2 + j] : 0.f;
+    }
+  for (int l = 0; l < run.n; ++l) {
+    const ntg_flat_layer_t& ly = run.layer[l];
+    if (ly.has_affine) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float a, b = 0.f;
+          apply_affine(ly.aff, q[h][u], t[h][u], out_t != nullptr, a, b);
+          q[h][u] = a;
+          t[h][u] = b;
+        }
+    }
+    if (ly.act.kind != NTG_ACT_NONE) {
+      const ActC ac = act_consts(ly.act);
+      const float* v = fv + (2 * l) * kFlatSamples;
+      const float* s = v + kFlatSamples;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float v2 = v[kFlatRows + lane + 32 * h], sv2 = s[kFlatRows + lane + 32 * h];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          act_apply<!RELU, !RELU>(ac, q[h][u], t[h][u], v[w + u], v2, s[w + u], sv2);
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t i = r0 + w + u, j = c0 + lane + 32 * h;
+      if (i >= n1 || j >= n2) continue;
+      out_q[i * n2 + j] = q[h][u];
+      if (out_t) out_t[i * n2 + j] = t[h][u];
+    }
 }
 
 bool rows_vec(const float* x1, const float* x2, int64_t d) {
@@ -395,4 +497,44 @@ extern "C" int ntg_cov_diag(void* stream, const float* x, int64_t n, int64_t d, 
   NTG_REQUIRE(x && cov, "ntg_cov_diag: null pointer");
   NTG_REQUIRE(n > 0 && d > 0, "ntg_cov_diag: sizes must be positive");
   return cov_rows(as_stream(stream), x, n, nullptr, 0, d, cov, nullptr);
+}
+
+extern "C" int ntg_flat_rules(void* stream, const float* in_q, const float* in_t, int64_t n1,
+                              int64_t n2, const float* var1, int64_t s1, const float* var2,
+                              int64_t s2, int32_t n_layers, const ntg_flat_layer_t* layers,
+                              float* out_q, float* out_t, float* cov1, float* cov2) {
+  NTG_REQUIRE(in_q && var1 && var2 && layers && out_q, "ntg_flat_rules: null pointer");
+  NTG_REQUIRE(n1 > 0 && n2 > 0 && s1 > 0 && s2 > 0, "ntg_flat_rules: bad sizes");
+  NTG_REQUIRE(n_layers > 0 && n_layers <= NTG_FLAT_MAX_LAYERS, "ntg_flat_rules: bad layer count");
+  FlatRun run;
+  run.n = n_layers;
+  bool relu = true;
+  for (int l = 0; l < n_layers; ++l) {
+    const ntg_act_t& a = layers[l].act;
+    NTG_REQUIRE(a.kind >= NTG_ACT_NONE && a.kind <= NTG_ACT_GELU,
+                "ntg_flat_rules: unknown activation kind");
+    relu = relu && (a.kind == NTG_ACT_NONE || (a.kind == NTG_ACT_ABRELU && a.stabilize <= 0.f));
+    run.layer[l] = layers[l];
+  }
+  const int64_t blocks = ceil_div(n1, kFlatRows) * ceil_div(n2, kFlatCols);
+  NTG_REQUIRE(blocks < (1ll << 31), "ntg_flat_rules: kernel too large");
+  const size_t sm = sizeof(float) * 2 * kFlatSamples * n_layers;
+  cudaStream_t s = as_stream(stream);
+  if (relu)
+    flat_rules_kernel<true><<<(unsigned)blocks, 256, sm, s>>>(run, in_q, in_t, n1, n2, var1, s1,
+                                                              var2, s2, out_q, out_t, cov1, cov2);
+  else
+    flat_rules_kernel<false><<<(unsigned)blocks, 256, sm, s>>>(run, in_q, in_t, n1, n2, var1, s1,
+                                                               var2, s2, out_q, out_t, cov1, cov2);
+  note_launch();
+  return check_launch("ntg_flat_rules");
+}
+
+extern "C" int ntg_flat_input(void* stream, const float* x1, const float* x2, int64_t n1,
+                              int64_t n2, int64_t d, float* nngp, float* cov1, float* cov2,
+                              int32_t precision, void* workspace, size_t workspace_bytes) {
+  const int rc = ntg_gram(stream, x1, x2, n1, n2, d, nngp, precision, workspace, workspace_bytes);
+  if (rc != NTG_OK || !cov1) return rc;
+  NTG_REQUIRE(cov2, "ntg_flat_input: cov1 and cov2 go together");
+  return cov_rows(as_stream(stream), x1, n1, x2, n2, d, cov1, cov2);
 }

@@ -233,9 +233,7 @@ def _act_cov(cv, ast, ds, a, c):
 def _act_rule(k: Kernel, p: dict, ctx: _Ctx) -> Kernel:
     """elementwise.py:1250-1275 + ABRelu :423-477 / Erf :67-112."""
     if not k.is_gaussian:
-        raise ValueError('The input to the activation function must be Gaussian, '
-                         'i.e. a random affine transform is required before the '
-                         'activation function.')
+        raise ValueError(_NOT_GAUSSIAN)
     q, t, c1, c2 = _tensors(k)
     ds = k.diagonal_spatial
     a, c = O.spatial_ac(q, 2, ds)
@@ -400,6 +398,52 @@ def _flatten_rule(k: Kernel, p: dict, ctx: _Ctx) -> Kernel:
                    is_reversed=False, diagonal_spatial=False)
 
 
+_NOT_GAUSSIAN = ('The input to the activation function must be Gaussian, i.e. a random affine '
+                 'transform is required before the activation function.')
+
+
+def _flat_run(k: Kernel, specs, i: int) -> int:
+    """End of the run of Dense / activation layers from specs[i] that _flat_rules takes on k:
+    flat kernels, no do_stabilize (it rescales by the pre-activation maximum). An activation
+    right on the scalar-zero NTK of an input kernel stays with _act_rule, which keeps it."""
+    first = next((s.kind for s in specs[i:] if s.kind != 'identity'), None)
+    if k.nngp.ndim != 2 or first is None or (first == 'act' and _zero_ntk(k)):
+        return i
+    end = i
+    while end < len(specs) and (specs[end].kind in ('dense', 'identity') or (
+            specs[end].kind == 'act' and not specs[end].params.get('do_stabilize'))):
+        end += 1
+    return end if any(s.kind != 'identity' for s in specs[i:end]) else i
+
+
+def _flat_rules(k: Kernel, specs, ctx: _Ctx) -> Kernel:
+    """The rules of a run of layers (linear.py:899-926, elementwise.py:1250-1275) on flat
+    kernels, one launch per NTG_FLAT_MAX_LAYERS affine / activation pairs."""
+    layers = []
+    shape1, shape2, gaussian = k.shape1, k.shape2, k.is_gaussian
+    for s in specs:
+        p = s.params
+        if s.kind == 'dense':
+            fan = shape1[-1] / p['s'][0] if p['parameterization'] == 'standard' else None
+            layers.append([_affine_struct(p['W_std'], p['b_std'], p['parameterization'], fan),
+                           O.NO_ACT])
+            gaussian = True
+        elif s.kind == 'act':
+            if not gaussian:
+                raise ValueError(_NOT_GAUSSIAN)
+            if not layers or layers[-1][1] is not O.NO_ACT:
+                layers.append([None, O.NO_ACT])
+            layers[-1][1] = _act_struct(p, ctx)
+            gaussian = False
+        shape1, shape2 = s.shape_fn(shape1), s.shape_fn(shape2)
+    q, t = k.nngp.contiguous(), None if k.ntk is None or _zero_ntk(k) else k.ntk.contiguous()
+    c1, c2 = k.cov1, k.cov2
+    for j in range(0, len(layers), L.FLAT_MAX_LAYERS):
+        q, t, c1, c2 = O.flat_rules(q, t, c1, c2, layers[j:j + L.FLAT_MAX_LAYERS], _has_ntk(k))
+    return k.replace(nngp=q, ntk=t, cov1=c1, cov2=c2, is_gaussian=gaussian, is_input=False,
+                     shape1=shape1, shape2=shape2)
+
+
 RULES = {'dense': _dense_rule, 'conv': _conv_rule, 'act': _act_rule, 'pool': _pool_rule,
          'gpool': _gpool_rule, 'flatten': _flatten_rule}
 
@@ -537,8 +581,10 @@ def _normalize_get(get):
 
 
 def _input_kernel(x1: torch.Tensor, x2: Optional[torch.Tensor], diagonal_spatial: bool,
-                  compute_ntk: bool, channel_axis_none: bool, ctx: _Ctx) -> Kernel:
-    """requirements.py:641-830 (batch axis 0, channel axis -1)."""
+                  compute_ntk: bool, channel_axis_none: bool, ctx: _Ctx,
+                  inner: bool = False) -> Kernel:
+    """requirements.py:641-830 (batch axis 0, channel axis -1). inner: the Kernel goes to a
+    Dense rule, which reads the self covariances of x2 = None on nngp's diagonal in place."""
     shape1 = tuple(x1.shape)
     shape2 = shape1 if x2 is None else tuple(x2.shape)
     if x1.ndim < 2:
@@ -552,14 +598,11 @@ def _input_kernel(x1: torch.Tensor, x2: Optional[torch.Tensor], diagonal_spatial
     prec = 1 if ctx.precision == 'mixed' else 0
     xb = x1 if x2 is None else x2
     if x1.ndim == 2:
-        nngp = O.gram(x1, xb, prec)
-        if x2 is None:
-            # the self covariances are the Gram diagonal itself, so that a self
-            # pair has var1 * var2 - nngp^2 == 0 exactly
-            cov1 = torch.diagonal(nngp).contiguous()
-        else:
-            cov1 = O.cov_diag(x1)
-        cov2 = None if x2 is None else O.cov_diag(x2)
+        # x2 None: the self covariances are the Gram diagonal itself, so that a self
+        # pair has var1 * var2 - nngp^2 == 0 exactly
+        nngp, cov1, cov2 = O.flat_input(x1, x2, prec)
+        if x2 is None and not inner:
+            cov1 = cov1.contiguous()
     elif diagonal_spatial:
         # per-position channel dot products [N1, N2, *spatial]
         nngp = O.input_ds(x1, xb)
@@ -604,6 +647,11 @@ class KernelFn:
         i = 0
         while i < len(specs):
             s = specs[i]
+            end = _flat_run(k, specs, i)
+            if end > i:
+                k = _flat_rules(k, specs[i:end], ctx)
+                i = end
+                continue
             nxt = specs[i + 1] if i + 1 < len(specs) else None
             if s.kind in ('dense', 'conv') and nxt is not None and nxt.kind == 'act' \
                     and not nxt.params.get('do_stabilize'):
@@ -682,7 +730,9 @@ class KernelFn:
             k = _chain.try_fused(self, x1, x2t, ds, compute_ntk, ctx)
             if k is None:
                 cnone = bool(self.specs) and self.specs[0].channel_axis_none
-                k = _input_kernel(x1, x2t, ds, compute_ntk, cnone, ctx)
+                first = next((sp for sp in self.specs if sp.kind != 'identity'), None)
+                k = _input_kernel(x1, x2t, ds, compute_ntk, cnone, ctx,
+                                  inner=first is not None and first.kind == 'dense')
                 k = self.apply_kernel(k, ctx)
         if names is None:
             return k
