@@ -191,11 +191,13 @@ def self_chain(x: torch.Tensor, plan: ChainPlan, ctx: _Ctx):
 
 
 def try_fused(kfn, x1: torch.Tensor, x2: Optional[torch.Tensor], diagonal_spatial: bool,
-              compute_ntk: bool, ctx: _Ctx) -> Optional[Kernel]:
+              compute_ntk: bool, ctx: _Ctx, compare: bool = True) -> Optional[Kernel]:
+    """The fused chain's Kernel, or None for another network; compare: x1_is_x2 is wanted
+    (an element-wise comparison of x1 and x2), else it says whether x2 was left out."""
     plan = plan_chain(kfn.specs, tuple(x1.shape), diagonal_spatial)
     if plan is None or (x2 is not None and tuple(x2.shape[1:]) != tuple(x1.shape[1:])):
         return None
-    k = run_fused(plan, x1, x2, ctx)
+    k = run_fused(plan, x1, x2, ctx, x1_is_x2=None if compare else x2 is None)
     k = kfn.apply_kernel(k, ctx, specs=plan.post)
     if not compute_ntk:
         k = k.replace(ntk=None)

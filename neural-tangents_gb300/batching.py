@@ -112,7 +112,7 @@ def _forward_grid(kernel_fn, x1t, x2t, bs, precision):
         old = _chain.SELF_CHUNK
         _chain.SELF_CHUNK = max(1, min(old, bs))
         try:
-            k = _chain.run_fused(plan, x1t, x2t, ctx)
+            k = _chain.run_fused(plan, x1t, x2t, ctx, x1_is_x2=x2t is None)
         finally:
             _chain.SELF_CHUNK = old
         return kernel_fn.apply_kernel(k, ctx, specs=plan.post)
@@ -173,7 +173,9 @@ def batch(kernel_fn, batch_size: int = 0, device_count: int = -1, store_on_devic
                 old = _chain.SELF_CHUNK
                 _chain.SELF_CHUNK = max(1, min(old, bs))
                 try:
-                    k = _chain.run_fused(plan, x1t, x2t, ctx)
+                    k = _chain.run_fused(
+                        plan, x1t, x2t, ctx,
+                        x1_is_x2=None if names is None or 'x1_is_x2' in names else x2t is None)
                 finally:
                     _chain.SELF_CHUNK = old
                 k = kernel_fn.apply_kernel(k, ctx, specs=plan.post)

@@ -639,8 +639,6 @@ __global__ void input_fs_t_kernel(const float* __restrict__ g, const float* __re
 //   gx2[i2, h', w', k] += sum_{i1, h, w}   G[i1, i2, h, h', w, w'] x1[i1, h, w, k] / K
 constexpr int kIfC = 32;
 
-__device__ int g_bwd_error = 0;
-
 constexpr int kIfRing = 4;
 
 // Two-pass form of the input-covariance adjoint, each pass a pure stream over G
@@ -656,7 +654,7 @@ template <int K, bool COLS>
 __global__ void __launch_bounds__(256)
     input_fs_pass_kernel(const float* __restrict__ g, const float* __restrict__ x1,
                          const float* __restrict__ x2, float* __restrict__ gx, int64_t n1,
-                         int64_t n2, int A, float inv_k) {
+                         int64_t n2, int A, float inv_k, int* err) {
   constexpr int C = kIfC;
   constexpr int XF = C * K;
   __shared__ __align__(128) float gs[kIfRing][C * C];
@@ -779,7 +777,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (tid == 0 && s_err) {
-    atomicExch(&g_bwd_error, NTG_ERR_WAIT_TIMEOUT);
+    raise_timeout(err);
     for (int64_t p = issued > kIfRing ? issued - kIfRing : 0; p < issued; ++p)
       bar_wait(smem_addr(&bars[p % kIfRing]), (uint32_t)((p / kIfRing) & 1));
   }
@@ -1051,6 +1049,8 @@ extern "C" int ntg_input_fs_bwd2(void* stream, const float* g, const float* x1,
                     ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(x1) |
                       reinterpret_cast<uintptr_t>(x2)) & 15) == 0;
   if (fast && n2 * a < (1ll << 31)) {
+    int* err = device_error_word();
+    NTG_REQUIRE(err, "ntg_input_fs_bwd2: no device error word");
     const float inv_k = 1.f / (float)k;
     // rows into gx1, then columns into gx2 (gx1 for the per-sample covariances, or when
     // x2 is x1); two launches on one stream, so a shared gx is never written concurrently
@@ -1059,20 +1059,20 @@ extern "C" int ntg_input_fs_bwd2(void* stream, const float* g, const float* x1,
     float* gc = n2 > 0 ? gx2 : gx1;
     switch (k) {
       case 1:
-        input_fs_pass_kernel<1, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k);
-        input_fs_pass_kernel<1, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k);
+        input_fs_pass_kernel<1, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k, err);
+        input_fs_pass_kernel<1, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k, err);
         break;
       case 2:
-        input_fs_pass_kernel<2, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k);
-        input_fs_pass_kernel<2, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k);
+        input_fs_pass_kernel<2, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k, err);
+        input_fs_pass_kernel<2, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k, err);
         break;
       case 3:
-        input_fs_pass_kernel<3, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k);
-        input_fs_pass_kernel<3, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k);
+        input_fs_pass_kernel<3, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k, err);
+        input_fs_pass_kernel<3, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k, err);
         break;
       default:
-        input_fs_pass_kernel<4, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k);
-        input_fs_pass_kernel<4, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k);
+        input_fs_pass_kernel<4, false><<<grid_r, 256, 0, s>>>(g, x1, x2, gx1, n1, n2, (int)a, inv_k, err);
+        input_fs_pass_kernel<4, true><<<grid_c, 256, 0, s>>>(g, x1, x2, gc, n1, n2, (int)a, inv_k, err);
         break;
     }
     note_launch();
@@ -1158,16 +1158,6 @@ extern "C" int ntg_input_ds_bwd(void* stream, const float* g, const float* x1, c
   }
   return check_launch("ntg_input_ds_bwd");
 }
-
-namespace ntg {
-int bwd_take_device_error() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_bwd_error, sizeof(int)) != cudaSuccess) return -1;
-  const int zero = 0;
-  if (v != 0 && cudaMemcpyToSymbol(g_bwd_error, &zero, sizeof(int)) != cudaSuccess) return -1;
-  return v;
-}
-}  // namespace ntg
 
 extern "C" int ntg_diag_add(void* stream, const float* src, float* dst, int64_t n, int64_t a,
                             int64_t c, int64_t s_n, int64_t s_a, int64_t s_c) {

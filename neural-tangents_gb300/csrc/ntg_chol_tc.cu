@@ -45,8 +45,6 @@ constexpr int kSmallM = 16;    // right-hand sides of the cooperative solves
 constexpr int kGT = 128;       // rows of a split-K product tile (one per thread)
 constexpr int kGK = 32;        // columns staged in shared memory per step
 
-__device__ int g_chol_error = 0;
-
 __host__ __device__ __forceinline__ int64_t mini(int64_t a, int64_t b) { return a < b ? a : b; }
 
 // Grid of a grid-stride loop over n elements, 256 threads a block.
@@ -1119,14 +1117,6 @@ int inv_apply_many(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, fl
 }
 
 }  // namespace
-
-int chol_take_device_error() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_chol_error, sizeof(int)) != cudaSuccess) return -1;
-  const int zero = 0;
-  if (v != 0 && cudaMemcpyToSymbol(g_chol_error, &zero, sizeof(int)) != cudaSuccess) return -1;
-  return v;
-}
 
 }  // namespace ntg
 

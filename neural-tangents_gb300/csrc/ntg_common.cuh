@@ -19,12 +19,11 @@ int fail(int code, const std::string& msg);
 int check_launch(const char* what);
 void note_launch(uint64_t n = 1);
 int32_t tune(int32_t knob);  // current value of an NTG_TUNE_* knob
-// Read and clear the device error words of the adjoint kernels (ntg_bwd.cu)
-// and of the tensor-core Gram (ntg_gram_tc.cu); -1 if the read failed.
-int bwd_take_device_error();
-int gram_take_device_error();
-int gemm_take_device_error();  // ntg_gemm_tc.cu
-int chol_take_device_error();  // ntg_chol_tc.cu
+// The current device's error word, which a kernel whose bounded wait runs out sets through
+// raise_timeout: host memory mapped into the device, so that ntg_device_status reads it
+// without a copy (five copies from device symbols took 70 us of every public call). One
+// word per device, allocated once; null if that failed.
+int* device_error_word();
 
 // Tensor-core (tcgen05) split-precision Gram; defined in ntg_gram_tc.cu.
 int gram_tc(cudaStream_t stream, const float* x1, const float* x2, int64_t n1, int64_t n2,
@@ -45,6 +44,11 @@ constexpr float kPi = 3.14159265358979323846f;
 // that runs out returns false; the kernel then raises its device error word.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kLineWaitLimit = 1u << 20;
+
+__device__ __forceinline__ void raise_timeout(int* err) {
+  *reinterpret_cast<volatile int*>(err) = NTG_ERR_WAIT_TIMEOUT;
+  __threadfence_system();
+}
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

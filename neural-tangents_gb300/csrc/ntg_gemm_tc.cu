@@ -67,14 +67,13 @@ constexpr uint32_t GTMEM_COLS = 128;
 constexpr uint64_t GWAIT = 1ull << 21;
 constexpr uint32_t GIDESC = tc::idesc(2, GM, GN);  // kind::tf32
 
-__device__ int g_gemm_error = 0;
-
 struct GemmArgs {
   float* c;
   int64_t ldc, m, n, k;
   float alpha, beta;
   int32_t lower;
   int32_t tiles_n;
+  int* err;
 };
 
 __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t acc) {
@@ -173,7 +172,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
         issued = kc + 1;
       }
       if (!ok) {
-        atomicExch(&g_gemm_error, NTG_ERR_WAIT_TIMEOUT);
+        raise_timeout(p.err);
         s_fail = 1;
       }
     }
@@ -200,7 +199,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
       }
       tc::commit(tc::smem_u32(&bars[3 * GSTAGES]));  // accumulator complete (or all issued)
       if (!ok) {
-        atomicExch(&g_gemm_error, NTG_ERR_WAIT_TIMEOUT);
+        raise_timeout(p.err);
         s_fail = 1;
       }
     }
@@ -221,13 +220,13 @@ __global__ void __launch_bounds__(GTHREADS, 1)
       if (lane == 0) tc::mbar_arrive(tc::smem_u32(&bars[GSTAGES + s]));
     }
     if (!ok && lane == 0) {
-      atomicExch(&g_gemm_error, NTG_ERR_WAIT_TIMEOUT);
+      raise_timeout(p.err);
       s_fail = 1;
     }
     ready = tc::mbar_wait(tc::smem_u32(&bars[3 * GSTAGES]), 0, GWAIT);
     ready = __all_sync(0xffffffffu, ready);
     if (!ready && lane == 0) {
-      atomicExch(&g_gemm_error, NTG_ERR_WAIT_TIMEOUT);
+      raise_timeout(p.err);
       s_fail = 1;
     }
   }
@@ -318,14 +317,6 @@ __global__ void __launch_bounds__(GTHREADS, 1)
 
 }  // namespace
 
-int gemm_take_device_error() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(int)) != cudaSuccess) return -1;
-  const int zero = 0;
-  if (v != 0 && cudaMemcpyToSymbol(g_gemm_error, &zero, sizeof(int)) != cudaSuccess) return -1;
-  return v;
-}
-
 int gemm_tf32x3(cudaStream_t s, const float* a, int64_t lda, const float* b, int64_t ldb,
                 float* c, int64_t ldc, int64_t m, int64_t n, int64_t k, float alpha, float beta,
                 int lower) {
@@ -357,7 +348,8 @@ int gemm_tf32x3(cudaStream_t s, const float* a, int64_t lda, const float* b, int
   });
   if (attr_err != cudaSuccess)
     return fail(NTG_ERR_CUDA, std::string("ntg_gemm_tc: ") + cudaGetErrorString(attr_err));
-  GemmArgs p{c, ldc, m, n, k, alpha, beta, lower, (int32_t)tn};
+  GemmArgs p{c, ldc, m, n, k, alpha, beta, lower, (int32_t)tn, device_error_word()};
+  NTG_REQUIRE(p.err, "ntg_gemm_tc: no device error word");
   gemm_tf32x3_kernel<<<(unsigned)tiles, GTHREADS, GSMEM, s>>>(ma, mb, p);
   note_launch();
   return check_launch("ntg_gemm_tc");

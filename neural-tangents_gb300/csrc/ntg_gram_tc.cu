@@ -29,8 +29,6 @@ constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // A_hi, A_lo, B_hi, B_l
 constexpr uint32_t TMEM_COLS = BN;
 constexpr uint64_t WAIT_LIMIT = 1ull << 20;   // about a second of polling
 
-__device__ int g_gram_error = 0;
-
 // hi = bf16(x), lo = bf16(x - hi) for x [n, d] into [npad, dpad] (zero padding), eight
 // consecutive entries of a row per thread: two 16-byte loads (when rows are 16-byte
 // aligned) and one 16-byte store into each of hi and lo.
@@ -126,7 +124,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     gram_tc_kernel(const __grid_constant__ CUtensorMap ta_hi, const __grid_constant__ CUtensorMap ta_lo,
                    const __grid_constant__ CUtensorMap tb_hi, const __grid_constant__ CUtensorMap tb_lo,
                    float* __restrict__ out, int64_t n1, int64_t n2, int64_t dpad, float inv_d,
-                   int sym, int64_t ntiles, int64_t nbn, int* err) {
+                   int sym, int64_t ntiles, int64_t nbn, int* err, int* word) {
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment for the swizzled tiles
   uint8_t* smem = reinterpret_cast<uint8_t*>(
@@ -194,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!ok) {
         atomicExch(err, 1);
-        atomicExch(&g_gram_error, NTG_ERR_WAIT_TIMEOUT);
+        raise_timeout(word);
         s_fail = 1;
       }
     }
@@ -231,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mma_commit(smem_u32(drain));  // every MMA issued, retired before TMEM is freed
       if (!ok) {
         atomicExch(err, 2);
-        atomicExch(&g_gram_error, NTG_ERR_WAIT_TIMEOUT);
+        raise_timeout(word);
         s_fail = 1;
       }
     }
@@ -244,7 +242,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!mbar_wait(smem_u32(&tfull[b]), (uint32_t)((it >> 1) & 1))) {
         if (lane == 0) {
           atomicExch(err, 3);
-          atomicExch(&g_gram_error, NTG_ERR_WAIT_TIMEOUT);
+          raise_timeout(word);
           s_fail = 1;
         }
         break;
@@ -306,14 +304,6 @@ int make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t dpad, int b
 
 }  // namespace
 
-int gram_take_device_error() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_gram_error, sizeof(int)) != cudaSuccess) return -1;
-  const int zero = 0;
-  if (v != 0 && cudaMemcpyToSymbol(g_gram_error, &zero, sizeof(int)) != cudaSuccess) return -1;
-  return v;
-}
-
 size_t gram_tc_workspace(int64_t n1, int64_t n2, int64_t d) {
   const int64_t dpad = ceil_div(d, BK) * BK;
   const int64_t p1 = ceil_div(n1, BM) * BM, p2 = ceil_div(n2, BN) * BN;
@@ -325,6 +315,8 @@ int gram_tc(cudaStream_t s, const float* x1, const float* x2, int64_t n1, int64_
   NTG_REQUIRE(workspace && ws_bytes >= gram_tc_workspace(n1, n2, d),
               "ntg_gram: precision 1 needs ntg_gram_workspace_bytes(n1, n2, d) of workspace");
   NTG_REQUIRE(ceil_div(n1, BM) <= 65535, "ntg_gram: n1 too large");
+  int* word = device_error_word();
+  NTG_REQUIRE(word, "ntg_gram: no device error word");
   const int64_t dpad = ceil_div(d, BK) * BK;
   const int64_t p1 = ceil_div(n1, BM) * BM, p2 = ceil_div(n2, BN) * BN;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
@@ -374,7 +366,7 @@ int gram_tc(cudaStream_t s, const float* x1, const float* x2, int64_t n1, int64_
   const unsigned ctas = (unsigned)std::min<int64_t>(ntiles, num_sms > 0 ? num_sms : 148);
   gram_tc_kernel<<<ctas, kThreads, P_SMEM_BYTES, s>>>(m[0], m[1], m[2], m[3], out, n1, n2, dpad,
                                                       1.f / (float)d, sym ? 1 : 0, ntiles, nbn,
-                                                      err);
+                                                      err, word);
   note_launch();
   return check_launch("ntg_gram (tcgen05)");
 }

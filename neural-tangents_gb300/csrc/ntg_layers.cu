@@ -324,14 +324,12 @@ __global__ void __launch_bounds__(kThreads)
 // ---------------------------------------------------------------------------
 constexpr int kRing = 4;
 
-__device__ int g_device_error = 0;
-
 template <bool HAS_T>
 __global__ void __launch_bounds__(kThreads)
     conv3_line_bulk_kernel(const float* __restrict__ in_q, const float* __restrict__ in_t,
                            float* __restrict__ out_q, float* __restrict__ out_t, int64_t batch,
                            int64_t n2, int A, int C, ntg_affine_t aff, ntg_act_t act,
-                           ntg_var_t var1, ntg_var_t var2) {
+                           ntg_var_t var1, ntg_var_t var2, int* err) {
   extern __shared__ __align__(128) float smem[];
   const int plane = C * C;
   const int P = C + 2;
@@ -496,7 +494,7 @@ __global__ void __launch_bounds__(kThreads)
     buf ^= 1;
   }
   if (!ok && threadIdx.x == 0) {
-    atomicExch(&g_device_error, NTG_ERR_WAIT_TIMEOUT);
+    raise_timeout(err);
     // let every issued copy land (bounded) before the CTA's shared memory is released
     for (int j = 0; j < len; ++j) bar_wait(smem_addr(&bars[j % kRing]), (uint32_t)((j / kRing) & 1));
   }
@@ -550,7 +548,7 @@ __global__ void __launch_bounds__(kThreads)
                       float* __restrict__ out_q, float* __restrict__ out_t, int64_t batch,
                       int64_t n2, int A, ntg_affine_t aff, ntg_act_t act, ntg_var_t var1,
                       ntg_var_t var2, float* __restrict__ pre_q, float* __restrict__ pre_t,
-                      float* __restrict__ hp_q, float* __restrict__ hp_t) {
+                      float* __restrict__ hp_q, float* __restrict__ hp_t, int* err) {
   extern __shared__ __align__(128) float smem[];
   __shared__ int s_err;
   float* ring_q = smem;                           // [RING][plane]
@@ -801,7 +799,7 @@ __global__ void __launch_bounds__(kThreads)
   if (tid == 0) {
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (s_err) {
-      atomicExch(&g_device_error, NTG_ERR_WAIT_TIMEOUT);
+      raise_timeout(err);
       // let every issued copy land (bounded) before the CTA's shared memory is released
       for (int p = next > RING ? next - RING : 0; p < next; ++p)
         bar_wait(smem_addr(&bars[p % RING]), (uint32_t)((p / RING) & 1));
@@ -1048,7 +1046,8 @@ __device__ __forceinline__ void skew_vjp_body(
     const float* __restrict__ pre_q, const float* __restrict__ pre_t,
     const float* __restrict__ g_q, const float* __restrict__ g_t, float* __restrict__ gin_q,
     float* __restrict__ gin_t, int64_t batch, int64_t n2, int A, float w2, ntg_act_t act,
-    ntg_var_t var1, ntg_var_t var2, float* __restrict__ gvar1, float* __restrict__ gvar2) {
+    ntg_var_t var1, ntg_var_t var2, float* __restrict__ gvar1, float* __restrict__ gvar2,
+    int* err) {
   extern __shared__ __align__(128) float smem[];
   __shared__ int s_err;
   constexpr int GP = POOLED ? kSkewPlane / 4 : kSkewPlane;  // floats of a cotangent plane
@@ -1283,7 +1282,7 @@ __device__ __forceinline__ void skew_vjp_body(
   if (tid == 0) {
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     if (s_err) {
-      atomicExch(&g_device_error, NTG_ERR_WAIT_TIMEOUT);
+      raise_timeout(err);
       // let every issued copy land (bounded) before the CTA's shared memory is released
       for (int p = next > kVjpRing ? next - kVjpRing : 0; p < next; ++p)
         bar_wait(smem_addr(&bars[p % kVjpRing]), (uint32_t)((p / kVjpRing) & 1));
@@ -1297,9 +1296,9 @@ __global__ void __launch_bounds__(kThreads)
                           const float* __restrict__ g_q, const float* __restrict__ g_t,
                           float* __restrict__ gin_q, float* __restrict__ gin_t, int64_t batch,
                           int64_t n2, int A, float w2, ntg_act_t act, ntg_var_t var1,
-                          ntg_var_t var2, float* __restrict__ gvar1, float* __restrict__ gvar2) {
+                          ntg_var_t var2, float* __restrict__ gvar1, float* __restrict__ gvar2, int* err) {
   skew_vjp_body<POOLED>(pre_q, pre_t, g_q, g_t, gin_q, gin_t, batch, n2, A, w2, act, var1, var2,
-                        gvar1, gvar2);
+                        gvar1, gvar2, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -1703,13 +1702,15 @@ cudaError_t launch_skew_k(cudaStream_t s, int64_t blocks, size_t sm, const float
                           int64_t n2, int64_t a, ntg_affine_t aff, ntg_act_t act, ntg_var_t var1,
                           ntg_var_t var2, float* pre_q, float* pre_t, float* hp_q,
                           float* hp_t) {
+  int* err = device_error_word();
+  if (!err) return cudaErrorMemoryAllocation;
   cudaError_t e = cudaFuncSetAttribute(conv3_skew_kernel<HAS_T, RING, ACTK, HP>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)skew_smem_bytes_pre<RING>());
   if (e == cudaSuccess)
     conv3_skew_kernel<HAS_T, RING, ACTK, HP><<<(unsigned)blocks, kThreads, sm, s>>>(
         in_q, in_t, out_q, out_t, batch, n2, (int)a, aff, act, var1, var2, pre_q, pre_t, hp_q,
-        hp_t);
+        hp_t, err);
   return e;
 }
 
@@ -1793,19 +1794,21 @@ extern "C" int ntg_conv_fs(void* stream, const float* in_q, const float* in_t, f
     NTG_REQUIRE(blocks < (1ll << 31), "ntg_conv_fs: grid too large");
     const size_t sm = sizeof(float) * (2 * kRing * c * c + 4 * (c + 2) * (c + 2)) +
                       sizeof(uint64_t) * kRing;
+    int* err = device_error_word();
+    NTG_REQUIRE(err, "ntg_conv_fs: no device error word");
     cudaError_t e;
     if (in_t) {
       e = cudaFuncSetAttribute(conv3_line_bulk_kernel<true>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e == cudaSuccess)
         conv3_line_bulk_kernel<true><<<(unsigned)blocks, kThreads, sm, s>>>(
-            in_q, in_t, out_q, out_t, batch, n2, (int)a, (int)c, aff, act, var1, var2);
+            in_q, in_t, out_q, out_t, batch, n2, (int)a, (int)c, aff, act, var1, var2, err);
     } else {
       e = cudaFuncSetAttribute(conv3_line_bulk_kernel<false>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e == cudaSuccess)
         conv3_line_bulk_kernel<false><<<(unsigned)blocks, kThreads, sm, s>>>(
-            in_q, nullptr, out_q, out_t, batch, n2, (int)a, (int)c, aff, act, var1, var2);
+            in_q, nullptr, out_q, out_t, batch, n2, (int)a, (int)c, aff, act, var1, var2, err);
     }
     if (e != cudaSuccess) return fail(NTG_ERR_CUDA, std::string("ntg_conv_fs: ") + cudaGetErrorString(e));
   } else if (line_ok) {
@@ -1922,6 +1925,8 @@ cudaError_t launch_skew_vjp(cudaStream_t s, int64_t blocks, const float* pre_q, 
                             int64_t batch, int64_t n2, int64_t a, float w2, ntg_act_t act,
                             ntg_var_t var1, ntg_var_t var2, float* gvar1, float* gvar2) {
   constexpr size_t sm = skew_vjp_smem_bytes<POOLED>();
+  int* err = device_error_word();
+  if (!err) return cudaErrorMemoryAllocation;
   cudaError_t e = cudaFuncSetAttribute(conv3_skew_vjp_kernel<POOLED>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   // all of the unified L1 / shared memory as shared memory: the resident CTAs' rings
@@ -1931,7 +1936,7 @@ cudaError_t launch_skew_vjp(cudaStream_t s, int64_t blocks, const float* pre_q, 
   if (e == cudaSuccess)
     conv3_skew_vjp_kernel<POOLED><<<(unsigned)blocks, kThreads, sm, s>>>(
         pre_q, pre_t, g_q, g_t, gin_q, gin_t, batch, n2, (int)a, w2, act, var1, var2, gvar1,
-        gvar2);
+        gvar2, err);
   return e;
 }
 
@@ -2105,22 +2110,4 @@ extern "C" int ntg_flatten_fs(void* stream, const float* in, float* out, int64_t
   flatten_fs_kernel<<<(unsigned)batch, kThreads, 0, as_stream(stream)>>>(in, out, a, c);
   note_launch();
   return check_launch("ntg_flatten_fs");
-}
-
-extern "C" int ntg_device_status(void) {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_device_error, sizeof(int)) != cudaSuccess)
-    return check_launch("ntg_device_status");
-  const int zero = 0;
-  if (v != 0 && cudaMemcpyToSymbol(g_device_error, &zero, sizeof(int)) != cudaSuccess)
-    return check_launch("ntg_device_status");
-  // every word is read and cleared, so one timeout is reported once
-  const int others[4] = {bwd_take_device_error(), gram_take_device_error(),
-                         gemm_take_device_error(), chol_take_device_error()};
-  for (int o : others) {
-    if (o < 0) return check_launch("ntg_device_status");
-    if (v == 0) v = o;
-  }
-  if (v != 0) return fail(v, "a bounded device wait ran out in a streamed kernel");
-  return NTG_OK;
 }

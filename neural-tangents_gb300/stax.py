@@ -582,9 +582,11 @@ def _normalize_get(get):
 
 def _input_kernel(x1: torch.Tensor, x2: Optional[torch.Tensor], diagonal_spatial: bool,
                   compute_ntk: bool, channel_axis_none: bool, ctx: _Ctx,
-                  inner: bool = False) -> Kernel:
+                  inner: bool = False, compare: bool = True) -> Kernel:
     """requirements.py:641-830 (batch axis 0, channel axis -1). inner: the Kernel goes to a
-    Dense rule, which reads the self covariances of x2 = None on nngp's diagonal in place."""
+    Dense rule, which reads the self covariances of x2 = None on nngp's diagonal in place and
+    replaces the scalar-zero NTK. compare: x1_is_x2 is wanted, which takes the host a look
+    at both inputs (a synchronisation); otherwise it says whether x2 was left out."""
     shape1 = tuple(x1.shape)
     shape2 = shape1 if x2 is None else tuple(x2.shape)
     if x1.ndim < 2:
@@ -621,8 +623,10 @@ def _input_kernel(x1: torch.Tensor, x2: Optional[torch.Tensor], diagonal_spatial
             nngp = nngp.reshape(nngp.shape[0], nngp.shape[1], a, a)
             cov1 = cov1.reshape(cov1.shape[0], a, a)
             cov2 = None if cov2 is None else cov2.reshape(cov2.shape[0], a, a)
-    ntk = torch.zeros((), device=x1.device) if compute_ntk else None
-    x1_is_x2 = x2 is None or (x1.shape == x2.shape and bool(torch.equal(x1, x2)))
+    ntk = None
+    if compute_ntk:
+        ntk = torch.zeros(()) if inner else torch.zeros((), device=x1.device)
+    x1_is_x2 = x2 is None or (compare and x1.shape == x2.shape and bool(torch.equal(x1, x2)))
     return Kernel(nngp=nngp, ntk=ntk, cov1=cov1, cov2=cov2, x1_is_x2=x1_is_x2,
                   is_gaussian=False, is_reversed=False, is_input=False, diagonal_batch=True,
                   diagonal_spatial=bool(diagonal_spatial), shape1=shape1, shape2=shape2)
@@ -727,12 +731,14 @@ class KernelFn:
                     return k
                 vals = tuple(getattr(k, n) for n in names)
                 return vals[0] if single is not None else analytic_kernel(names, vals)
-            k = _chain.try_fused(self, x1, x2t, ds, compute_ntk, ctx)
+            compare = names is None or 'x1_is_x2' in names
+            k = _chain.try_fused(self, x1, x2t, ds, compute_ntk, ctx, compare)
             if k is None:
                 cnone = bool(self.specs) and self.specs[0].channel_axis_none
                 first = next((sp for sp in self.specs if sp.kind != 'identity'), None)
                 k = _input_kernel(x1, x2t, ds, compute_ntk, cnone, ctx,
-                                  inner=first is not None and first.kind == 'dense')
+                                  inner=first is not None and first.kind == 'dense',
+                                  compare=compare)
                 k = self.apply_kernel(k, ctx)
         if names is None:
             return k
