@@ -264,6 +264,21 @@ int ntg_chain_fwd(void* stream, const ntg_chain_t* prog, const float* x1, const 
 int ntg_chain_fwd_sym(void* stream, const ntg_chain_t* prog, const float* x, int64_t r0,
                       int64_t n1, int64_t c0, int64_t n2, const float* var, float* out_q,
                       float* out_t, int64_t ld_out);
+/* The same with the caller's scratch (ntg_chain_workspace_bytes(), 16-byte aligned, not shared
+ * by calls that may overlap): the two calls above take stream-ordered memory for it.
+ *   mode 0: ntg_chain_fwd; mode 1: ntg_chain_fwd_sym (x2 == x1, var2 == var1);
+ *   mode 2: the self pairs (r0 + i, r0 + i), i < n1, of x1 == x2, into out[i]. */
+size_t ntg_chain_workspace_bytes(void);
+/* The pre-activation variance maps of every conv layer of the network, as the calls above
+ * read them: var [N, var_stride], layer l's S x S map at var_off[l]; of two inputs in one
+ * launch (n2 == 0: of x1 only). */
+int ntg_chain_vars(void* stream, const ntg_chain_t* prog, const float* x1, int64_t n1, float* var1,
+                   const float* x2, int64_t n2, float* var2, void* workspace,
+                   size_t workspace_bytes);
+int ntg_chain_fwd_ws(void* stream, const ntg_chain_t* prog, const float* x1, const float* x2,
+                     int64_t r0, int64_t n1, int64_t c0, int64_t n2, const float* var1,
+                     const float* var2, float* out_q, float* out_t, int64_t ld_out, int32_t mode,
+                     void* workspace, size_t workspace_bytes);
 
 /* ---- kernel regression (predict.gradient_descent_mse, t = None) -------- */
 /* Factor A = K + lambda I = L L^T in FP32 (predict.py:1224-1258 with

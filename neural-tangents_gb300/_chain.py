@@ -10,8 +10,7 @@ in one CTA with nothing but the readout written to HBM. The readout is
 GlobalAvgPool (after any number of AvgPool(2, 2)), AvgPool(2, 2) down to 1x1
 followed by Flatten, or Flatten right after the last segment. The activation
 rules need the per-sample pre-activation variances of every conv layer; those
-come from the per-sample chain, run with the materialised layer kernels
-(N samples instead of N1*N2 pairs). Layers after the readout run through the
+come from a kernel of their own (ntg_chain_vars), one CTA per sample. Layers after the readout run through the
 ordinary layer rules on [N1, N2] kernels. Anything else falls back to the
 layer-by-layer path.
 """
@@ -28,7 +27,6 @@ from .kernel import Kernel
 from .stax import Padding, _Ctx, _act_struct, _affine_struct
 
 S0 = 32
-SELF_CHUNK = 128
 
 
 @dataclasses.dataclass
@@ -151,53 +149,21 @@ def _program(plan: ChainPlan, channels: int, ctx: _Ctx) -> L.Chain:
 
 def self_chain(x: torch.Tensor, plan: ChainPlan, ctx: _Ctx):
     """Per-sample kernels through the chain: (variance maps [N, total], readout cov [N])."""
-    n = x.shape[0]
-    total = sum((S0 >> sgi) ** 2 * plan.nconv[sgi] for sgi in range(plan.nseg))
-    var = torch.empty((n, max(total, 1)), device=x.device, dtype=torch.float32)
-    covr = torch.empty((n,), device=x.device, dtype=torch.float32)
-    for c0 in range(0, n, SELF_CHUNK):
-        xc = x[c0:c0 + SELF_CHUNK].contiguous()
-        m = xc.shape[0]
-        cov = O.input_fs(xc, None)
-        off = 0
-        li = 0
-        S = S0
-        for sgi in range(plan.nseg):
-            for _ in range(plan.nconv[sgi]):
-                p, act, cin = plan.convs[li]
-                fan = cin * 9 / p['s'][0] if p['parameterization'] == 'standard' else None
-                aff = _affine_struct(p['W_std'], p['b_std'], p['parameterization'], fan)
-                pre, _ = O.conv_fs(cov, None, m, 0, S, S, 3, 3, 1, 1, 1, 1, S, S, False, aff,
-                                   O.NO_ACT, O.NO_VAR, O.NO_VAR, False, (m,))
-                d = torch.diagonal(torch.diagonal(pre, dim1=1, dim2=2), dim1=1, dim2=2)
-                var[c0:c0 + m, off:off + S * S].copy_(d.reshape(m, S * S))
-                if act is not None:
-                    v = O.var_view(pre, False)
-                    cov, _ = O.affine_act(pre, None, m, 0, S, S, False, False, O.IDENTITY_AFFINE,
-                                          _act_struct(act, ctx), v, v, False)
-                else:
-                    cov = pre
-                off += S * S
-                li += 1
-            if sgi < plan.nseg - 1:
-                cov = O.pool(cov, m, S, S, 2, 2, 2, 2, 0, 0, S // 2, S // 2, False, False, True,
-                             False, (m, S // 2, S // 2, S // 2, S // 2))
-                S //= 2
-        if plan.readout == 0:
-            covr[c0:c0 + m] = O.global_pool(cov, 1, True, 1.)
-        else:
-            covr[c0:c0 + m] = O.flatten_fs(cov, 1, S, S)
-    return var, covr
+    pg = _program(plan, x.shape[-1], ctx)
+    x = x.contiguous()
+    var = O.chain_vars(pg, x)
+    return var, O.chain_fwd_self(pg, x, var)
 
 
 def try_fused(kfn, x1: torch.Tensor, x2: Optional[torch.Tensor], diagonal_spatial: bool,
-              compute_ntk: bool, ctx: _Ctx, compare: bool = True) -> Optional[Kernel]:
-    """The fused chain's Kernel, or None for another network; compare: x1_is_x2 is wanted
-    (an element-wise comparison of x1 and x2), else it says whether x2 was left out."""
+              compute_ntk: bool, ctx: _Ctx, whole: bool = True) -> Optional[Kernel]:
+    """The fused chain's Kernel, or None for another network; whole: every field of it is
+    wanted, x1_is_x2 (an element-wise comparison of x1 and x2) and the per-sample kernels
+    too, else nngp and ntk are."""
     plan = plan_chain(kfn.specs, tuple(x1.shape), diagonal_spatial)
     if plan is None or (x2 is not None and tuple(x2.shape[1:]) != tuple(x1.shape[1:])):
         return None
-    k = run_fused(plan, x1, x2, ctx, x1_is_x2=None if compare else x2 is None)
+    k = run_fused(plan, x1, x2, ctx, x1_is_x2=None if whole else x2 is None, covs=whole)
     k = kfn.apply_kernel(k, ctx, specs=plan.post)
     if not compute_ntk:
         k = k.replace(ntk=None)
@@ -206,15 +172,21 @@ def try_fused(kfn, x1: torch.Tensor, x2: Optional[torch.Tensor], diagonal_spatia
 
 def run_fused(plan: ChainPlan, x1: torch.Tensor, x2: Optional[torch.Tensor], ctx: _Ctx,
               out: Optional[tuple] = None, rows=None, cols=None, selfs=None,
-              x1_is_x2: Optional[bool] = None) -> Kernel:
+              x1_is_x2: Optional[bool] = None, covs: bool = True) -> Kernel:
     """Readout Kernel of the chain for all pairs of x1 x x2 (x2 None: x1 x x1).
 
     ``x1_is_x2`` given skips the element-wise comparison of x1 and x2 (a host
-    synchronisation, not allowed while a CUDA graph is being captured)."""
+    synchronisation, not allowed while a CUDA graph is being captured). covs=False: nobody
+    reads cov1 and cov2, which take the self pairs of a block (x1, x2); the layers after the
+    readout do when there is an activation among them."""
     pg = _program(plan, x1.shape[-1], ctx)
+    covs = covs or any(s.kind == 'act' for s in plan.post)
+    cov1 = cov2 = None
     if selfs is None:
-        var1, cov1 = self_chain(x1, plan, ctx)
-        var2, cov2 = (var1, None) if x2 is None else self_chain(x2, plan, ctx)
+        if x2 is None:
+            var1 = var2 = O.chain_vars(pg, x1)
+        else:
+            var1, var2 = O.chain_vars(pg, x1, x2)
     else:
         var1, cov1, var2, cov2 = selfs
     xb = x1 if x2 is None else x2
@@ -229,6 +201,16 @@ def run_fused(plan: ChainPlan, x1: torch.Tensor, x2: Optional[torch.Tensor], ctx
         O.chain_fwd_sym(pg, x1, 0, n1, 0, n1, var1, out_q, out_t, n2)
     else:
         O.chain_fwd(pg, x1, xb, 0, n1, 0, n2, var1, var2, out_q, out_t, n2)
+    if cov1 is None:
+        # the readout kernel of a sample with itself: out_q's diagonal, or its own self pairs
+        # (nobody reads them: zeros keep the Kernel's shape)
+        if x2 is None:
+            cov1 = torch.diagonal(out_q) if plan.post else torch.diagonal(out_q).clone()
+        elif covs:
+            cov1, cov2 = O.chain_fwd_self(pg, x1, var1), O.chain_fwd_self(pg, xb, var2)
+        else:
+            none = out_q.new_zeros(max(n1, n2))
+            cov1, cov2 = none[:n1], none[:n2]
     shape1 = tuple(x1.shape)
     shape2 = tuple(xb.shape)
     for s in plan.spatial:

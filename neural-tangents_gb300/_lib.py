@@ -92,6 +92,11 @@ SIGNATURES = {
                        _I64], C.c_int),
     'ntg_chain_fwd_sym': ([_P, C.POINTER(Chain), _P, _I64, _I64, _I64, _I64, _P, _P, _P, _I64],
                           C.c_int),
+    'ntg_chain_workspace_bytes': ([], C.c_size_t),
+    'ntg_chain_vars': ([_P, C.POINTER(Chain), _P, _I64, _P, _P, _I64, _P, _P, C.c_size_t],
+                       C.c_int),
+    'ntg_chain_fwd_ws': ([_P, C.POINTER(Chain), _P, _P, _I64, _I64, _I64, _I64, _P, _P, _P, _P,
+                          _I64, _I32, _P, C.c_size_t], C.c_int),
     'ntg_act_bwd': ([_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I32, Act, Var, Var, _P,
                      _P], C.c_int),
     'ntg_act_pool_bwd': ([_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, Act, Var, Var, _P,

@@ -221,17 +221,42 @@ def flatten_fs(x: torch.Tensor, bnd: int, a: int, c: int) -> torch.Tensor:
     return out
 
 
-def chain_fwd(prog: L.Chain, x1, x2, r0, n1, c0, n2, var1, var2, out_q, out_t, ld_out):
+def chain_vars(prog: L.Chain, x1, x2=None):
+    """Pre-activation variance maps [N, var_stride] of every conv layer of the chain: of x1, or
+    (of x1, of x2)."""
     import ctypes
-    L.call('ntg_chain_fwd', L.stream(), ctypes.byref(prog), L.ptr(x1), L.ptr(x2), r0, n1, c0, n2,
-           L.ptr(var1), L.ptr(var2), out_q.data_ptr(), None if out_t is None else out_t.data_ptr(),
-           ld_out)
+    nbytes = int(L.load().ntg_chain_workspace_bytes())
+    ws = torch.empty((nbytes,), device=x1.device, dtype=torch.uint8)
+    var = [None if x is None else torch.empty((x.shape[0], prog.var_stride), device=x1.device,
+                                              dtype=torch.float32) for x in (x1, x2)]
+    L.call('ntg_chain_vars', L.stream(), ctypes.byref(prog), L.ptr(x1), x1.shape[0],
+           L.ptr(var[0]), L.ptr(x2), 0 if x2 is None else x2.shape[0], L.ptr(var[1]),
+           ws.data_ptr(), nbytes)
+    return var[0] if x2 is None else tuple(var)
+
+
+def _chain(prog, x1, x2, r0, n1, c0, n2, var1, var2, out_q, out_t, ld_out, mode):
+    import ctypes
+    nbytes = int(L.load().ntg_chain_workspace_bytes())
+    ws = torch.empty((nbytes,), device=x1.device, dtype=torch.uint8)
+    L.call('ntg_chain_fwd_ws', L.stream(), ctypes.byref(prog), L.ptr(x1), L.ptr(x2), r0, n1, c0,
+           n2, L.ptr(var1), L.ptr(var2), out_q.data_ptr(),
+           None if out_t is None else out_t.data_ptr(), ld_out, mode, ws.data_ptr(), nbytes)
+
+
+def chain_fwd(prog: L.Chain, x1, x2, r0, n1, c0, n2, var1, var2, out_q, out_t, ld_out):
+    _chain(prog, x1, x2, r0, n1, c0, n2, var1, var2, out_q, out_t, ld_out, 0)
 
 
 def chain_fwd_sym(prog: L.Chain, x, r0, n1, c0, n2, var, out_q, out_t, ld_out):
     """Pairs (r0.., c0..) of x with itself, each written at (i, j) and (j, i) of the
     whole kernel out [., ld_out]; the tile is diagonal (only i <= j evaluated) or
     has disjoint row and column ranges."""
-    import ctypes
-    L.call('ntg_chain_fwd_sym', L.stream(), ctypes.byref(prog), L.ptr(x), r0, n1, c0, n2,
-           L.ptr(var), out_q.data_ptr(), None if out_t is None else out_t.data_ptr(), ld_out)
+    _chain(prog, x, x, r0, n1, c0, n2, var, var, out_q, out_t, ld_out, 1)
+
+
+def chain_fwd_self(prog: L.Chain, x, var):
+    """nngp [N] of the pairs (x[i], x[i])."""
+    out = torch.empty((x.shape[0],), device=x.device, dtype=torch.float32)
+    _chain(prog, x, x, 0, x.shape[0], 0, 1, var, var, out, None, 1, 2)
+    return out

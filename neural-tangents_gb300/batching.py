@@ -5,8 +5,7 @@ signature that evaluates the N1 x N2 kernel in tiles of at most
 ``batch_size`` rows and columns. Unlike the reference (batching.py:647-679),
 N1 and N2 need not be multiples of ``batch_size``: the edge tiles are ragged.
 For networks the fused chain kernel covers, the whole grid is one launch of
-that kernel (the per-sample chains run once per sample, in ``batch_size``
-chunks) and ``batch_size`` only bounds the per-sample working set.
+that kernel whatever ``batch_size`` (its working set does not grow with N).
 """
 from __future__ import annotations
 
@@ -109,12 +108,7 @@ def _forward_grid(kernel_fn, x1t, x2t, bs, precision):
     ctx = _Ctx(precision)
     plan = _chain.plan_chain(kernel_fn.specs, tuple(x1t.shape), bool(kernel_fn.diagonal))
     if plan is not None and (x2t is None or x2t.shape[1:] == x1t.shape[1:]):
-        old = _chain.SELF_CHUNK
-        _chain.SELF_CHUNK = max(1, min(old, bs))
-        try:
-            k = _chain.run_fused(plan, x1t, x2t, ctx, x1_is_x2=x2t is None)
-        finally:
-            _chain.SELF_CHUNK = old
+        k = _chain.run_fused(plan, x1t, x2t, ctx, x1_is_x2=x2t is None, covs=False)
         return kernel_fn.apply_kernel(k, ctx, specs=plan.post)
     xb = x1t if x2t is None else x2t
     rows = []
@@ -170,14 +164,9 @@ def batch(kernel_fn, batch_size: int = 0, device_count: int = -1, store_on_devic
         if isinstance(kernel_fn, KernelFn) and not ds:
             plan = _chain.plan_chain(kernel_fn.specs, tuple(x1t.shape), False)
             if plan is not None and (x2t is None or x2t.shape[1:] == x1t.shape[1:]):
-                old = _chain.SELF_CHUNK
-                _chain.SELF_CHUNK = max(1, min(old, bs))
-                try:
-                    k = _chain.run_fused(
-                        plan, x1t, x2t, ctx,
-                        x1_is_x2=None if names is None or 'x1_is_x2' in names else x2t is None)
-                finally:
-                    _chain.SELF_CHUNK = old
+                whole = names is None or not set(names) <= {'nngp', 'ntk'}
+                k = _chain.run_fused(plan, x1t, x2t, ctx,
+                                     x1_is_x2=None if whole else x2t is None, covs=whole)
                 k = kernel_fn.apply_kernel(k, ctx, specs=plan.post)
                 if names is not None and 'ntk' not in names:
                     k = k.replace(ntk=None)
@@ -261,7 +250,6 @@ class CapturedBatch:
                 x2_shape is not None and tuple(x2_shape[1:]) != tuple(x1_shape[1:])):
             raise NotImplementedError('CapturedBatch needs a network on the fused chain path')
         self.kernel_fn, self.precision = kernel_fn, precision
-        self.bs = batch_size or max(x1_shape[0], (x2_shape or x1_shape)[0])
         self.x1 = torch.zeros(tuple(x1_shape), device=dev)
         self.x2 = None if x2_shape is None else torch.zeros(tuple(x2_shape), device=dev)
         side = torch.cuda.Stream()
@@ -276,12 +264,8 @@ class CapturedBatch:
 
     def _run(self):
         ctx = _Ctx(self.precision)
-        old = _chain.SELF_CHUNK
-        _chain.SELF_CHUNK = max(1, min(old, self.bs))
-        try:
-            k = _chain.run_fused(self.plan, self.x1, self.x2, ctx, x1_is_x2=self.x2 is None)
-        finally:
-            _chain.SELF_CHUNK = old
+        k = _chain.run_fused(self.plan, self.x1, self.x2, ctx, x1_is_x2=self.x2 is None,
+                             covs=False)
         k = self.kernel_fn.apply_kernel(k, ctx, specs=self.plan.post)
         return _select(k, self.names, self.single)
 

@@ -1,0 +1,14 @@
+// Instances of the fused chain kernel for any segment shape with ABRelu and Erf activations.
+#include "ntg_chain_kernel.cuh"
+
+namespace ntg {
+
+cudaError_t launch_chain_any(const ntg_chain_t& pg, const ChainArgs& a) {
+  switch (pg.nconv[0]) {
+    case 1: return launch_chain_k<1, 0, 0, 0>(pg, a);
+    case 2: return launch_chain_k<2, 0, 0, 0>(pg, a);
+    default: return launch_chain_k<3, 0, 0, 0>(pg, a);
+  }
+}
+
+}  // namespace ntg

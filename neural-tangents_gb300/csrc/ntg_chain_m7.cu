@@ -1,0 +1,10 @@
+// Instances of the fused chain kernel for segments of 2, 2, 2 convs.
+#include "ntg_chain_kernel.cuh"
+
+namespace ntg {
+
+cudaError_t launch_chain_myrtle7(bool relu_only, const ntg_chain_t& pg, const ChainArgs& a) {
+  return launch_myrtle<2, 2, 2>(relu_only, pg, a);
+}
+
+}  // namespace ntg

@@ -88,9 +88,11 @@ __device__ __forceinline__ float prod_minus_sq(float v1, float v2, float q, int 
   return d;
 }
 
+// One special-function instruction; inputs below 2^-126 count as zero (handling them took
+// three more instructions per root).
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 
@@ -157,16 +159,15 @@ __device__ __forceinline__ P2 sub2(P2 a, P2 b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
   return d;
 }
-__device__ __forceinline__ P2 mul2(P2 a, P2 b) {
-  P2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-  return d;
-}
 __device__ __forceinline__ P2 fma2(P2 a, P2 b, P2 c) {
   P2 d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
   return d;
 }
+// A product rounded by itself: as an explicit fused multiply-add with zero, because ptxas
+// contracts mul.rn.f32x2 with an add or subtract that follows, and var1 var2 - q^2 of a self
+// pair would not be 0.
+__device__ __forceinline__ P2 mul2(P2 a, P2 b) { return fma2(a, b, p2s(0.f)); }
 
 // Per-layer activation constants, computed once per layer (uniform).
 struct ActC {
@@ -286,11 +287,12 @@ __device__ __forceinline__ void act_apply(const ActC& c, float& q, float& t, flo
 
 // The ABRelu branch of act_apply (do_stabilize off) on a packed pair, with
 // the same operation sequence per lane. COMP: -1 reads c.comp, 0 / 1 fix the
-// plain / compensated var1 var2 - q^2 at compile time.
-template <int COMP = -1>
-__device__ __forceinline__ void abrelu2(const ActC& c, P2& q, P2& t, P2 v1, P2 v2, P2 sv1,
-                                        P2 sv2) {
-  const P2 n = mul2(sv1, sv2);
+// plain / compensated var1 var2 - q^2 at compile time. ROOTS: n = sqrt(v1) sqrt(v2) is given;
+// else it is sqrt(v1 v2 + 2^-126), which has no zero to look out for: where both variances
+// and q vanish the angle counts as 0 instead of pi / 2, which only ntk' = ntk dot would see,
+// so this form is for kernels whose ntk vanishes with the variances.
+template <int COMP, bool ROOTS>
+__device__ __forceinline__ void abrelu2_n(const ActC& c, P2& q, P2& t, P2 v1, P2 v2, P2 n) {
   const P2 pr = mul2(v1, v2), qq = mul2(q, q);
   P2 d = sub2(pr, qq);
   if (COMP == 1 || (COMP < 0 && c.comp)) {
@@ -298,10 +300,15 @@ __device__ __forceinline__ void abrelu2(const ActC& c, P2& q, P2& t, P2 v1, P2 v
     const P2 pe = fma2(v1, v2, mul2(pr, m1)), qe = fma2(q, q, mul2(qq, m1));
     d = add2(d, sub2(pe, qe));
   }
+  if (!ROOTS) n = fma2(v1, v2, p2s(1.17549435e-38f));
   float d0, d1, q0, q1, n0, n1;
   p2u(d, d0, d1);
   p2u(q, q0, q1);
   p2u(n, n0, n1);
+  if (!ROOTS) {
+    n0 = sqrt_approx(n0);
+    n1 = sqrt_approx(n1);
+  }
   const float s0 = sqrt_approx(fmaxf(d0, 0.f)), s1 = sqrt_approx(fmaxf(d1, 0.f));
   const float den0 = n0 + fabsf(q0), den1 = n1 + fabsf(q1);
   const P2 sp = p2(s0, s1);
@@ -321,11 +328,24 @@ __device__ __forceinline__ void abrelu2(const ActC& c, P2& q, P2& t, P2 v1, P2 v
   p2u(dneg, a0, a1);
   p2u(dpos, b0, b1);
   float dot0 = (q0 < 0.f) ? a0 : b0, dot1 = (q1 < 0.f) ? a1 : b1;
-  dot0 = (den0 == 0.f) ? c.h_zero : dot0;
-  dot1 = (den1 == 0.f) ? c.h_zero : dot1;
+  if (ROOTS) {
+    dot0 = (den0 == 0.f) ? c.h_zero : dot0;
+    dot1 = (den1 == 0.f) ? c.h_zero : dot1;
+  }
   const P2 dot = p2(dot0, dot1);
   q = fma2(p2s(c.factor), sp, mul2(dot, q));
   t = mul2(t, dot);
+}
+
+template <int COMP = -1>
+__device__ __forceinline__ void abrelu2(const ActC& c, P2& q, P2& t, P2 v1, P2 v2, P2 sv1,
+                                        P2 sv2) {
+  abrelu2_n<COMP, true>(c, q, t, v1, v2, mul2(sv1, sv2));
+}
+
+template <int COMP = -1>
+__device__ __forceinline__ void abrelu2_v(const ActC& c, P2& q, P2& t, P2 v1, P2 v2) {
+  abrelu2_n<COMP, false>(c, q, t, v1, v2, v1);
 }
 
 // sqrt(var) as every kernel of the library evaluates it (one approximate

@@ -732,7 +732,8 @@ class KernelFn:
                 vals = tuple(getattr(k, n) for n in names)
                 return vals[0] if single is not None else analytic_kernel(names, vals)
             compare = names is None or 'x1_is_x2' in names
-            k = _chain.try_fused(self, x1, x2t, ds, compute_ntk, ctx, compare)
+            whole = names is None or not set(names) <= {'nngp', 'ntk'}
+            k = _chain.try_fused(self, x1, x2t, ds, compute_ntk, ctx, whole)
             if k is None:
                 cnone = bool(self.specs) and self.specs[0].channel_axis_none
                 first = next((sp for sp in self.specs if sp.kind != 'identity'), None)
