@@ -279,6 +279,28 @@ int ntg_chain_fwd_ws(void* stream, const ntg_chain_t* prog, const float* x1, con
                      int64_t r0, int64_t n1, int64_t c0, int64_t n2, const float* var1,
                      const float* var2, float* out_q, float* out_t, int64_t ld_out, int32_t mode,
                      void* workspace, size_t workspace_bytes);
+/* Whole conv network on diagonal-spatial kernels (linear.py:3381-3437): inputs x1 [N1, a, c, K],
+ * x2 [N2, a, c, K] (NULL: x1 with itself, n2 == n1, the pairs i <= j evaluated and mirrored);
+ * each layer a stride-1, zero-padded fh x fw window (a Dense is 1 x 1) to ao x co positions,
+ * its affine rule and activation; then sum over the positions / divisor * scale. Writes nngp
+ * (and ntk unless NULL) [N1, N2], the per-sample readouts cov1 [N1], cov2 [N2] and, as
+ * scratch, the layers' variance maps var1 [N1, var_stride], var2 [N2, var_stride]. The caller
+ * sets var_off to the running sum of ao * co and var_stride to their total; plane is ignored. */
+enum { NTG_DS_MAX_LAYERS = 16 };
+typedef struct {
+  int32_t fh, fw, ph, pw, ao, co, var_off;
+  ntg_affine_t aff;
+  ntg_act_t act;
+} ntg_ds_layer_t;
+typedef struct {
+  int32_t nlayers, a, c, channels;
+  int32_t var_stride, plane;
+  float divisor, scale;
+  ntg_ds_layer_t layer[NTG_DS_MAX_LAYERS];
+} ntg_ds_chain_t;
+int ntg_ds_chain(void* stream, const ntg_ds_chain_t* prog, const float* x1, const float* x2,
+                 int64_t n1, int64_t n2, float* var1, float* var2, float* cov1, float* cov2,
+                 float* out_q, float* out_t);
 
 /* ---- kernel regression (predict.gradient_descent_mse, t = None) -------- */
 /* Factor A = K + lambda I = L L^T in FP32 (predict.py:1224-1258 with

@@ -24,7 +24,7 @@ import torch
 from . import _lib as L
 from . import _ops as O
 from .kernel import Kernel
-from .stax import Padding, _Ctx, _act_struct, _affine_struct
+from .stax import Padding, _Ctx, _act_struct, _affine_struct, _conv_geometry
 
 S0 = 32
 
@@ -220,3 +220,91 @@ def run_fused(plan: ChainPlan, x1: torch.Tensor, x2: Optional[torch.Tensor], ctx
                   else bool(x1_is_x2), is_gaussian=plan.is_gaussian,
                   is_reversed=False, is_input=False, diagonal_batch=True, diagonal_spatial=False,
                   shape1=shape1, shape2=shape2)
+
+
+# ---------------------------------------------------------------------------
+# Conv networks on diagonal-spatial kernels (ntg_ds_chain)
+# ---------------------------------------------------------------------------
+
+DS_MAX_SMEM = 100 * 1024  # two CTAs per SM; larger images go layer by layer
+
+
+def plan_ds(specs, x_shape, ctx: _Ctx):
+    """(program, layers after the readout, is_gaussian) of a serial network whose layers up to a
+    Flatten / GlobalAvgPool / GlobalSumPool readout are stride-1 zero-padded Conv, Dense and
+    activations, on [N, A, K] or [N, A, C, K] inputs; None for another network."""
+    if len(x_shape) not in (3, 4):
+        return None
+    specs = [s for s in specs if s.kind != 'identity']
+    ridx = next((i for i, s in enumerate(specs) if s.kind in ('gpool', 'flatten')), None)
+    if not ridx or ridx > 2 * L.DS_MAX_LAYERS or specs[0].kind == 'act':
+        return None
+    a, c = x_shape[1], x_shape[2] if len(x_shape) == 4 else 1
+    pg = L.DsChain()
+    pg.a, pg.c, pg.channels = a, c, x_shape[-1]
+    shape, n, off, gaussian, plane = tuple(x_shape), 0, 0, False, a * c
+    for s in specs[:ridx]:
+        p = s.params
+        if s.kind == 'act':
+            if not gaussian or p.get('do_stabilize'):
+                return None
+            pg.layer[n - 1].act = _act_struct(p, ctx)
+            gaussian = False
+            continue
+        if s.kind not in ('conv', 'dense') or n == L.DS_MAX_LAYERS:
+            return None
+        fh = fw = 1
+        ph, pw, ao, co = 0, 0, a, c
+        if s.kind == 'conv':
+            nsp = len(p['filter_shape'])
+            if nsp != len(x_shape) - 2 or p['padding'] == Padding.CIRCULAR or \
+                    any(st != 1 for st in p['strides']):
+                return None
+            fh, fw, _, _, ph, pw, ao, co = _conv_geometry(p, a, c, nsp == 2)
+        fan = None
+        if p['parameterization'] == 'standard':
+            fan = shape[-1] * fh * fw / p['s'][0]
+        if min(ao, co) < 1 or ph >= fh or pw >= fw:
+            return None
+        ly = pg.layer[n]
+        ly.fh, ly.fw, ly.ph, ly.pw, ly.ao, ly.co, ly.var_off = fh, fw, ph, pw, ao, co, off
+        ly.aff = _affine_struct(p['W_std'], p['b_std'], p['parameterization'], fan)
+        ly.act = O.NO_ACT
+        plane = max(plane, a * co)
+        off += ao * co
+        a, c, n, gaussian = ao, co, n + 1, True
+        shape = s.shape_fn(shape)
+    ro = specs[ridx]
+    pg.nlayers, pg.var_stride = n, off
+    flatten = ro.kind == 'flatten'
+    average = flatten or ro.params['pool'] == 'avg'
+    # linear.py:1771-1801 on diagonal kernels: the mean of the positions, divided by their
+    # number once more for GlobalAvgPool
+    pg.divisor = float(a * c) if average else 1.
+    pg.scale = 1. / (a * c) if average and not flatten else 1.
+    if 4 * (pg.channels * pg.a * pg.c + off + 4 * plane) > DS_MAX_SMEM or pg.c > 512 or \
+            pg.a > 4096:
+        return None
+    return pg, specs[:ridx + 1], specs[ridx + 1:], gaussian and not flatten
+
+
+def try_ds(kfn, x1: torch.Tensor, x2: Optional[torch.Tensor], compute_ntk: bool, ctx: _Ctx,
+           whole: bool) -> Optional[Kernel]:
+    """The Kernel of a network plan_ds covers, on diagonal-spatial kernels; whole: see
+    try_fused."""
+    if x2 is not None and x2.shape[1:] != x1.shape[1:]:
+        return None
+    plan = plan_ds(kfn.specs, tuple(x1.shape), ctx)
+    if plan is None:
+        return None
+    pg, spatial, post, gaussian = plan
+    q, t, c1, c2 = O.ds_chain(pg, x1, x2, compute_ntk)
+    shape1 = tuple(x1.shape)
+    shape2 = shape1 if x2 is None else tuple(x2.shape)
+    for s in spatial:
+        shape1, shape2 = s.shape_fn(shape1), s.shape_fn(shape2)
+    same = x2 is None or (whole and x1.shape == x2.shape and bool(torch.equal(x1, x2)))
+    k = Kernel(nngp=q, ntk=t, cov1=c1, cov2=c2, x1_is_x2=same, is_gaussian=gaussian,
+               is_reversed=False, is_input=False, diagonal_batch=True,
+               diagonal_spatial=spatial[-1].kind != 'flatten', shape1=shape1, shape2=shape2)
+    return kfn.apply_kernel(k, ctx, specs=post)

@@ -22,6 +22,7 @@ NTG_PAD_ZERO, NTG_PAD_CIRCULAR = 0, 1
 NTG_TUNE_STENCIL_RING = 0
 CHAIN_MAX_SEG, CHAIN_MAX_LAYERS = 4, 16
 FLAT_MAX_LAYERS = 32
+DS_MAX_LAYERS = 16
 
 ERRORS = {
     1: 'invalid argument', 2: 'CUDA error', 3: 'unsupported', 4: 'not positive definite',
@@ -53,6 +54,18 @@ class Chain(C.Structure):
                 ('readout', C.c_int32), ('nconv', C.c_int32 * CHAIN_MAX_SEG),
                 ('aff', Affine * CHAIN_MAX_LAYERS), ('act', Act * CHAIN_MAX_LAYERS),
                 ('var_off', C.c_int64 * CHAIN_MAX_LAYERS), ('var_stride', C.c_int64)]
+
+
+class DsLayer(C.Structure):
+    _fields_ = [('fh', C.c_int32), ('fw', C.c_int32), ('ph', C.c_int32), ('pw', C.c_int32),
+                ('ao', C.c_int32), ('co', C.c_int32), ('var_off', C.c_int32), ('aff', Affine),
+                ('act', Act)]
+
+
+class DsChain(C.Structure):
+    _fields_ = [('nlayers', C.c_int32), ('a', C.c_int32), ('c', C.c_int32),
+                ('channels', C.c_int32), ('var_stride', C.c_int32), ('plane', C.c_int32),
+                ('divisor', C.c_float), ('scale', C.c_float), ('layer', DsLayer * DS_MAX_LAYERS)]
 
 
 _P, _I64, _I32, _F = C.c_void_p, C.c_int64, C.c_int32, C.c_float
@@ -97,6 +110,7 @@ SIGNATURES = {
                        C.c_int),
     'ntg_chain_fwd_ws': ([_P, C.POINTER(Chain), _P, _P, _I64, _I64, _I64, _I64, _P, _P, _P, _P,
                           _I64, _I32, _P, C.c_size_t], C.c_int),
+    'ntg_ds_chain': ([_P, C.POINTER(DsChain), _P, _P, _I64, _I64, _P, _P, _P, _P, _P, _P], C.c_int),
     'ntg_act_bwd': ([_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _I32, Act, Var, Var, _P,
                      _P], C.c_int),
     'ntg_act_pool_bwd': ([_P, _P, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, Act, Var, Var, _P,

@@ -221,6 +221,23 @@ def flatten_fs(x: torch.Tensor, bnd: int, a: int, c: int) -> torch.Tensor:
     return out
 
 
+def ds_chain(prog: L.DsChain, x1, x2, want_t: bool):
+    """nngp, ntk [N1, N2], cov1, cov2 after the readout of a conv network on diagonal-spatial
+    kernels (x2 None: x1 with itself, cov2 None)."""
+    import ctypes
+    n1, n2 = x1.shape[0], (x1 if x2 is None else x2).shape[0]
+
+    def new(*shape):
+        return torch.empty(shape, device=x1.device, dtype=torch.float32)
+
+    q, t = new(n1, n2), new(n1, n2) if want_t else None
+    v1, c1 = new(n1, prog.var_stride), new(n1)
+    v2, c2 = (None, None) if x2 is None else (new(n2, prog.var_stride), new(n2))
+    L.call('ntg_ds_chain', L.stream(), ctypes.byref(prog), L.ptr(x1), L.ptr(x2), n1, n2, L.ptr(v1),
+           L.ptr(v2), L.ptr(c1), L.ptr(c2), L.ptr(q), L.ptr(t))
+    return q, t, c1, c2
+
+
 def chain_vars(prog: L.Chain, x1, x2=None):
     """Pre-activation variance maps [N, var_stride] of every conv layer of the chain: of x1, or
     (of x1, of x2)."""
