@@ -1098,9 +1098,11 @@ extern "C" int ntg_gemm_ex(void* stream, const float* a, const float* b, float* 
                            int32_t accumulate) {
   NTG_REQUIRE(a && b && c && m > 0 && n > 0 && k > 0, "ntg_gemm_ex: bad arguments");
   NTG_REQUIRE(ceil_div(m, 64) <= 65535, "ntg_gemm_ex: m too large");
-  dim3 grid((unsigned)ceil_div(n, 64), (unsigned)ceil_div(m, 64));
-  gemm_ex_kernel<<<grid, 256, 0, as_stream(stream)>>>(a, b, c, m, n, k, trans_a, alpha,
-                                                      accumulate);
+  if (!gemm_small(as_stream(stream), a, b, c, m, n, k, trans_a, alpha, accumulate)) {
+    dim3 grid((unsigned)ceil_div(n, 64), (unsigned)ceil_div(m, 64));
+    gemm_ex_kernel<<<grid, 256, 0, as_stream(stream)>>>(a, b, c, m, n, k, trans_a, alpha,
+                                                        accumulate);
+  }
   note_launch();
   return check_launch("ntg_gemm_ex");
 }

@@ -30,6 +30,10 @@ int gram_tc(cudaStream_t stream, const float* x1, const float* x2, int64_t n1, i
             int64_t d, float* out, void* workspace, size_t ws_bytes);
 size_t gram_tc_workspace(int64_t n1, int64_t n2, int64_t d);
 
+// Small FP32 products, defined in ntg_flat.cu; false: not a small one, nothing was launched.
+bool gemm_small(cudaStream_t s, const float* a, const float* b, float* c, int64_t m, int64_t n,
+                int64_t k, bool trans_a, float alpha, bool accumulate);
+
 #define NTG_REQUIRE(cond, msg)                                   \
   do {                                                           \
     if (!(cond)) return ::ntg::fail(NTG_ERR_INVALID_ARG, (msg)); \

@@ -7,15 +7,14 @@
 // to the others, so they stay exact unit vectors) is split into 32-wide blocks.
 // A sweep pairs every two blocks once, in the round-robin order of a tournament
 // (nb - 1 rounds of nb / 2 disjoint pairs). In a round:
-//   jacobi_inner_kernel   one CTA per pair runs up to two sweeps of cyclic parallel
+//   jacobi_inner_kernel   one CTA per pair runs a sweep of cyclic parallel
 //                         Jacobi on the 64 x 64 matrix of its two blocks in shared
 //                         memory and writes the accumulated rotation U (64 x 64);
 //                         what couplings remain stay in A for the next sweeps;
 //   jacobi_apply_kernel   A <- U^T A U tile by tile (a 64 x 64 tile of A couples
-//                         two pairs and depends only on their rotations);
-//   jacobi_apply_v_kernel V <- V U.
+//                         two pairs and depends only on their rotations) and V <- V U.
 // After each sweep off(A) / ||A||_F is read back (one 16-byte copy) and the sweeps
-// stop below the tolerance. Eigenvalues are the diagonal of the final A, not sorted.
+// stop below the tolerance (or when rounding stops them). Eigenvalues are the diagonal of the final A, not sorted.
 // FP32 rounding accumulates over the rounds (about 1e-5 relative at n = 1000), so the
 // pairs are then refined with double-float products (see the refinement below).
 #include <cmath>
@@ -29,7 +28,6 @@ namespace {
 
 constexpr int JB = 32;        // block width
 constexpr int JP = 2 * JB;    // a pair: 64 indices
-constexpr int JPS = JP + 1;
 
 __host__ __device__ __forceinline__ void rr_pair(int nplayers, int round, int k, int& a, int& b) {
   // circle method: player nplayers - 1 fixed, the others rotate
@@ -52,221 +50,255 @@ __device__ __forceinline__ int pair_index(int pa, int pb, int l) {
   return (l < JB ? pa : pb) * JB + (l & (JB - 1));
 }
 
-// Rotation (c, s) that zeroes s_pq of [[app, apq], [apq, aqq]] (Golub & Van Loan 8.5.1);
-// (1, 0) when the coupling is negligible.
-__device__ __forceinline__ void sym_schur2(float app, float aqq, float apq, float tiny, float& c,
-                                          float& s) {
-  if (fabsf(apq) <= tiny) {
-    c = 1.f;
-    s = 0.f;
-    return;
-  }
-  const float tau = (aqq - app) / (2.f * apq);
-  const float t = copysignf(1.f, tau) / (fabsf(tau) + sqrtf(fmaf(tau, tau, 1.f)));
-  c = 1.f / sqrtf(fmaf(t, t, 1.f));
-  s = t * c;
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
-// One CTA per pair of blocks: S = A[idx, idx] (64 x 64), rotated in place by cyclic
-// parallel Jacobi (32 disjoint rotations per round, 63 rounds per sweep) until a sweep
-// leaves no coupling above 1e-5 of its pivots or `inner_sweeps` sweeps ran; U (64 x 64,
+// Rotation (c, s) that zeroes the coupling of [[app, apq], [apq, aqq]] (Golub & Van Loan
+// 8.5.1): t = apq / (h +- sqrt(h^2 + apq^2)), h = (aqq - app) / 2, entries at most 1 in size.
+// The angle may be approximate (the coupling left over is rounding sized); c and s are brought
+// back to c^2 + s^2 = 1 by one Newton step, so that thousands of rotations do not drift.
+__device__ __forceinline__ void sym_schur2(float app, float aqq, float apq, float& c, float& s) {
+  const float h = 0.5f * (aqq - app);
+  const float r = sqrt_approx(fmaf(h, h, apq * apq));
+  const float t = apq * rcp_approx(h + copysignf(r, h));
+  c = rsqrt_approx(fmaf(t, t, 1.f));
+  s = t * c;
+  const float e = 0.5f * fmaf(-s, s, fmaf(-c, c, 1.f));
+  c = fmaf(c, e, c);
+  s = fmaf(s, e, s);
+}
+
+constexpr int kInnerThreads = 512;
+
+// The tournament as a fixed permutation of positions (Brent & Luk): pair k sits at positions
+// 2k, 2k + 1; after a round the player at position i moves to round_move(i), position 0 stays,
+// and after 63 rounds everyone is back.
+__device__ __forceinline__ int round_move(int i) {
+  if (i & 1) return i == 1 ? 2 : i - 2;
+  return i == 0 ? 0 : i == JP - 2 ? JP - 1 : i + 2;
+}
+// Column position -> offset in a stored row: even positions, then odd ones, so that the 32
+// pairs of a row are 32 consecutive words of either half, before and after the move.
+__device__ __forceinline__ int col_slot(int pos) { return (pos & 1) * (JP / 2) + (pos >> 1); }
+
+// One CTA per pair of blocks: S = A[idx, idx] (64 x 64, scaled to entries at most 1), rotated
+// by cyclic parallel Jacobi (32 disjoint rotations per round, 63 rounds per sweep) until a
+// sweep leaves no coupling above 1e-5 of its pivots or `inner_sweeps` sweeps ran; U (64 x 64,
 // row-major) accumulates the rotations.
-__global__ void __launch_bounds__(256)
+//
+// A serial chain of rounds, so a round is built to be short: lane b of every warp computes the
+// rotation of pair b for itself (three loads, three special functions), which spares an
+// exchange through shared memory and its barrier; S is read from one copy and written to the
+// other, already moved to the next round's positions, so that addresses are constants of the
+// thread, accesses free of bank conflicts, and one barrier closes the round; U stays in
+// registers, four rows a warp, a lane's two columns moving to its neighbours by shuffles.
+// Bound by the latency of a round (load, rotation, update, barrier) and the 496 cycles of
+// shared-memory wavefronts and shuffles in it. A sweep takes 30 us; with one warp computing
+// the rotations by IEEE divisions and roots and two barriers a round it was 77 us.
+__global__ void __launch_bounds__(kInnerThreads)
     jacobi_inner_kernel(const float* __restrict__ A, int64_t lda, int nblk, int round,
                         int inner_sweeps, float* __restrict__ Uout, const int* done) {
   if (*done) return;
-  __shared__ float S[JP][JPS];
-  __shared__ float U[JP][JPS];
-  __shared__ float cs[JP / 2][2];
-  __shared__ int pq[JP / 2][2];
-  __shared__ float smax;
+  __shared__ float ism[2 * JP * JP];  // two copies of S
+  __shared__ unsigned s_max;
+  constexpr int N = JP * JP;
   int pa, pb;
   rr_pair(nblk, round, blockIdx.x, pa, pb);
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < JP * JP; idx += blockDim.x) {
-    const int i = idx / JP, j = idx % JP;
-    S[i][j] = A[(int64_t)pair_index(pa, pb, i) * lda + pair_index(pa, pb, j)];
-    U[i][j] = (i == j) ? 1.f : 0.f;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) s_max = 0;
+  __syncthreads();
+  float v[N / kInnerThreads];
+  unsigned m = 0;  // bit patterns of non-negative floats order as they do (NaN above all)
+#pragma unroll
+  for (int e = 0; e < N / kInnerThreads; ++e) {
+    const int idx = tid + kInnerThreads * e, i = idx / JP, j = idx % JP;
+    v[e] = A[(int64_t)pair_index(pa, pb, i) * lda + pair_index(pa, pb, j)];
+    m = max(m, __float_as_uint(fabsf(v[e])));
   }
-  if (tid == 0) smax = 0.f;
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (lane == 0) atomicMax(&s_max, m);
   __syncthreads();
-  if (tid < JP) atomicMax(reinterpret_cast<int*>(&smax), __float_as_int(fabsf(S[tid][tid])));
+  // a power of two near the largest entry; all zero: nothing to rotate
+  const bool zero = s_max == 0;
+  const int ex = min(max(254 - (int)(s_max >> 23), 1), 254);
+  const float scale = __uint_as_float((unsigned)ex << 23);
+#pragma unroll
+  for (int e = 0; e < N / kInnerThreads; ++e) {
+    const int idx = tid + kInnerThreads * e, i = idx / JP, j = idx % JP;
+    ism[i * JP + col_slot(j)] = v[e] * scale;
+  }
   __syncthreads();
+  // the rotation of pair `lane`, the blocks (warp, lane), (warp + 16, lane) of S, and columns
+  // 2 lane, 2 lane + 1 of rows 4 warp .. of U
+  const int dg = 2 * lane * JP + lane;
+  const int ct = col_slot(round_move(2 * lane)), cb = col_slot(round_move(2 * lane + 1));
+  float ut[4], ub[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    ut[u] = 4 * warp + u == 2 * lane ? 1.f : 0.f;
+    ub[u] = 4 * warp + u == 2 * lane + 1 ? 1.f : 0.f;
+  }
   // couplings below this are already zero at float32 resolution of the pair's matrix
-  const float tiny = 1e-9f * smax;
-  for (int sw = 0; sw < inner_sweeps; ++sw) {
-    int rotated = 0;  // this thread's rotations of the sweep (combined below)
+  float dmax = fmaxf(fabsf(ism[dg]), fabsf(ism[dg + JP + JP / 2]));
+  dmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(dmax)));
+  const float tiny = 1e-9f * dmax;
+  int cur = 0;
+  for (int sw = 0; sw < (zero ? 0 : inner_sweeps); ++sw) {
+    int rotated = 0;  // the same in every warp
+#pragma unroll 1
     for (int r = 0; r < JP - 1; ++r) {
-      if (tid < JP / 2) {
-        int p, q;
-        rr_pair(JP, r, tid, p, q);
-        float c, s;
-        const float apq = S[p][q];
-        const float thr = fmaxf(tiny, 1e-7f * sqrtf(fabsf(S[p][p] * S[q][q])));
-        sym_schur2(S[p][p], S[q][q], apq, thr, c, s);
+      const float* Sc = ism + cur * N;
+      float* Sn = ism + (cur ^ 1) * N;
+      const float app = Sc[dg], apq = Sc[dg + JP / 2], aqq = Sc[dg + JP + JP / 2];
+      float m4[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float* p = Sc + 2 * (warp + 16 * h) * JP + lane;
+        m4[h][0] = p[0];
+        m4[h][1] = p[JP / 2];
+        m4[h][2] = p[JP];
+        m4[h][3] = p[JP + JP / 2];
+      }
+      const float pp = fabsf(app * aqq), a2 = apq * apq;
+      float c = 1.f, sn = 0.f;
+      if (fabsf(apq) > tiny && a2 > 1e-14f * pp) {
+        sym_schur2(app, aqq, apq, c, sn);
         // another sweep is needed while some coupling is still above 1e-5 of its pivots
         // (the smaller ones are rotated too, but leave the rest to the outer sweeps and
         // the refinement)
-        if (fabsf(apq) > 1e-5f * sqrtf(fabsf(S[p][p] * S[q][q])) && fabsf(apq) > tiny)
-          rotated = 1;
-        cs[tid][0] = c;
-        cs[tid][1] = s;
-        pq[tid][0] = p;
-        pq[tid][1] = q;
+        if (a2 > 1e-10f * pp) rotated = 1;
       }
-      __syncthreads();
-      // S <- J^T S J on 2 x 2 blocks (pair a rows, pair b columns)
-      for (int blk = tid; blk < (JP / 2) * (JP / 2); blk += blockDim.x) {
-        const int a = blk / (JP / 2), b = blk % (JP / 2);
-        const int p = pq[a][0], q = pq[a][1], r2 = pq[b][0], s2 = pq[b][1];
-        const float ca = cs[a][0], sa = cs[a][1], cb = cs[b][0], sb = cs[b][1];
-        const float m00 = S[p][r2], m01 = S[p][s2], m10 = S[q][r2], m11 = S[q][s2];
+      // S <- J^T S J
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int a = warp + 16 * h;
+        const float ca = __shfl_sync(0xffffffffu, c, a), sa = __shfl_sync(0xffffffffu, sn, a);
         // columns: (x, y) -> (c x - s y, s x + c y)
-        const float n00 = cb * m00 - sb * m01, n01 = sb * m00 + cb * m01;
-        const float n10 = cb * m10 - sb * m11, n11 = sb * m10 + cb * m11;
+        const float n00 = c * m4[h][0] - sn * m4[h][1], n01 = sn * m4[h][0] + c * m4[h][1];
+        const float n10 = c * m4[h][2] - sn * m4[h][3], n11 = sn * m4[h][2] + c * m4[h][3];
         // rows
-        float o00 = ca * n00 - sa * n10, o01 = ca * n01 - sa * n11;
-        float o10 = sa * n00 + ca * n10, o11 = sa * n01 + ca * n11;
-        if (a == b && sa != 0.f) {
+        float o01 = ca * n01 - sa * n11, o10 = sa * n00 + ca * n10;
+        if (a == lane && sa != 0.f) {
           o01 = 0.f;
           o10 = 0.f;
         }
-        S[p][r2] = o00;
-        S[p][s2] = o01;
-        S[q][r2] = o10;
-        S[q][s2] = o11;
+        float* rt = Sn + round_move(2 * a) * JP;
+        float* rb = Sn + round_move(2 * a + 1) * JP;
+        rt[ct] = ca * n00 - sa * n10;
+        rt[cb] = o01;
+        rb[ct] = o10;
+        rb[cb] = sa * n01 + ca * n11;
       }
-      // U <- U J
-      for (int e = tid; e < JP * (JP / 2); e += blockDim.x) {
-        const int i = e / (JP / 2), b = e % (JP / 2);
-        const int p = pq[b][0], q = pq[b][1];
-        const float c = cs[b][0], s = cs[b][1];
-        const float x = U[i][p], y = U[i][q];
-        U[i][p] = c * x - s * y;
-        U[i][q] = s * x + c * y;
+      // U <- U J, then each column to the lane of its next position (round_move)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float x = c * ut[u] - sn * ub[u], y = sn * ut[u] + c * ub[u];
+        const float t = __shfl_up_sync(0xffffffffu, lane == 0 ? y : x, 1);
+        const float w = __shfl_down_sync(0xffffffffu, y, 1);
+        ut[u] = lane == 0 ? x : t;
+        ub[u] = lane == 31 ? x : w;
       }
+      cur ^= 1;
       __syncthreads();
     }
-    // every thread's flag, combined at a barrier (no shared flag for thread 0 to reset
-    // while another warp still reads it)
     if (!__syncthreads_or(rotated)) break;
   }
-  float* u = Uout + (int64_t)blockIdx.x * JP * JP;
-  for (int idx = tid; idx < JP * JP; idx += blockDim.x) u[idx] = U[idx / JP][idx % JP];
+  float* u = Uout + (int64_t)blockIdx.x * N;
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    *reinterpret_cast<float2*>(u + (4 * warp + e) * JP + 2 * lane) = make_float2(ut[e], ub[e]);
 }
 
-// A[rows_i, cols_j] <- U_i^T A[rows_i, cols_j] U_j for the pair tile (i, j) = blockIdx.
+constexpr int JPV = JP + 4;  // pitch of rows read as 16-byte words
+constexpr size_t kApplySmem = 3 * (size_t)JP * JPV * sizeof(float);
+
+// acc += X Y of 64 x 64 matrices in shared memory, thread (ty, tx): rows 4 ty + u, columns
+// 4 tx + v. TX: X is stored transposed.
+template <bool TX>
+__device__ __forceinline__ void mm64(float (&acc)[4][4], const float (*X)[JPV],
+                                     const float (*Y)[JPV], int ty, int tx) {
+#pragma unroll 4
+  for (int k = 0; k < JP; k += 4) {
+    float a[4][4];  // [u][k]
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 v = *reinterpret_cast<const float4*>(TX ? &X[k + e][4 * ty] : &X[4 * ty + e][k]);
+      if (TX) {
+        a[0][e] = v.x; a[1][e] = v.y; a[2][e] = v.z; a[3][e] = v.w;
+      } else {
+        a[e][0] = v.x; a[e][1] = v.y; a[e][2] = v.z; a[e][3] = v.w;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 b = *reinterpret_cast<const float4*>(&Y[k + e][4 * tx]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        acc[u][0] = fmaf(a[u][e], b.x, acc[u][0]);
+        acc[u][1] = fmaf(a[u][e], b.y, acc[u][1]);
+        acc[u][2] = fmaf(a[u][e], b.z, acc[u][2]);
+        acc[u][3] = fmaf(a[u][e], b.w, acc[u][3]);
+      }
+    }
+  }
+}
+
+// blockIdx.y < pairs: A[rows_i, cols_j] <- U_i^T A[rows_i, cols_j] U_j for the pair tile
+// (i, j) = (blockIdx.y, blockIdx.x); else V[rows, cols_j] <- V[rows, cols_j] U_j for 64
+// consecutive rows. Both only wait for the rotations, so one launch takes them.
 __global__ void __launch_bounds__(256)
-    jacobi_apply_kernel(float* __restrict__ A, int64_t lda, int nblk, int round,
-                        const float* __restrict__ Uall, const int* done) {
+    jacobi_apply_kernel(float* __restrict__ A, float* __restrict__ V, int64_t ld, int nblk,
+                        int round, const float* __restrict__ Uall, const int* done) {
   if (*done) return;
-  __shared__ float T[JP][JPS];
-  __shared__ float Ui[JP][JPS];
-  __shared__ float Uj[JP][JPS];
-  int ia, ib, ja, jb;
-  rr_pair(nblk, round, blockIdx.y, ia, ib);
+  extern __shared__ __align__(16) float asm_[];
+  float(*T)[JPV] = reinterpret_cast<float(*)[JPV]>(asm_);
+  float(*Uj)[JPV] = T + JP;
+  float(*Ui)[JPV] = T + 2 * JP;
+  const int pairs = gridDim.x;
+  const bool vec = (int)blockIdx.y >= pairs;
+  int ia = 0, ib = 0, ja, jb;
   rr_pair(nblk, round, blockIdx.x, ja, jb);
+  if (!vec) rr_pair(nblk, round, blockIdx.y, ia, ib);
+  const int64_t r0 = vec ? (int64_t)(blockIdx.y - pairs) * JP : 0;
+  float* M = vec ? V : A;
   const float* ui = Uall + (int64_t)blockIdx.y * JP * JP;
   const float* uj = Uall + (int64_t)blockIdx.x * JP * JP;
   const int tid = threadIdx.x;
-  for (int idx = tid; idx < JP * JP; idx += blockDim.x) {
-    const int r = idx / JP, c = idx % JP;
-    T[r][c] = A[(int64_t)pair_index(ia, ib, r) * lda + pair_index(ja, jb, c)];
-    Ui[r][c] = ui[idx];
-    Uj[r][c] = uj[idx];
+  auto row_of = [&](int r) { return vec ? r0 + r : (int64_t)pair_index(ia, ib, r); };
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int idx = tid + 256 * it, r = idx >> 4, c = (idx & 15) * 4;
+    *reinterpret_cast<float4*>(&T[r][c]) =
+        *reinterpret_cast<const float4*>(M + row_of(r) * ld + pair_index(ja, jb, c));
+    *reinterpret_cast<float4*>(&Uj[r][c]) = *reinterpret_cast<const float4*>(uj + 4 * idx);
+    if (!vec) *reinterpret_cast<float4*>(&Ui[r][c]) = *reinterpret_cast<const float4*>(ui + 4 * idx);
   }
   __syncthreads();
-  // thread (ty, tx): rows 4 ty .. 4 ty + 3, columns tx, tx + 16, tx + 32, tx + 48
   const int tx = tid & 15, ty = tid >> 4;
-  float acc[4][4];
-  // W = T U_j
+  float acc[4][4] = {};
+  mm64<false>(acc, T, Uj, ty, tx);  // T U_j
+  if (!vec) {
+    __syncthreads();
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
-  for (int k = 0; k < JP; ++k) {
-    float a[4], b[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) a[u] = T[4 * ty + u][k];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) b[v] = Uj[k][tx + 16 * v];
+    for (int u = 0; u < 4; ++u)
+      *reinterpret_cast<float4*>(&T[4 * ty + u][4 * tx]) =
+          make_float4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
+    __syncthreads();
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) T[4 * ty + u][tx + 16 * v] = acc[u][v];
-  __syncthreads();
-  // out = U_i^T W
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
-  for (int k = 0; k < JP; ++k) {
-    float a[4], b[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) a[u] = Ui[k][4 * ty + u];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) b[v] = T[k][tx + 16 * v];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
+      for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
+    mm64<true>(acc, Ui, T, ty, tx);  // U_i^T (T U_j)
   }
   // the pair's own tile keeps what the inner sweeps left of its couplings (they need not
   // have run to convergence): the outer sweeps and the off-diagonal norm see them
 #pragma unroll
   for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-      A[(int64_t)pair_index(ia, ib, 4 * ty + u) * lda + pair_index(ja, jb, tx + 16 * v)] =
-          acc[u][v];
-}
-
-// V[rows, cols_j] <- V[rows, cols_j] U_j for 64 consecutive rows (blockIdx.y) and pair j.
-__global__ void __launch_bounds__(256)
-    jacobi_apply_v_kernel(float* __restrict__ V, int64_t ldv, int nblk, int round,
-                          const float* __restrict__ Uall, const int* done) {
-  if (*done) return;
-  __shared__ float T[JP][JPS];
-  __shared__ float Uj[JP][JPS];
-  int ja, jb;
-  rr_pair(nblk, round, blockIdx.x, ja, jb);
-  const float* uj = Uall + (int64_t)blockIdx.x * JP * JP;
-  const int64_t r0 = (int64_t)blockIdx.y * JP;
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < JP * JP; idx += blockDim.x) {
-    const int r = idx / JP, c = idx % JP;
-    T[r][c] = V[(r0 + r) * ldv + pair_index(ja, jb, c)];
-    Uj[r][c] = uj[idx];
-  }
-  __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
-  float acc[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
-  for (int k = 0; k < JP; ++k) {
-    float a[4], b[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) a[u] = T[4 * ty + u][k];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) b[v] = Uj[k][tx + 16 * v];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-      V[(r0 + 4 * ty + u) * ldv + pair_index(ja, jb, tx + 16 * v)] = acc[u][v];
+    *reinterpret_cast<float4*>(M + row_of(4 * ty + u) * ld + pair_index(ja, jb, 4 * tx)) =
+        make_float4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
 }
 
 // A_work = A + shift I (padded with zeros to npad), V = I.
@@ -374,22 +406,25 @@ __device__ __forceinline__ void df_fma_e(float a, float xh, float xl, float& sh,
   sh = s2;
 }
 
-// C[i, j] = sum_k P[k, i] (Qh[k, j] + Ql[k, j]) + shift (Qh[i, j] + Ql[i, j]) over 64 x 64
-// tiles, double-float sums; P, Qh, Ql [n, n] row-major (Ql may be NULL). Output as
-// FP64 (c64) or as a double-float pair (ch, cl).
+// C[i, j] = sum_k P[k, i] (Qh[k, j] + Ql[k, j]) + shift (Qh[i, j] + Ql[i, j]) over T x T
+// tiles (T / 16 outputs per thread and side), double-float sums; P, Qh, Ql [n, n] row-major
+// (Ql may be NULL). Output as FP64 (c64) or as a double-float pair (ch, cl). Bound by the FP32
+// pipe (11 operations a product), so T = 32 where 64 would leave SMs without a tile.
+template <int T>
 __global__ void __launch_bounds__(256)
     df_gemm_tn_kernel(const float* __restrict__ P, const float* __restrict__ Qh,
                       const float* __restrict__ Ql, int64_t n, double shift,
                       double* __restrict__ c64, float* __restrict__ ch, float* __restrict__ cl) {
-  __shared__ float Ps[16][64 + 1];
-  __shared__ float Hs[16][64 + 1];
-  __shared__ float Ls[16][64 + 1];
+  constexpr int R = T / 16;
+  __shared__ float Ps[16][T + 1];
+  __shared__ float Hs[16][T + 1];
+  __shared__ float Ls[16][T + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t i0 = (int64_t)blockIdx.y * 64, j0 = (int64_t)blockIdx.x * 64;
-  float sh[4][4] = {}, sl[4][4] = {};
+  const int64_t i0 = (int64_t)blockIdx.y * T, j0 = (int64_t)blockIdx.x * T;
+  float sh[R][R] = {}, sl[R][R] = {};
   for (int64_t k0 = 0; k0 < n; k0 += 16) {
-    for (int idx = threadIdx.x; idx < 16 * 64; idx += 256) {
-      const int kk = idx / 64, c = idx % 64;
+    for (int idx = threadIdx.x; idx < 16 * T; idx += 256) {
+      const int kk = idx / T, c = idx % T;
       const bool kin = k0 + kk < n;
       Ps[kk][c] = (kin && i0 + c < n) ? P[(k0 + kk) * n + i0 + c] : 0.f;
       Hs[kk][c] = (kin && j0 + c < n) ? Qh[(k0 + kk) * n + j0 + c] : 0.f;
@@ -398,27 +433,27 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
-      float av[4], hv[4], lv[4];
+      float av[R], hv[R], lv[R];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        av[u] = Ps[k][ty * 4 + u];
-        hv[u] = Hs[k][tx * 4 + u];
-        lv[u] = Ls[k][tx * 4 + u];
+      for (int u = 0; u < R; ++u) {
+        av[u] = Ps[k][ty * R + u];
+        hv[u] = Hs[k][tx * R + u];
+        lv[u] = Ls[k][tx * R + u];
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < R; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) df_fma_e(av[u], hv[v], lv[v], sh[u][v], sl[u][v]);
+        for (int v = 0; v < R; ++v) df_fma_e(av[u], hv[v], lv[v], sh[u][v], sl[u][v]);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int64_t i = i0 + ty * 4 + u;
+  for (int u = 0; u < R; ++u) {
+    const int64_t i = i0 + ty * R + u;
     if (i >= n) continue;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int64_t j = j0 + tx * 4 + v;
+    for (int v = 0; v < R; ++v) {
+      const int64_t j = j0 + tx * R + v;
       if (j >= n) continue;
       double val = (double)sh[u][v] + (double)sl[u][v];
       if (shift != 0.0)
@@ -430,6 +465,17 @@ __global__ void __launch_bounds__(256)
         cl[i * n + j] = (float)(val - (double)h);
       }
     }
+  }
+}
+
+void df_gemm_tn(cudaStream_t s, const float* P, const float* Qh, const float* Ql, int64_t n,
+                double shift, double* c64, float* ch, float* cl) {
+  if (ceil_div(n, 64) * ceil_div(n, 64) >= 2 * 152) {
+    const dim3 g((unsigned)ceil_div(n, 64), (unsigned)ceil_div(n, 64));
+    df_gemm_tn_kernel<64><<<g, 256, 0, s>>>(P, Qh, Ql, n, shift, c64, ch, cl);
+  } else {
+    const dim3 g((unsigned)ceil_div(n, 32), (unsigned)ceil_div(n, 32));
+    df_gemm_tn_kernel<32><<<g, 256, 0, s>>>(P, Qh, Ql, n, shift, c64, ch, cl);
   }
 }
 
@@ -461,7 +507,8 @@ __global__ void refine_lambda_kernel(const double* __restrict__ S, const double*
 
 // E = the correction of X (see above); X1 = X (for the accumulate of X + X E).
 __global__ void refine_e_kernel(const double* __restrict__ S, const double* __restrict__ R,
-                                const double* __restrict__ lam, int64_t n, float* __restrict__ E) {
+                                const double* __restrict__ lam, int64_t n, double sep,
+                                float* __restrict__ E) {
   const int64_t total = n * n;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
@@ -469,11 +516,12 @@ __global__ void refine_e_kernel(const double* __restrict__ S, const double* __re
     const double r = R[idx];
     double e = 0.5 * r;
     if (i != j) {
-      // separated: the gap is large against the coupling and above the resolution of the
-      // float32 eigenvalues (1e-6 of the largest); closer pairs are a cluster
+      // separated: the gap is `sep` times the coupling or more (what a correction leaves over
+      // is its square) and above the resolution of the float32 eigenvalues (1e-6 of the
+      // largest); closer pairs are a cluster
       const double num = S[idx] + lam[j] * r;
       const double gap = lam[j] - lam[i];
-      if (fabs(gap) > 1e3 * fabs(num) && fabs(gap) > 1e-6 * lam[n]) e = num / gap;
+      if (fabs(gap) > sep * fabs(num) && fabs(gap) > 1e-6 * lam[n]) e = num / gap;
     }
     E[idx] = (float)e;
   }
@@ -543,19 +591,24 @@ extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, f
   const int nblk = (int)(npad / JB);  // even
   const int npairs = nblk / 2;
   const EighWs e = eigh_ws(workspace, npad);
+  if (cudaFuncSetAttribute(jacobi_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kApplySmem) != cudaSuccess)
+    return check_launch("ntg_eigh");
   eigh_init_kernel<<<egrid(npad * npad), 256, 0, s>>>(A, n, shift, e.w, e.v, npad);
   note_launch();
   if (cudaMemsetAsync(e.done, 0, sizeof(int), s) != cudaSuccess) return check_launch("ntg_eigh");
   int sweeps = 0;
+  double off2 = INFINITY;
   for (int sw = 0; sw < max_sweeps; ++sw) {
     for (int r = 0; r < nblk - 1; ++r) {
-      // two inner sweeps per pair and round: the outer sweeps converge as fast, and an
-      // inner problem driven to convergence early on is undone by the next rounds
-      jacobi_inner_kernel<<<npairs, 256, 0, s>>>(e.w, npad, nblk, r, 2, e.u, e.done);
-      jacobi_apply_kernel<<<dim3(npairs, npairs), 256, 0, s>>>(e.w, npad, nblk, r, e.u, e.done);
-      jacobi_apply_v_kernel<<<dim3(npairs, (unsigned)(npad / JP)), 256, 0, s>>>(
-          e.v, npad, nblk, r, e.u, e.done);
-      note_launch(3);
+      // one inner sweep per pair and round: an inner problem driven further is undone by the
+      // next rounds (n = 500: nine outer sweeps with one inner sweep or two, 7.4 against 12.0
+      // ms). A single pair is the whole matrix: to convergence.
+      jacobi_inner_kernel<<<npairs, kInnerThreads, 0, s>>>(e.w, npad, nblk, r,
+                                                           npairs == 1 ? 8 : 1, e.u, e.done);
+      jacobi_apply_kernel<<<dim3(npairs, (unsigned)(npairs + npad / JP)), 256, kApplySmem, s>>>(
+          e.w, e.v, npad, nblk, r, e.u, e.done);
+      note_launch(2);
     }
     ++sweeps;
     if (cudaMemsetAsync(e.norms, 0, 2 * sizeof(double), s) != cudaSuccess)
@@ -567,7 +620,9 @@ extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, f
         cudaStreamSynchronize(s) != cudaSuccess)
       return check_launch("ntg_eigh norms");
     const double fro2 = nh[0] + nh[1];
-    if (nh[0] <= tol * tol * fro2) break;
+    // converged, or down at what float32 rounding leaves (sweeps converge quadratically)
+    if (nh[0] <= tol * tol * fro2 || (nh[0] <= 1e-10 * fro2 && nh[0] > 0.1 * off2)) break;
+    off2 = nh[0];
   }
   eigh_extract_kernel<<<egrid(n * n), 256, 0, s>>>(e.w, e.v, npad, n, evals, evecs);
   note_launch();
@@ -580,17 +635,18 @@ extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, f
     float* yh = reinterpret_cast<float*>(lam + n + 1);
     float* yl = yh + n * n;
     float* E = yl + n * n;
-    const dim3 g((unsigned)ceil_div(n, 64), (unsigned)ceil_div(n, 64));
     for (int it = 0; it < refine_steps; ++it) {
       // Y = (K + shift I) X (K symmetric: K^T X), S = X^T Y, R = X^T X (as -R + I below)
-      df_gemm_tn_kernel<<<g, 256, 0, s>>>(A, evecs, nullptr, n, shift, nullptr, yh, yl);
-      df_gemm_tn_kernel<<<g, 256, 0, s>>>(evecs, yh, yl, n, 0.0, S, nullptr, nullptr);
-      df_gemm_tn_kernel<<<g, 256, 0, s>>>(evecs, evecs, nullptr, n, 0.0, R, nullptr, nullptr);
+      df_gemm_tn(s, A, evecs, nullptr, n, shift, nullptr, yh, yl);
+      df_gemm_tn(s, evecs, yh, yl, n, 0.0, S, nullptr, nullptr);
+      df_gemm_tn(s, evecs, evecs, nullptr, n, 0.0, R, nullptr, nullptr);
       identity_minus_kernel<<<egrid(n * n), 256, 0, s>>>(R, n);
       if (cudaMemsetAsync(lam + n, 0, sizeof(double), s) != cudaSuccess)
         return check_launch("ntg_eigh refine");
       refine_lambda_kernel<<<egrid(n), 256, 0, s>>>(S, R, n, lam);
-      refine_e_kernel<<<egrid(n * n), 256, 0, s>>>(S, R, lam, n, E);
+      // corrections up to 1e-2 where another step cleans up after them, 1e-3 in the last
+      const double sep = it + 1 < refine_steps ? 1e2 : 1e3;
+      refine_e_kernel<<<egrid(n * n), 256, 0, s>>>(S, R, lam, n, sep, E);
       note_launch(6);
       // X <- X + X E (the product reads a copy of X)
       if (cudaMemcpyAsync(yh, evecs, sizeof(float) * n * n, cudaMemcpyDeviceToDevice, s) !=

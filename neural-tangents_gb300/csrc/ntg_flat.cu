@@ -433,6 +433,106 @@ void launch_gram_small(bool sym, bool vec, cudaStream_t s, const float* x1, cons
 
 }  // namespace
 
+namespace {
+
+// Small products C[M, N] (+)= alpha op(A) B, op(A) = A [M, K] or (TA) A^T with A [K, M]: 32 x 32
+// tiles, 2 x 2 outputs per thread, slices of 16 streamed by a 4-stage cp.async ring. Bound by
+// the chain of K / 16 slices, so the sums can afford to be better than one long chain: each
+// slice is summed by itself and added with its rounding error kept (two-sum).
+template <bool TA>
+__global__ void __launch_bounds__(256)
+    gemm_small_kernel(const float* __restrict__ A, const float* __restrict__ B,
+                      float* __restrict__ C, int64_t M, int64_t N, int64_t K, float alpha,
+                      int accumulate) {
+  constexpr int T = 32, BK = 16, ST = 4, PA = TA ? T + 4 : BK + 4, RA = TA ? BK : T;
+  __shared__ __align__(16) float As[ST][RA * PA];
+  __shared__ __align__(16) float Bs[ST][BK * (T + 4)];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int64_t row0 = (int64_t)blockIdx.y * T, col0 = (int64_t)blockIdx.x * T;
+  const int64_t nk = (K + BK - 1) / BK;
+  auto stage = [&](int64_t s) {
+    if (s < nk) {
+      // rows of A (of length K, or M when transposed) and of B (length N), 4 bytes a copy
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int idx = threadIdx.x + 256 * e;
+        if (TA) {
+          const int r = idx >> 5, c = idx & 31;
+          const int64_t gk = s * BK + r, gi = row0 + c;
+          const bool in = gk < K && gi < M;
+          cp_async<false>(&As[s % ST][r * PA + c], in ? A + gk * M + gi : A, in);
+        } else {
+          const int r = idx >> 4, c = idx & 15;
+          const int64_t gk = s * BK + c, gi = row0 + r;
+          const bool in = gk < K && gi < M;
+          cp_async<false>(&As[s % ST][r * PA + c], in ? A + gi * K + gk : A, in);
+        }
+        const int r = idx >> 5, c = idx & 31;
+        const int64_t gk = s * BK + r, gj = col0 + c;
+        const bool in = gk < K && gj < N;
+        cp_async<false>(&Bs[s % ST][r * (T + 4) + c], in ? B + gk * N + gj : B, in);
+      }
+    }
+    cp_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < ST - 1; ++s) stage(s);
+  float hi[2][2] = {}, lo[2][2] = {};
+  for (int64_t s = 0; s < nk; ++s) {
+    cp_wait<ST - 2>();
+    __syncthreads();
+    stage(s + ST - 1);
+    const float* a = As[s % ST];
+    const float* b = Bs[s % ST];
+    float p[2][2] = {};
+#pragma unroll
+    for (int k = 0; k < BK; ++k) {
+      const float2 bv = *reinterpret_cast<const float2*>(b + k * (T + 4) + 2 * tx);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float av = TA ? a[k * PA + 2 * ty + u] : a[(2 * ty + u) * PA + k];
+        p[u][0] = fmaf(av, bv.x, p[u][0]);
+        p[u][1] = fmaf(av, bv.y, p[u][1]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const float t = __fadd_rn(hi[u][v], p[u][v]);
+        const float z = __fsub_rn(t, hi[u][v]);
+        lo[u][v] += __fadd_rn(__fsub_rn(hi[u][v], __fsub_rn(t, z)), __fsub_rn(p[u][v], z));
+        hi[u][v] = t;
+      }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int64_t gi = row0 + 2 * ty + u, gj = col0 + 2 * tx + v;
+      if (gi >= M || gj >= N) continue;
+      float* c = C + gi * N + gj;
+      // an infinite or NaN sum has no rounding error to add
+      const float r = alpha * (isfinite(hi[u][v]) ? hi[u][v] + lo[u][v] : hi[u][v]);
+      *c = accumulate ? *c + r : r;
+    }
+}
+
+}  // namespace
+
+bool gemm_small(cudaStream_t s, const float* a, const float* b, float* c, int64_t m, int64_t n,
+                int64_t k, bool trans_a, float alpha, bool accumulate) {
+  // below one 64 x 64 tile per SM: the eigenvectors of 500 points times 60 columns take 16 us
+  // (57 us on eight 64 x 64 tiles)
+  if (ceil_div(m, 64) * ceil_div(n, 64) >= 152 || ceil_div(m, 32) > 65535) return false;
+  const dim3 grid((unsigned)ceil_div(n, 32), (unsigned)ceil_div(m, 32));
+  if (trans_a)
+    gemm_small_kernel<true><<<grid, 256, 0, s>>>(a, b, c, m, n, k, alpha, accumulate);
+  else
+    gemm_small_kernel<false><<<grid, 256, 0, s>>>(a, b, c, m, n, k, alpha, accumulate);
+  return true;
+}
+
 int gram_fp32(cudaStream_t s, const float* x1, const float* x2, int64_t n1, int64_t n2, int64_t d,
               float* out) {
   NTG_REQUIRE(ceil_div(n1, 128) <= 65535, "ntg_gram: n1 too large");

@@ -1635,8 +1635,10 @@ extern "C" int ntg_gemm(void* stream, const float* a, const float* b, float* c, 
   NTG_REQUIRE(a && b && c, "ntg_gemm: null pointer");
   NTG_REQUIRE(m > 0 && n > 0 && k > 0, "ntg_gemm: sizes must be positive");
   NTG_REQUIRE(ceil_div(m, 64) <= 65535, "ntg_gemm: m too large");
-  dim3 grid((unsigned)ceil_div(n, 64), (unsigned)ceil_div(m, 64));
-  gemm_nn_kernel<<<grid, 256, 0, as_stream(stream)>>>(a, b, c, m, n, k, accumulate);
+  if (!gemm_small(as_stream(stream), a, b, c, m, n, k, false, 1.f, accumulate)) {
+    dim3 grid((unsigned)ceil_div(n, 64), (unsigned)ceil_div(m, 64));
+    gemm_nn_kernel<<<grid, 256, 0, as_stream(stream)>>>(a, b, c, m, n, k, accumulate);
+  }
   note_launch();
   return check_launch("ntg_gemm");
 }

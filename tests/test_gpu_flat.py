@@ -84,3 +84,22 @@ def test_long_run_is_split(nt):
         s.serial(s.Dense(1), s.Relu(), s.Relu())[2](x, None, 'nngp')
     y = np.asarray([[1., 2.], [3., 4.]], np.float32)
     assert s.Identity()[2](y, None).ntk.ndim == 0
+
+
+@pytest.mark.parametrize('m,n,k', [(1, 1, 1), (31, 33, 15), (32, 32, 16), (33, 65, 17),
+                                   (500, 60, 500), (640, 700, 100), (100, 4000, 33),
+                                   (768, 832, 40)])
+def test_small_products(nt, m, n, k):
+    """Both sides of the rule (152 tiles of 64 x 64), plain and transposed, accumulating."""
+    from nt_gb300 import _lib as L, predict
+    a, b = _data(m, k, 6), _data(k, n, 7)
+    want = a.double() @ b.double()
+    # at most a chain of k products
+    bound = (k + 3) * 2. ** -24 * (a.double().abs() @ b.double().abs())
+    assert bool(((predict._gemm(a, b).double() - want).abs() <= bound).all())
+    at = a.t().contiguous()
+    assert bool(((predict._gemm_tn(at, b).double() - want).abs() <= bound).all())
+    c = torch.ones((m, n), device='cuda')
+    L.call('ntg_gemm_ex', L.stream(), L.ptr(a), L.ptr(b), L.ptr(c), m, n, k, 0, -2., 1)
+    assert bool(((c.double() - (1. - 2. * want)).abs() <= 2 * bound + 2. ** -22
+                 * (1. + 2. * want.abs())).all())
