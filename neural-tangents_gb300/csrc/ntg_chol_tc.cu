@@ -30,6 +30,7 @@
 #include <string>
 
 #include "ntg_common.cuh"
+#include "ntg_exact_tc.cuh"
 
 namespace ntg {
 int gemm_tf32x3(cudaStream_t s, const float* a, int64_t lda, const float* b, int64_t ldb,
@@ -1055,10 +1056,13 @@ FactorWs factor_ws(void* ws, int64_t n, int64_t ldl) {
 // arrays [kDotBlocks * kSmallM] f64, the PcgState and the double-float split of the
 // current vector [n m] float2, and the split-K tiles of the triangular and double-float
 // products; for more, z [m * ldl] f32, y [m * ldl] f32 (the transposed right-hand sides
-// and their half-solved form) and the double-float split of x [n m] float2.
+// and their half-solved form) and the double-float split of x [n m] float2, or the digits
+// of the exact residual.
 size_t solve_ws_bytes(int64_t n, int64_t m, int64_t ldl) {
   size_t b = 256 + (size_t)n * m * (sizeof(double) + 2 * sizeof(float)) + 256;
-  if (m > kSmallM) b += 2 * (size_t)m * ldl * sizeof(float) + 512 + (size_t)n * m * sizeof(float2);
+  if (m > kSmallM)
+    b += 2 * (size_t)m * ldl * sizeof(float) + 512 +
+         (exact_residual_pays(n, m) ? exact_residual_bytes(n, m) : (size_t)n * m * sizeof(float2));
   else b += (size_t)3 * n * m * sizeof(double) + 3 * kDotBlocks * kSmallM * sizeof(double) +
             sizeof(PcgState) + 256 + (size_t)n * m * sizeof(float2) + 256 +
             tri_part_bytes(n, m) + 256 + df_part_bytes(n, n, m) + 256;
@@ -1356,10 +1360,15 @@ extern "C" int ntg_chol_solve_tc(void* stream, const float* A, const float* L, i
     if (it == refine_iters && !final_residual) break;
     if (cudaMemsetAsync(rnorm, 0, sizeof(double), s) != cudaSuccess)
       return check_launch("ntg_chol_solve_tc memset");
-    split_df_kernel<<<grid_for(n * m), 256, 0, s>>>(x64, m, n, m, xsplit, nullptr);
-    residual_df_kernel<<<dim3((unsigned)ceil_div(m, 64), (unsigned)ceil_div(n, 64)), 256, 0, s>>>(
-        A, n, lambda, B, B64, x64, xsplit, m, r32, rnorm);
-    note_launch(2);
+    if (exact_residual_pays(n, m)) {
+      rc = exact_residual(s, A, n, lambda, B, B64, x64, m, r32, rnorm, xsplit, it > 0);
+      if (rc) return rc;
+    } else {
+      split_df_kernel<<<grid_for(n * m), 256, 0, s>>>(x64, m, n, m, xsplit, nullptr);
+      residual_df_kernel<<<dim3((unsigned)ceil_div(m, 64), (unsigned)ceil_div(n, 64)), 256, 0, s>>>(
+          A, n, lambda, B, B64, x64, xsplit, m, r32, rnorm);
+      note_launch(2);
+    }
     if (it == refine_iters) break;
     rc = apply(r32, nullptr);
     if (rc) return rc;

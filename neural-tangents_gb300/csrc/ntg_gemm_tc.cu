@@ -39,7 +39,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 int make_map_2d(CUtensorMap* m, CUtensorMapDataType dtype, int elem_bytes, const void* base,
                 int64_t rows, int64_t cols, int64_t ld, int box_rows, int box_cols,
-                const char* who) {
+                const char* who, CUtensorMapSwizzle swizzle) {
   auto fn = encode_fn();
   if (!fn) return fail(NTG_ERR_CUDA, std::string(who) + ": cuTensorMapEncodeTiled unavailable");
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
@@ -47,7 +47,7 @@ int make_map_2d(CUtensorMap* m, CUtensorMapDataType dtype, int elem_bytes, const
   cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t es[2] = {1, 1};
   CUresult r = fn(m, dtype, 2, const_cast<void*>(base), dims, strides, box, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(NTG_ERR_CUDA, std::string(who) + ": cuTensorMapEncodeTiled failed");
   return NTG_OK;

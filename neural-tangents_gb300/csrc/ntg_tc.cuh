@@ -66,6 +66,17 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
   return d;
 }
 
+// The same with 64-byte rows and the 64-byte swizzle: 8-row groups 512 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr & 0x3FFFF) >> 4);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(512 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)4 << 61;  // SWIZZLE_64B
+  return d;
+}
+
 // Instruction descriptor: D F32, A/B of format `fmt` (kind::f16: 1 = BF16;
 // kind::tf32: 2 = TF32), both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc(uint32_t fmt, int m, int n) {
@@ -106,11 +117,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn();
 
 // Row-major [rows, cols] tensor of `elem_bytes` elements with a row pitch of
-// `ld` elements, read in boxes of box_rows x box_cols with 128-byte swizzle;
-// out-of-range elements read as zero.
+// `ld` elements, read in boxes of box_rows x box_cols with 128- or 64-byte swizzle (the bytes
+// of a box row); out-of-range elements read as zero.
 int make_map_2d(CUtensorMap* m, CUtensorMapDataType dtype, int elem_bytes, const void* base,
                 int64_t rows, int64_t cols, int64_t ld, int box_rows, int box_cols,
-                const char* who);
+                const char* who, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
 }  // namespace tc
 }  // namespace ntg

@@ -141,3 +141,56 @@ def test_concurrent_factorisations_on_two_streams(nt):
         a = a + 1e-3 * np.trace(a) / 700 * np.eye(700)
         lf = out[i].cpu().numpy().astype(np.float64)
         assert np.max(np.abs(lf @ lf.T - a)) / np.max(np.abs(a)) < 1e-5
+
+
+@pytest.mark.parametrize('n,m', [(1024, 65), (1030, 300), (777, 500), (2050, 65), (1500, 1500)])
+def test_exact_residual(nt, n, m):
+    """The tensor-core residual of many right-hand sides (from 2^26 products on) against
+    float64: the largest residual of a returned solution, whose true size is 1e-9 to 1e-7 of
+    the products it cancels. The digits carry 40 bits of each product, sums are exact, and
+    float64's own sums are good to n 2^-53."""
+    from nt_gb300 import predict
+    g = torch.Generator(device='cuda').manual_seed(n + m)
+    x = torch.randn((n, 64), generator=g, device='cuda', dtype=torch.float64)
+    # a kernel with a large constant part and scales that differ from row to row
+    s = torch.exp(torch.randn((n, 1), generator=g, device='cuda', dtype=torch.float64))
+    k = ((x @ x.t() / 64 + 1.) ** 2 * s * s.t()).float()
+    b = torch.randn((n, m), generator=g, device='cuda')
+    b[:, 0] = 0.
+    solver = predict.CholeskySolver(k, 1e-2, False)
+    xs, x64 = solver.solve(b, refine_iters=1, want_x64=True)
+    a = k.double() + float(solver.lam[0]) * torch.eye(n, device='cuda', dtype=torch.float64)
+    r = b.double() - a @ x64
+    size = (a.abs().amax(1, keepdim=True) * x64.abs().amax(0, keepdim=True)).max()
+    assert abs(float(solver.residual) - float(r.abs().max())) < n ** .5 * 2. ** -38 * float(size)
+    # and what the step made of it: the solution is that of float64 to float32 rounding
+    want = torch.linalg.solve(a, b.double())
+    assert float((x64 - want).norm() / want.norm()) < 1e-6
+    assert float(xs[:, 0].abs().max()) == 0.
+    # another solver's NaN row reaches every solution, as it does in float64
+    bad = k.clone()
+    bad[3, 5] = bad[5, 3] = float('nan')
+    with pytest.warns(UserWarning, match='not positive definite'):
+        out = predict.CholeskySolver(bad, 1e-2, False).solve(b, refine_iters=1)
+    assert bool(torch.isnan(out).all())
+
+
+def test_exact_residual_in_bands(nt):
+    """A's digits are made 7168 rows at a time from there on: the largest residual once more,
+    under the same bound, at two bands and a remainder of columns."""
+    from nt_gb300 import predict
+    n, m = 7300, 70
+    g = torch.Generator(device='cuda').manual_seed(1)
+    x = torch.randn((n, 64), generator=g, device='cuda')
+    k = (x @ x.t() / 64 + 1.) ** 2
+    k = (k + k.t()) / 2
+    b = torch.randn((n, m), generator=g, device='cuda')
+    # the large rows, and so the largest residual, in either band in turn
+    for rows in (slice(0, 64), slice(n - 64, n)):
+        b2 = b * 1e-4
+        b2[rows] = b[rows]
+        solver = predict.CholeskySolver(k, 1e-1, False)
+        _, x64 = solver.solve(b2, refine_iters=1, want_x64=True)
+        r = b2.double() - k.double() @ x64 - float(solver.lam[0]) * x64
+        size = (k.abs().amax(1, keepdim=True) * x64.abs().amax(0, keepdim=True)).max()
+        assert abs(float(solver.residual) - float(r.abs().max())) < n ** .5 * 2. ** -38 * float(size)
