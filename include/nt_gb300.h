@@ -282,13 +282,18 @@ int ntg_chain_fwd_ws(void* stream, const ntg_chain_t* prog, const float* x1, con
 /* Whole conv network on diagonal-spatial kernels (linear.py:3381-3437): inputs x1 [N1, a, c, K],
  * x2 [N2, a, c, K] (NULL: x1 with itself, n2 == n1, the pairs i <= j evaluated and mirrored);
  * each layer a stride-1, zero-padded fh x fw window (a Dense is 1 x 1) to ao x co positions,
- * its affine rule and activation; then sum over the positions / divisor * scale. Writes nngp
+ * its affine rule and activation and, for pool_h > 0, the sum over pool_h x pool_w windows of
+ * both positions at strides pool_sh, pool_sw (inside the map, remainders dropped) times
+ * pool_scale; then sum over the positions / divisor * scale. Behind a pooling the result is
+ * that of the full-spatial rules with a Flatten readout. Writes nngp
  * (and ntk unless NULL) [N1, N2], the per-sample readouts cov1 [N1], cov2 [N2] and, as
  * scratch, the layers' variance maps var1 [N1, var_stride], var2 [N2, var_stride]. The caller
  * sets var_off to the running sum of ao * co and var_stride to their total; plane is ignored. */
 enum { NTG_DS_MAX_LAYERS = 16 };
 typedef struct {
   int32_t fh, fw, ph, pw, ao, co, var_off;
+  int32_t pool_h, pool_w, pool_sh, pool_sw;
+  float pool_scale;
   ntg_affine_t aff;
   ntg_act_t act;
 } ntg_ds_layer_t;

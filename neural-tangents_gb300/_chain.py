@@ -24,7 +24,7 @@ import torch
 from . import _lib as L
 from . import _ops as O
 from .kernel import Kernel
-from .stax import Padding, _Ctx, _act_struct, _affine_struct, _conv_geometry
+from .stax import Padding, _Ctx, _act_struct, _affine_struct, _conv_geometry, _pads
 
 S0 = 32
 
@@ -223,26 +223,49 @@ def run_fused(plan: ChainPlan, x1: torch.Tensor, x2: Optional[torch.Tensor], ctx
 
 
 # ---------------------------------------------------------------------------
-# Conv networks on diagonal-spatial kernels (ntg_ds_chain)
+# Conv networks on diagonal-spatial kernels and on bands around them (ntg_ds_chain)
 # ---------------------------------------------------------------------------
 
 DS_MAX_SMEM = 100 * 1024  # two CTAs per SM; larger images go layer by layer
+# One CTA walks all planes of a pair's band, 3 - 9 us a plane with the layers of its level, so
+# that many planes take long for few pairs. 49 (two 2 x 2 poolings, one of 4 x 4): 0.36 - 0.49 ms
+# from 1 to 256 pairs of 8 x 8 to 32 x 32 images, against 1.1 - 2.9 ms by the layer rules or the
+# whole-kernel chain; 225 (three poolings): 1.3 - 1.9 ms against 1.3 - 1.4 ms up to 32 pairs.
+BAND_MAX_PLANES = 49
 
 
-def plan_ds(specs, x_shape, ctx: _Ctx):
+def _narrow_band(specs, size) -> bool:
+    """Whether the poolings leave a Flatten no more than BAND_MAX_PLANES offsets to see."""
+    d = [0] * len(size)
+    pools = [s.params for s in specs if s.kind == 'pool']
+    for p in reversed(pools):
+        if len(p['window_shape']) != len(size):
+            return False
+        d = [s * x + k - 1 for x, k, s in zip(d, p['window_shape'], p['strides'])]
+    planes = 1
+    for x, m in zip(d, size):
+        planes *= 2 * min(x, m - 1) + 1
+    return bool(pools) and planes <= BAND_MAX_PLANES
+
+
+def plan_ds(specs, x_shape, ctx: _Ctx, pools: bool = False):
     """(program, layers after the readout, is_gaussian) of a serial network whose layers up to a
     Flatten / GlobalAvgPool / GlobalSumPool readout are stride-1 zero-padded Conv, Dense and
-    activations, on [N, A, K] or [N, A, C, K] inputs; None for another network."""
+    activations, on [N, A, K] or [N, A, C, K] inputs; None for another network. pools: a network
+    with AvgPool / SumPool layers among these, their windows inside the maps, and a Flatten
+    readout, which sees a band around the spatial diagonal."""
     if len(x_shape) not in (3, 4):
         return None
     specs = [s for s in specs if s.kind != 'identity']
     ridx = next((i for i, s in enumerate(specs) if s.kind in ('gpool', 'flatten')), None)
-    if not ridx or ridx > 2 * L.DS_MAX_LAYERS or specs[0].kind == 'act':
+    if not ridx or ridx > 3 * L.DS_MAX_LAYERS or specs[0].kind == 'act':
+        return None
+    if pools and (specs[ridx].kind != 'flatten' or not _narrow_band(specs[:ridx], x_shape[1:-1])):
         return None
     a, c = x_shape[1], x_shape[2] if len(x_shape) == 4 else 1
     pg = L.DsChain()
     pg.a, pg.c, pg.channels = a, c, x_shape[-1]
-    shape, n, off, gaussian, plane = tuple(x_shape), 0, 0, False, a * c
+    shape, n, off, gaussian, plane, pooled = tuple(x_shape), 0, 0, False, a * c, []
     for s in specs[:ridx]:
         p = s.params
         if s.kind == 'act':
@@ -250,6 +273,23 @@ def plan_ds(specs, x_shape, ctx: _Ctx):
                 return None
             pg.layer[n - 1].act = _act_struct(p, ctx)
             gaussian = False
+            continue
+        if s.kind == 'pool' and pools:
+            if not n or pg.layer[n - 1].pool_h:
+                return None
+            (kh, sh), (kw, sw) = [
+                (p['window_shape'][d], p['strides'][d]) if d < len(x_shape) - 2 else (1, 1)
+                for d in (0, 1)]
+            if len(p['window_shape']) != len(x_shape) - 2 or kh > a or kw > c or any(
+                    _pads(m, f, st, p['padding']) != (0, (m - f) // st + 1)
+                    for m, f, st in ((a, kh, sh), (c, kw, sw))):
+                return None
+            ly = pg.layer[n - 1]
+            ly.pool_h, ly.pool_w, ly.pool_sh, ly.pool_sw = kh, kw, sh, sw
+            ly.pool_scale = 1. / (kh * kw) ** 2 if p['pool'] == 'avg' else 1.
+            pooled.append((kh, kw, sh, sw, a, c))
+            a, c = (a - kh) // sh + 1, (c - kw) // sw + 1
+            shape = s.shape_fn(shape)
             continue
         if s.kind not in ('conv', 'dense') or n == L.DS_MAX_LAYERS:
             return None
@@ -282,19 +322,26 @@ def plan_ds(specs, x_shape, ctx: _Ctx):
     # number once more for GlobalAvgPool
     pg.divisor = float(a * c) if average else 1.
     pg.scale = 1. / (a * c) if average and not flatten else 1.
-    if 4 * (pg.channels * pg.a * pg.c + off + 4 * plane) > DS_MAX_SMEM or pg.c > 512 or \
-            pg.a > 4096:
+    # the offsets of each level, from the readout back, and the entries of the pooled planes
+    da = dc = entries = 0
+    m, k = a, c
+    for kh, kw, sh, sw, pa, pc in reversed(pooled):
+        entries += (2 * da + 1) * (2 * dc + 1) * m * k
+        da, dc = min(sh * da + kh - 1, pa - 1), min(sw * dc + kw - 1, pc - 1)
+        m, k = pa, pc
+    if 4 * (pg.channels * pg.a * pg.c + off + 4 * plane + 2 * entries) > DS_MAX_SMEM or \
+            pg.c > 512 or pg.a > 4096:
         return None
     return pg, specs[:ridx + 1], specs[ridx + 1:], gaussian and not flatten
 
 
 def try_ds(kfn, x1: torch.Tensor, x2: Optional[torch.Tensor], compute_ntk: bool, ctx: _Ctx,
-           whole: bool) -> Optional[Kernel]:
-    """The Kernel of a network plan_ds covers, on diagonal-spatial kernels; whole: see
-    try_fused."""
+           whole: bool, pools: bool = False) -> Optional[Kernel]:
+    """The Kernel of a network plan_ds covers, on diagonal-spatial kernels or (pools) on a band
+    around them; whole: see try_fused."""
     if x2 is not None and x2.shape[1:] != x1.shape[1:]:
         return None
-    plan = plan_ds(kfn.specs, tuple(x1.shape), ctx)
+    plan = plan_ds(kfn.specs, tuple(x1.shape), ctx, pools)
     if plan is None:
         return None
     pg, spatial, post, gaussian = plan

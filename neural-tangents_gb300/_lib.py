@@ -58,8 +58,9 @@ class Chain(C.Structure):
 
 class DsLayer(C.Structure):
     _fields_ = [('fh', C.c_int32), ('fw', C.c_int32), ('ph', C.c_int32), ('pw', C.c_int32),
-                ('ao', C.c_int32), ('co', C.c_int32), ('var_off', C.c_int32), ('aff', Affine),
-                ('act', Act)]
+                ('ao', C.c_int32), ('co', C.c_int32), ('var_off', C.c_int32),
+                ('pool_h', C.c_int32), ('pool_w', C.c_int32), ('pool_sh', C.c_int32),
+                ('pool_sw', C.c_int32), ('pool_scale', C.c_float), ('aff', Affine), ('act', Act)]
 
 
 class DsChain(C.Structure):

@@ -733,8 +733,9 @@ class KernelFn:
                 return vals[0] if single is not None else analytic_kernel(names, vals)
             compare = names is None or 'x1_is_x2' in names
             whole = names is None or not set(names) <= {'nngp', 'ntk'}
-            k = _chain.try_ds(self, x1, x2t, compute_ntk, ctx, whole) if ds else \
-                _chain.try_fused(self, x1, x2t, ds, compute_ntk, ctx, whole)
+            k = _chain.try_ds(self, x1, x2t, compute_ntk, ctx, whole, pools=not ds)
+            if k is None and not ds:
+                k = _chain.try_fused(self, x1, x2t, ds, compute_ntk, ctx, whole)
             if k is None:
                 cnone = bool(self.specs) and self.specs[0].channel_axis_none
                 first = next((sp for sp in self.specs if sp.kind != 'identity'), None)
