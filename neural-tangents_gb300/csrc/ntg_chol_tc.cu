@@ -35,7 +35,7 @@
 namespace ntg {
 int gemm_tf32x3(cudaStream_t s, const float* a, int64_t lda, const float* b, int64_t ldb,
                 float* c, int64_t ldc, int64_t m, int64_t n, int64_t k, float alpha, float beta,
-                int lower);
+                int lower, int tri = 0);
 
 namespace {
 
@@ -1098,7 +1098,9 @@ int inv_apply_small(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, f
 }
 
 // X = (L L^T)^-1 X for many right-hand sides on the tensor cores, through the transposed
-// right-hand sides z = X^T [m, ldl]: y = z L^-T (= (L^-1 X)^T), z = y L^-1 (= X'^T).
+// right-hand sides z = X^T [m, ldl]: y = z L^-T (= (L^-1 X)^T), z = y L^-1 (= X'^T). Each
+// tile's sum runs over the triangle only (4096 right-hand sides, n 4096: 907 -> 470 us a
+// product).
 int inv_apply_many(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, float* X, int64_t m,
                    float* z, float* y) {
   {
@@ -1107,10 +1109,10 @@ int inv_apply_many(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, fl
     note_launch();
   }
   // y[c, j] = sum_i z[c, i] L^-1[j, i]: NT with B = L^-1 (row-major)
-  int rc = gemm_tf32x3(s, z, ldl, f.linvf, ldl, y, ldl, m, n, n, 1.f, 0.f, 0);
+  int rc = gemm_tf32x3(s, z, ldl, f.linvf, ldl, y, ldl, m, n, n, 1.f, 0.f, 0, 1);
   if (rc) return rc;
   // z[c, i] = sum_j y[c, j] L^-T[i, j]: NT with B = L^-T (row-major)
-  rc = gemm_tf32x3(s, y, ldl, f.uinv, ldl, z, ldl, m, n, n, 1.f, 0.f, 0);
+  rc = gemm_tf32x3(s, y, ldl, f.uinv, ldl, z, ldl, m, n, n, 1.f, 0.f, 0, 2);
   if (rc) return rc;
   {
     dim3 g((unsigned)ceil_div(n, 32), (unsigned)ceil_div(m, 32));

@@ -71,8 +71,8 @@ struct GemmArgs {
   float* c;
   int64_t ldc, m, n, k;
   float alpha, beta;
-  int32_t lower;
-  int32_t tiles_n;
+  int32_t lower, tri;
+  int32_t tiles_m, tiles_n;
   int* err;
 };
 
@@ -125,12 +125,18 @@ __global__ void __launch_bounds__(GTHREADS, 1)
     while ((i + 1) * (i + 2) / 2 <= idx) ++i;
     tm = i;
     tn = idx - i * (i + 1) / 2;
+  } else if (p.tri) {  // the column tiles with the longest sums first
+    tn = blockIdx.x / p.tiles_m;
+    tm = blockIdx.x - tn * p.tiles_m;
+    if (p.tri == 1) tn = p.tiles_n - 1 - tn;
   } else {
     tm = blockIdx.x / p.tiles_n;
     tn = blockIdx.x - tm * p.tiles_n;
   }
   const int64_t m0 = tm * GM, n0 = tn * GN;
-  const int nk = (int)((p.k + GK - 1) / GK);
+  // the k that this tile's rows of a triangular B can be non-zero at
+  const int64_t k0 = p.tri == 2 ? n0 : 0, k1 = p.tri == 1 && n0 + GN < p.k ? n0 + GN : p.k;
+  const int nk = (int)((k1 - k0 + GK - 1) / GK);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -167,8 +173,8 @@ __global__ void __launch_bounds__(GTHREADS, 1)
         const uint32_t full = tc::smem_u32(&bars[s]);
         uint8_t* st = smem + s * GSTAGE;
         tc::mbar_expect_tx(full, 2 * GTILE);
-        tc::tma_load_2d(tc::smem_u32(st), &ta, full, kc * GK, (int32_t)m0);
-        tc::tma_load_2d(tc::smem_u32(st + 2 * GTILE), &tb, full, kc * GK, (int32_t)n0);
+        tc::tma_load_2d(tc::smem_u32(st), &ta, full, (int32_t)k0 + kc * GK, (int32_t)m0);
+        tc::tma_load_2d(tc::smem_u32(st + 2 * GTILE), &tb, full, (int32_t)k0 + kc * GK, (int32_t)n0);
         issued = kc + 1;
       }
       if (!ok) {
@@ -319,7 +325,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
 
 int gemm_tf32x3(cudaStream_t s, const float* a, int64_t lda, const float* b, int64_t ldb,
                 float* c, int64_t ldc, int64_t m, int64_t n, int64_t k, float alpha, float beta,
-                int lower) {
+                int lower, int tri) {
   NTG_REQUIRE(a && b && c, "ntg_gemm_tc: null pointer");
   NTG_REQUIRE(m > 0 && n > 0 && k > 0, "ntg_gemm_tc: sizes must be positive");
   NTG_REQUIRE(lda >= k && ldb >= k && ldc >= n, "ntg_gemm_tc: leading dimensions too small");
@@ -328,6 +334,7 @@ int gemm_tf32x3(cudaStream_t s, const float* a, int64_t lda, const float* b, int
   NTG_REQUIRE((reinterpret_cast<uintptr_t>(a) & 15) == 0 && (reinterpret_cast<uintptr_t>(b) & 15) == 0,
               "ntg_gemm_tc: A and B must be 16-byte aligned");
   NTG_REQUIRE(!lower || m == n, "ntg_gemm_tc: the lower-triangle update needs m == n");
+  NTG_REQUIRE(tri == 0 || (n == k && !lower), "ntg_gemm_tc: a triangular B is square");
   NTG_REQUIRE(m <= (1ll << 31) - GM && n <= (1ll << 31) - GN && k <= (1ll << 31) - GK,
               "ntg_gemm_tc: sizes too large");
   const int64_t tm = ceil_div(m, GM), tn = ceil_div(n, GN);
@@ -348,7 +355,8 @@ int gemm_tf32x3(cudaStream_t s, const float* a, int64_t lda, const float* b, int
   });
   if (attr_err != cudaSuccess)
     return fail(NTG_ERR_CUDA, std::string("ntg_gemm_tc: ") + cudaGetErrorString(attr_err));
-  GemmArgs p{c, ldc, m, n, k, alpha, beta, lower, (int32_t)tn, device_error_word()};
+  GemmArgs p{c,     ldc, m,           n,           k, alpha, beta,
+             lower, tri, (int32_t)tm, (int32_t)tn, device_error_word()};
   NTG_REQUIRE(p.err, "ntg_gemm_tc: no device error word");
   gemm_tf32x3_kernel<<<(unsigned)tiles, GTHREADS, GSMEM, s>>>(ma, mb, p);
   note_launch();
@@ -361,5 +369,5 @@ extern "C" int ntg_gemm_tc(void* stream, const float* a, int64_t lda, const floa
                            int64_t ldb, float* c, int64_t ldc, int64_t m, int64_t n, int64_t k,
                            float alpha, float beta, int32_t lower) {
   return ntg::gemm_tf32x3(ntg::as_stream(stream), a, lda, b, ldb, c, ldc, m, n, k, alpha, beta,
-                          lower);
+                          lower, 0);
 }

@@ -194,3 +194,17 @@ def test_exact_residual_in_bands(nt):
         r = b2.double() - k.double() @ x64 - float(solver.lam[0]) * x64
         size = (k.abs().amax(1, keepdim=True) * x64.abs().amax(0, keepdim=True)).max()
         assert abs(float(solver.residual) - float(r.abs().max())) < n ** .5 * 2. ** -38 * float(size)
+
+
+@pytest.mark.parametrize('n,m', [(1, 17), (127, 17), (128, 130), (129, 40), (257, 17), (390, 300)])
+def test_many_right_hand_sides_at_tile_edges(nt, n, m):
+    """Products with the triangular inverses stop at the triangle, tile by tile: kappa <= 5, so
+    one refinement step leaves the float32 rounding of the solution."""
+    from nt_gb300 import predict
+    rng = np.random.default_rng(n)
+    q = rng.standard_normal((n, n))
+    a = np.eye(n) + q @ q.T / n  # eigenvalues in [1, 5 + o(1)]
+    b = rng.standard_normal((n, m)).astype(np.float32)
+    x = predict.CholeskySolver(_t(a), 0., True).solve(_t(b), refine_iters=1)
+    want = np.linalg.solve(a.astype(np.float32).astype(np.float64), b.astype(np.float64))
+    assert np.max(np.abs(x.cpu().numpy() - want)) < 1e-6 * np.max(np.abs(want))
