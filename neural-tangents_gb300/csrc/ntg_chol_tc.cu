@@ -530,7 +530,7 @@ __global__ void accumulate_tc_kernel(double* __restrict__ x, const float* __rest
 constexpr double kPcgTol = 1e-10;   // residual reduction from the starting point
 constexpr double kPcgFloor = 1e-15; // or residual below this times max |b|
 constexpr int kPcgStall = 2;        // or no halving of the best residual for this many steps
-constexpr int kDotBlocks = 128;
+constexpr int kDotBlocks = 304;     // two per SM
 
 struct PcgState {
   double rho[2][kSmallM];   // r.z of the current / next iteration
@@ -541,7 +541,35 @@ struct PcgState {
   double rmax[kSmallM];     // max |r_j| of the last residual
   int active[kSmallM];
   int all_done;
+  int ticket;               // blocks of the running kernel that have finished
 };
+
+// The kernels of a solve follow one another in a stream, most of them shorter than the gap
+// between two launches. Each lets the next one be set up while it runs and waits, before its
+// first access to memory, for the one before to have finished and its writes to be visible
+// (launch_next sets the launch attribute; without it both are no-ops). With the sums, splits
+// and checks of an iteration in the kernels next to them, 5000 points and ten right-hand sides
+// take 245 us an iteration (290 in twelve plain launches), an iteration after convergence,
+// eight kernels that return at once, 14 us (48).
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KA, typename... A>
+void launch_next(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
+  note_launch();
+}
 
 __device__ __forceinline__ void df_add(float& sh, float& sl, float bh, float bl) {
   const float s = sh + bh;
@@ -552,10 +580,11 @@ __device__ __forceinline__ void df_add(float& sh, float& sl, float bh, float bl)
 }
 
 // Columns [0, mc) of X (FP64 [n, ldx]) as double-float pairs xs[j, c] = (hi, lo) (pitch
-// mc), split once per product so that the row kernel below runs on the FP32 pipes only.
+// mc), split once per product so that the row kernel below runs on the FP32 pipes only; x32
+// (nullable, pitch mc): their float32 rounding.
 __global__ void split_df_kernel(const double* __restrict__ X, int64_t ldx, int64_t n, int64_t mc,
-                                float2* __restrict__ xs, const PcgState* st) {
-  if (st && st->all_done) return;
+                                float2* __restrict__ xs, float* __restrict__ x32) {
+  after_previous();
   const int64_t total = n * mc;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -563,6 +592,7 @@ __global__ void split_df_kernel(const double* __restrict__ X, int64_t ldx, int64
     const double v = X[j * ldx + c];
     const float h = (float)v;
     xs[i] = make_float2(h, (float)(v - (double)h));
+    if (x32) x32[i] = h;
   }
 }
 
@@ -585,6 +615,7 @@ __global__ void __launch_bounds__(kGT)
                      int64_t ks, int tri, const float* __restrict__ X,
                      const float2* __restrict__ xs, int64_t m, float* __restrict__ part,
                      float2* __restrict__ part2, const int* skip) {
+  after_previous();
   if (skip && *skip) return;
   constexpr int MRP = (MR + 3) & ~3;
   constexpr int NP = (MR + 1) / 2;           // packed column pairs (DF)
@@ -715,56 +746,100 @@ __device__ __forceinline__ void tile_range(int64_t row, int tri, int ks, int64_t
   hi = tri == 1 ? row / ks + 1 : nkb;
 }
 
-// Y[i, c] = sum of the row's tiles, in tile order (FP32 products).
-__global__ void gemv_reduce_kernel(const float* __restrict__ part, int64_t rows, int64_t m,
-                                   int tri, int ks, int64_t nkb, float* __restrict__ Y,
-                                   const int* skip) {
+// A block of 256 threads on [rows, m] arrays, m <= kSmallM: cw (the power of two from m on)
+// neighbouring threads take a row, so that a thread keeps its column.
+struct RowCol {
+  int64_t row, step;
+  int c;
+};
+__device__ __forceinline__ RowCol row_col(int64_t m) {
+  const int cw = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : m <= 8 ? 8 : 16, per = 256 / cw;
+  return RowCol{(int64_t)blockIdx.x * per + threadIdx.x / cw, (int64_t)gridDim.x * per,
+                (int)threadIdx.x % cw};
+}
+// The block's sums of v by column -> part[block][kSmallM].
+__device__ __forceinline__ void column_sums(double v, int64_t m, double* part) {
+  __shared__ double red[8][kSmallM];
+  const int cw = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : m <= 8 ? 8 : 16;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int o = 16; o >= cw; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane < cw) red[warp][lane] = v;
+  __syncthreads();
+  if (threadIdx.x < m) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[w][threadIdx.x];
+    part[blockIdx.x * kSmallM + threadIdx.x] = t;
+  }
+}
+
+// Y[i, c] = sum of the row's tiles, in tile order (FP32 products). Yd, xs (nullable): Y in FP64
+// and as a double-float split. r (nullable): the blocks' sums of r_c Y_c into dots. start:
+// clears the state for a new iteration.
+__global__ void __launch_bounds__(256)
+    gemv_reduce_kernel(const float* __restrict__ part, int64_t rows, int64_t m, int tri, int ks,
+                       int64_t nkb, float* __restrict__ Y, double* __restrict__ Yd,
+                       float2* __restrict__ xs, const double* __restrict__ r,
+                       double* __restrict__ dots, PcgState* start, const int* skip) {
+  after_previous();
   if (skip && *skip) return;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < rows * m;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = idx / m;
+  if (start && blockIdx.x == 0 && threadIdx.x == 0) start->all_done = start->ticket = 0;
+  const RowCol at = row_col(m);
+  double d = 0.0;
+  for (int64_t row = at.row; row < rows && at.c < m; row += at.step) {
+    const int64_t idx = row * m + at.c;
     int64_t lo, hi;
     tile_range(row, tri, ks, nkb, lo, hi);
     float v = 0.f;
+#pragma unroll 8
     for (int64_t kb = lo; kb < hi; ++kb) v += part[kb * rows * m + idx];
     Y[idx] = v;
+    if (Yd) Yd[idx] = (double)v;
+    if (xs) xs[idx] = make_float2(v, 0.f);
+    if (r) d = fma(r[idx], (double)v, d);
   }
+  if (r) column_sums(d, m, dots);
 }
 
 // Double-float products, finished: v = sum of the row's tiles (+ lambda X[i, c] when
 // lambda is given: the square (K + lambda I) x), then out = v (mode 0), b - v (mode 1)
 // or b + v (mode 2), b = B64 when given, else B (nullable: 0), as FP64 (out) and / or
-// FP32 (out32). B, B64, X, out and out32 have row pitch ldo (the tiles' pitch is m).
-__global__ void df_reduce_kernel(const float2* __restrict__ part2, int64_t rows, int64_t m,
+// FP32 (out32). B, B64, X, out and out32 have row pitch ldo (the tiles' pitch is m). dots
+// (nullable): the blocks' sums of X_c v_c.
+__global__ void __launch_bounds__(256) df_reduce_kernel(const float2* __restrict__ part2, int64_t rows, int64_t m,
                                  int64_t nkb, const double* lambda, const float* __restrict__ B,
                                  const double* __restrict__ B64, const double* __restrict__ X,
                                  int64_t ldo, int mode,
                                  double* __restrict__ out, float* __restrict__ out32,
-                                 const int* skip) {
+                                 double* __restrict__ dots, const int* skip) {
+  after_previous();
   if (skip && *skip) return;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < rows * m;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = idx / m, c = idx - row * m, o = row * ldo + c;
+  const RowCol at = row_col(m);
+  double d = 0.0;
+  for (int64_t row = at.row; row < rows && at.c < m; row += at.step) {
+    const int64_t idx = row * m + at.c, o = row * ldo + at.c;
     float hi = 0.f, lo = 0.f;
+#pragma unroll 4
     for (int64_t kb = 0; kb < nkb; ++kb) {
       const float2 p = part2[kb * rows * m + idx];
       df_add(hi, lo, p.x, p.y);
     }
     double v = (double)hi + (double)lo;
     if (lambda) v += lambda[0] * X[o];
+    if (dots) d = fma(X[o], v, d);
     const double b = B64 ? B64[o] : B ? (double)B[o] : 0.0;
     const double r = mode == 1 ? b - v : mode == 2 ? b + v : v;
     if (out) out[o] = r;
     if (out32) out32[o] = (float)r;
   }
+  if (dots) column_sums(d, m, dots);
 }
 
 template <int MR>
 void launch_df_part(cudaStream_t s, dim3 grid, const float* A, int64_t lda, int64_t rows,
                     int64_t ncols, int64_t ks, const float2* xs, int64_t m, float2* part2,
                     const int* skip) {
-  gemv_part_kernel<MR, true><<<grid, kGT, 0, s>>>(A, lda, rows, ncols, ks, 0, nullptr, xs, m,
-                                                  nullptr, part2, skip);
+  launch_next(s, gemv_part_kernel<MR, true>, grid, kGT, A, lda, rows, ncols, ks, 0, nullptr, xs,
+              m, nullptr, part2, skip);
 }
 
 size_t tri_part_bytes(int64_t n, int64_t m) {
@@ -781,7 +856,7 @@ void launch_matvec(cudaStream_t s, const float* A, int64_t lda, int64_t rows, in
                    const double* lambda, const float* B, const double* B64, const double* X,
                    const float2* xs,
                    int64_t m, int64_t ldo, int mode, double* out, float* out32, float2* part2,
-                   const PcgState* st) {
+                   double* dots, const PcgState* st) {
   const int* skip = st ? &st->all_done : nullptr;
   const int64_t ks = split_ks(rows, ncols, kFullTiles), nkb = ceil_div(ncols, ks);
   const dim3 grid((unsigned)nkb, (unsigned)ceil_div(rows, kGT));
@@ -793,120 +868,148 @@ void launch_matvec(cudaStream_t s, const float* A, int64_t lda, int64_t rows, in
 #undef NTG_MV
     default: launch_df_part<kSmallM>(s, grid, A, lda, rows, ncols, ks, xs, m, part2, skip);
   }
-  df_reduce_kernel<<<grid_for(rows * m), 256, 0, s>>>(part2, rows, m, nkb, lambda, B, B64, X,
-                                                      ldo, mode, out, out32, skip);
+  launch_next(s, df_reduce_kernel, dim3(kDotBlocks), 256, part2, rows, m, nkb, lambda, B, B64, X,
+              ldo, mode, out, out32, dots, skip);
 }
-// part[blk][j] = sum over the block's rows of u[i, j] * v[i, j] (v FP64, or vf FP32).
-__global__ void __launch_bounds__(256)
-    col_dots_kernel(const double* __restrict__ u, const double* __restrict__ v,
-                    const float* __restrict__ vf, int64_t n, int64_t m, double* __restrict__ part,
-                    const PcgState* st) {
-  if (st && st->all_done) return;  // st == nullptr: the set-up product, always computed
-  __shared__ double red[8][kSmallM];
-  double acc[kSmallM];
+
+// Sum of the blocks' parts of every column, by the 256 threads of a block -> out[kSmallM].
+__device__ __forceinline__ void sum_parts(const double* __restrict__ part, double* out) {
+  __shared__ double red[16][kSmallM];
+  const int c = threadIdx.x & 15, g = threadIdx.x >> 4;
+  double t = 0.0;
 #pragma unroll
-  for (int c = 0; c < kSmallM; ++c) acc[c] = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-#pragma unroll
-    for (int c = 0; c < kSmallM; ++c)
-      if (c < m) acc[c] = fma(u[i * m + c], vf ? (double)vf[i * m + c] : v[i * m + c], acc[c]);
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int c = 0; c < kSmallM; ++c) {
-    double x = acc[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) red[warp][c] = x;
+  for (int b = g; b < kDotBlocks; b += 16) t += part[b * kSmallM + c];
+  red[g][c] = t;
+  __syncthreads();
+  if (threadIdx.x < kSmallM) {
+    t = 0.0;
+    for (int w = 0; w < 16; ++w) t += red[w][threadIdx.x];
+    out[threadIdx.x] = t;
   }
   __syncthreads();
-  if (threadIdx.x < m) {
-    double t = 0.0;
-    for (int w = 0; w < 8; ++w) t += red[w][threadIdx.x];
-    part[blockIdx.x * kSmallM + threadIdx.x] = t;
-  }
 }
 
-__device__ __forceinline__ double sum_parts(const double* part, int c) {
+// Whether this block is the last of the grid to get here; its view of the others' writes is
+// then complete.
+__device__ __forceinline__ bool last_block(PcgState* st) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&st->ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// The maxima of non-negative values are taken on their 64-bit patterns, where a NaN is the
+// largest. max_parts: over all blocks' parts of every column, by the 256 threads of a block.
+__device__ __forceinline__ double pattern_max(double a, double b) {
+  return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+}
+
+__device__ __forceinline__ void max_parts(const double* part, double* out) {
+  __shared__ double red[16][kSmallM];
+  const int c = threadIdx.x & 15, g = threadIdx.x >> 4;
   double t = 0.0;
-  for (int b = 0; b < kDotBlocks; ++b) t += part[b * kSmallM + c];
-  return t;
+  for (int b = g; b < (int)gridDim.x; b += 16)
+    t = pattern_max(t, *reinterpret_cast<const volatile double*>(part + b * kSmallM + c));
+  red[g][c] = t;
+  __syncthreads();
+  if (threadIdx.x < kSmallM) {
+    for (int w = 0; w < 16; ++w) t = pattern_max(t, red[w][threadIdx.x]);
+    out[threadIdx.x] = t;
+  }
+  __syncthreads();
 }
 
-// Set-up: bnorm, r0norm, rho[0] = r.z (from part), p = z, every column active.
-__global__ void pcg_init_kernel(const float* __restrict__ B, const float* __restrict__ z,
-                                double* __restrict__ p, const double* __restrict__ r, int64_t n,
-                                int64_t m, const double* __restrict__ part, PcgState* st) {
-  __shared__ double bmax[kSmallM], rmax[kSmallM];
+__device__ __forceinline__ void block_max(double* slot, double v) {
+  atomicMax(reinterpret_cast<unsigned long long*>(slot),
+            (unsigned long long)__double_as_longlong(fabs(v)));
+}
+
+// Set-up: p = z and its split; bnorm, r0norm, rho[0] = r.z (from part), every column active.
+// bpart, rpart: the blocks' maxima.
+__global__ void __launch_bounds__(256)
+    pcg_init_kernel(const float* __restrict__ B, const float* __restrict__ z,
+                    double* __restrict__ p, float2* __restrict__ xs, const double* __restrict__ r,
+                    int64_t n, int64_t m, const double* __restrict__ part, double* bpart,
+                    double* rpart, PcgState* st) {
+  after_previous();
+  __shared__ double bmax[kSmallM], rmax[kSmallM], rho[kSmallM];
   if (threadIdx.x < kSmallM) bmax[threadIdx.x] = rmax[threadIdx.x] = 0.0;
   __syncthreads();
-  for (int64_t i = threadIdx.x; i < n * m; i += blockDim.x) {
+  const RowCol at = row_col(m);
+  double bm = 0.0, rm = 0.0;
+  for (int64_t row = at.row; row < n && at.c < m; row += at.step) {
+    const int64_t i = row * m + at.c;
     p[i] = (double)z[i];
-    const int c = (int)(i % m);
-    atomicMax(reinterpret_cast<unsigned long long*>(&bmax[c]),
-              (unsigned long long)__double_as_longlong(fabs((double)B[i])));
-    atomicMax(reinterpret_cast<unsigned long long*>(&rmax[c]),
-              (unsigned long long)__double_as_longlong(fabs(r[i])));
+    xs[i] = make_float2(z[i], 0.f);
+    bm = pattern_max(bm, fabs((double)B[i]));
+    rm = pattern_max(rm, fabs(r[i]));
+  }
+  if (at.c < m) {
+    block_max(&bmax[at.c], bm);
+    block_max(&rmax[at.c], rm);
   }
   __syncthreads();
+  if (threadIdx.x < kSmallM) {
+    bpart[blockIdx.x * kSmallM + threadIdx.x] = bmax[threadIdx.x];
+    rpart[blockIdx.x * kSmallM + threadIdx.x] = rmax[threadIdx.x];
+  }
+  if (!last_block(st)) return;
+  max_parts(bpart, bmax);
+  max_parts(rpart, rmax);
+  sum_parts(part, rho);
   if (threadIdx.x < m) {
     const int c = threadIdx.x;
     st->bnorm[c] = bmax[c];
     st->r0norm[c] = rmax[c];
     st->rbest[c] = rmax[c];
     st->stall[c] = 0;
-    st->rho[0][c] = sum_parts(part, c);
+    st->rho[0][c] = rho[c];
     st->rmax[c] = rmax[c];
     st->active[c] = rmax[c] > kPcgFloor * bmax[c];
   }
-  if (threadIdx.x == 0) st->all_done = 0;
+  if (threadIdx.x == 0) st->ticket = 0;
 }
 
-// x += alpha p, r -= alpha q (alpha_c = rho_c / p.q), r32 = (float) r; the block's
-// max |r_c| into rpart.
+// x += alpha p, r -= alpha q (alpha_c = rho_c / p.q), r32 = (float) r; then, in the last
+// block, the convergence of each column by max |r_c|: one at or below kPcgTol max |b_c|
+// stops; all_done once none is left.
 __global__ void __launch_bounds__(256)
     pcg_step_kernel(double* __restrict__ x, double* __restrict__ r, float* __restrict__ r32,
                     const double* __restrict__ p, const double* __restrict__ q, int64_t n,
-                    int64_t m, const double* __restrict__ pq_part, double* __restrict__ rpart,
-                    PcgState* st, int cur) {
+                    int64_t m, const double* __restrict__ pq_part, double* rpart, PcgState* st,
+                    int cur) {
+  after_previous();
   if (st->all_done) return;
-  __shared__ double alpha[kSmallM];
-  __shared__ double rmax[kSmallM];
-  if (threadIdx.x < m) {
-    const int c = threadIdx.x;
-    const double pq = sum_parts(pq_part, c);
-    alpha[c] = (st->active[c] && pq > 0.0) ? st->rho[cur][c] / pq : 0.0;
-    rmax[c] = 0.0;
-  }
-  __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * m; i += stride) {
-    const int c = (int)(i % m);
-    const double a = alpha[c];
-    x[i] = fma(a, p[i], x[i]);
-    const double rv = fma(-a, q[i], r[i]);
-    r[i] = rv;
-    r32[i] = (float)rv;
-    atomicMax(reinterpret_cast<unsigned long long*>(&rmax[c]),
-              (unsigned long long)__double_as_longlong(fabs(rv)));
-  }
-  __syncthreads();
-  if (threadIdx.x < m) rpart[blockIdx.x * kSmallM + threadIdx.x] = rmax[threadIdx.x];
-}
-
-// Convergence: max |r_c| over the blocks' maxima; a column at or below kPcgTol max |b_c|
-// stops; all_done once none is left.
-__global__ void pcg_check_kernel(const double* __restrict__ rpart, int64_t m, int nblocks,
-                                 PcgState* st) {
-  if (st->all_done) return;
+  __shared__ double pq[kSmallM], rmax[kSmallM];
   __shared__ int any;
+  if (threadIdx.x < kSmallM) rmax[threadIdx.x] = 0.0;
   if (threadIdx.x == 0) any = 0;
+  sum_parts(pq_part, pq);
+  const RowCol at = row_col(m);
+  double rm = 0.0;
+  if (at.c < m) {
+    const int c = at.c;
+    const double a = (st->active[c] && pq[c] > 0.0) ? st->rho[cur][c] / pq[c] : 0.0;
+    for (int64_t row = at.row; row < n; row += at.step) {
+      const int64_t i = row * m + c;
+      x[i] = fma(a, p[i], x[i]);
+      const double rv = fma(-a, q[i], r[i]);
+      r[i] = rv;
+      r32[i] = (float)rv;
+      rm = pattern_max(rm, fabs(rv));
+    }
+    block_max(&rmax[c], rm);
+  }
   __syncthreads();
+  if (threadIdx.x < kSmallM) rpart[blockIdx.x * kSmallM + threadIdx.x] = rmax[threadIdx.x];
+  if (!last_block(st)) return;
+  max_parts(rpart, rmax);
   if (threadIdx.x < m) {
     const int c = threadIdx.x;
-    double mx = 0.0;
-    for (int b = 0; b < nblocks; ++b) mx = fmax(mx, rpart[b * kSmallM + c]);
+    const double mx = rmax[c];
     st->rmax[c] = mx;
     // the double-float products put a floor under the residual: a column whose best
     // residual has not halved in kPcgStall iterations has reached it and stops
@@ -922,35 +1025,34 @@ __global__ void pcg_check_kernel(const double* __restrict__ rpart, int64_t m, in
     if (st->active[c]) atomicOr(&any, 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0 && !any) st->all_done = 1;
+  if (threadIdx.x == 0) {
+    st->ticket = 0;
+    if (!any) st->all_done = 1;
+  }
 }
 
-// beta_c = (r.z)_new / rho_c; p = z + beta p; rho[nxt] = (r.z)_new.
+// beta_c = (r.z)_new / rho_c; p = z + beta p and its split; rho[nxt] = (r.z)_new.
 __global__ void __launch_bounds__(256)
-    pcg_dir_kernel(double* __restrict__ p, const float* __restrict__ z, int64_t n, int64_t m,
-                   const double* __restrict__ rz_part, PcgState* st, int cur) {
+    pcg_dir_kernel(double* __restrict__ p, float2* __restrict__ xs, const float* __restrict__ z,
+                   int64_t n, int64_t m, const double* __restrict__ rz_part, PcgState* st,
+                   int cur) {
+  after_previous();
   if (st->all_done) return;
-  __shared__ double beta[kSmallM];
+  __shared__ double rz[kSmallM];
+  sum_parts(rz_part, rz);
   const int nxt = cur ^ 1;
-  if (threadIdx.x < m) {
-    const int c = threadIdx.x;
-    const double rz = sum_parts(rz_part, c);
-    beta[c] = st->rho[cur][c] != 0.0 ? rz / st->rho[cur][c] : 0.0;
-    if (blockIdx.x == 0) st->rho[nxt][c] = rz;
+  const RowCol at = row_col(m);
+  if (at.c >= m) return;
+  const double beta = st->rho[cur][at.c] != 0.0 ? rz[at.c] / st->rho[cur][at.c] : 0.0;
+  if (blockIdx.x == 0 && threadIdx.x == at.c) st->rho[nxt][at.c] = rz[at.c];
+  if (!st->active[at.c]) return;
+  for (int64_t row = at.row; row < n; row += at.step) {
+    const int64_t i = row * m + at.c;
+    const double v = fma(beta, p[i], (double)z[i]);
+    p[i] = v;
+    const float h = (float)v;
+    xs[i] = make_float2(h, (float)(v - (double)h));
   }
-  __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * m; i += stride) {
-    const int c = (int)(i % m);
-    if (st->active[c]) p[i] = fma(beta[c], p[i], (double)z[i]);
-  }
-}
-
-__global__ void copy_to_float_kernel(const double* __restrict__ a, float* __restrict__ b,
-                                     int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    b[i] = (float)a[i];
 }
 
 __global__ void logdet_ld_kernel(const float* __restrict__ L, int64_t n, int64_t ldl,
@@ -1071,17 +1173,19 @@ size_t solve_ws_bytes(int64_t n, int64_t m, int64_t ldl) {
 
 // X = (L L^T)^-1 X for up to kSmallM right-hand sides: t = L^-1 X, X = L^-T t, each a
 // split-K triangular product (gemv_part_kernel) and its reduction; tpart holds
-// tri_part_bytes(n, m).
+// tri_part_bytes(n, m). Xd, xs, r, dots, start: of the last reduction (gemv_reduce_kernel).
 template <int MR>
 void launch_tri_part(cudaStream_t s, dim3 grid, const float* M, int64_t ld, int64_t n,
                      int64_t ks, int tri, const float* X, int64_t m, float* part,
                      const int* skip) {
-  gemv_part_kernel<MR, false><<<grid, kGT, 0, s>>>(M, ld, n, n, ks, tri, X, nullptr, m, part,
-                                                   nullptr, skip);
+  launch_next(s, gemv_part_kernel<MR, false>, grid, kGT, M, ld, n, n, ks, tri, X, nullptr, m,
+              part, nullptr, skip);
 }
 
 int inv_apply_small(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, float* X, int64_t m,
-                    float* t, float* tpart, const int* skip) {
+                    float* t, float* tpart, const int* skip, double* Xd = nullptr,
+                    float2* xs = nullptr, const double* r = nullptr, double* dots = nullptr,
+                    PcgState* start = nullptr) {
   const int64_t ks = split_ks(n, n, kTriTiles), nkb = ceil_div(n, ks);
   const dim3 grid((unsigned)nkb, (unsigned)ceil_div(n, kGT));
   auto tri = [&](const float* M, int tri, const float* in, float* out) {
@@ -1089,11 +1193,13 @@ int inv_apply_small(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, f
     else if (m <= 4) launch_tri_part<4>(s, grid, M, ldl, n, ks, tri, in, m, tpart, skip);
     else if (m <= 10) launch_tri_part<10>(s, grid, M, ldl, n, ks, tri, in, m, tpart, skip);
     else launch_tri_part<kSmallM>(s, grid, M, ldl, n, ks, tri, in, m, tpart, skip);
-    gemv_reduce_kernel<<<grid_for(n * m), 256, 0, s>>>(tpart, n, m, tri, (int)ks, nkb, out, skip);
+    const bool last = tri == 2;
+    launch_next(s, gemv_reduce_kernel, dim3(kDotBlocks), 256, tpart, n, m, tri, (int)ks, nkb, out,
+                last ? Xd : nullptr, last ? xs : nullptr, last ? r : nullptr, dots,
+                last ? start : nullptr, skip);
   };
   tri(f.linvf, 1, X, t);  // L^-1: lower
   tri(f.uinv, 2, t, X);   // L^-T: upper
-  note_launch(4);
   return check_launch("ntg_chol_solve_tc apply");
 }
 
@@ -1283,23 +1389,21 @@ extern "C" int ntg_chol_solve_tc(void* stream, const float* A, const float* L, i
   float* tpart = reinterpret_cast<float*>(align256(xs + n * m));
   float2* dpart = reinterpret_cast<float2*>(align256(reinterpret_cast<char*>(tpart) +
                                                      tri_part_bytes(n, m)));
-  auto apply = [&](float* xx, const int* skip) -> int {
-    if (m <= kSmallM) return inv_apply_small(s, f, ldl, n, xx, m, t32, tpart, skip);
-    return inv_apply_many(s, f, ldl, n, xx, m, z, y);
-  };
   if (cudaMemcpyAsync(X, B, sizeof(float) * n * m, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return check_launch("ntg_chol_solve_tc copy");
-  rc = apply(X, nullptr);
+  const bool few = m <= kSmallM, only = refine_iters == 0 && !final_residual;
+  rc = few ? inv_apply_small(s, f, ldl, n, X, m, t32, tpart, nullptr, only ? x64_out : x64,
+                             only ? nullptr : xs)
+           : inv_apply_many(s, f, ldl, n, X, m, z, y);
   if (rc) return rc;
-  if (refine_iters == 0 && !final_residual) {
-    if (x64_out) {
-      to_double_tc_kernel<<<grid_for(n * m), 256, 0, s>>>(X, x64_out, n * m);
+  if (!few) {
+    double* const xd = only ? x64_out : x64;
+    if (xd) {
+      to_double_tc_kernel<<<grid_for(n * m), 256, 0, s>>>(X, xd, n * m);
       note_launch();
     }
-    return check_launch("ntg_chol_solve_tc");
   }
-  to_double_tc_kernel<<<grid_for(n * m), 256, 0, s>>>(X, x64, n * m);
-  note_launch();
+  if (only) return check_launch("ntg_chol_solve_tc");
   // the FP64 solution, for products that must keep its precision (ntg_gemm_df)
   auto copy_x64 = [&]() -> int {
     if (x64_out && cudaMemcpyAsync(x64_out, x64, sizeof(double) * n * m,
@@ -1307,47 +1411,42 @@ extern "C" int ntg_chol_solve_tc(void* stream, const float* A, const float* L, i
       return check_launch("ntg_chol_solve_tc solution copy");
     return NTG_OK;
   };
-  if (m <= kSmallM) {
+  if (few) {
     // preconditioned conjugate gradients on (K + lambda I) x = b from x0 = (L L^T)^-1 b;
-    // (K + lambda I) v for v = x64 or p64 (subtract: b - ...), through the split of v
+    // (K + lambda I) v for v = x64 or p64 (subtract: b - ...), through the split of v in xs,
+    // which the kernel that wrote v has left there
     auto matvec = [&](const double* v, int subtract, const float* bb, double* out, float* o32,
-                      const PcgState* stp) {
-      split_df_kernel<<<grid_for(n * m), 256, 0, s>>>(v, m, n, m, xs, stp);
+                      double* dots, const PcgState* stp) {
       launch_matvec(s, A, n, n, n, lambda, bb, bb ? B64 : nullptr, v, xs, m, m, subtract, out, o32,
-                    dpart, stp);
-      note_launch(3);
+                    dpart, dots, stp);
     };
-    matvec(x64, 1, B, r64, r32, nullptr);
     if (refine_iters > 0) {
-      rc = apply(r32, nullptr);  // z0
+      matvec(x64, 1, B, r64, r32, nullptr, nullptr);
+      rc = inv_apply_small(s, f, ldl, n, r32, m, t32, tpart, nullptr, nullptr, nullptr, r64,
+                           part_rz, st);  // z0
       if (rc) return rc;
-      col_dots_kernel<<<kDotBlocks, 256, 0, s>>>(r64, nullptr, r32, n, m, part_rz, nullptr);
-      pcg_init_kernel<<<1, 1024, 0, s>>>(B, r32, p64, r64, n, m, part_rz, st);
-      note_launch(2);
+      launch_next(s, pcg_init_kernel, dim3(kDotBlocks), 256, B, r32, p64, xs, r64, n, m, part_rz,
+                  part, part_r, st);
       for (int it = 0; it < refine_iters; ++it) {
         const int cur = it & 1;
-        matvec(p64, 0, nullptr, q64, nullptr, st);
-        col_dots_kernel<<<kDotBlocks, 256, 0, s>>>(p64, q64, nullptr, n, m, part, st);
-        pcg_step_kernel<<<kDotBlocks, 256, 0, s>>>(x64, r64, r32, p64, q64, n, m, part, part_r,
-                                                   st, cur);
-        pcg_check_kernel<<<1, 32, 0, s>>>(part_r, m, kDotBlocks, st);
-        note_launch(4);
-        rc = apply(r32, &st->all_done);
+        matvec(p64, 0, nullptr, q64, nullptr, part, st);
+        launch_next(s, pcg_step_kernel, dim3(kDotBlocks), 256, x64, r64, r32, p64, q64, n, m, part,
+                    part_r, st, cur);
+        rc = inv_apply_small(s, f, ldl, n, r32, m, t32, tpart, &st->all_done, nullptr, nullptr,
+                             r64, part_rz);
         if (rc) return rc;
-        col_dots_kernel<<<kDotBlocks, 256, 0, s>>>(r64, nullptr, r32, n, m, part_rz, st);
-        pcg_dir_kernel<<<kDotBlocks, 256, 0, s>>>(p64, r32, n, m, part_rz, st, cur);
-        note_launch(2);
+        launch_next(s, pcg_dir_kernel, dim3(kDotBlocks), 256, p64, xs, r32, n, m, part_rz, st,
+                    cur);
       }
-      copy_to_float_kernel<<<grid_for(n * m), 256, 0, s>>>(x64, X, n * m);
-      note_launch();
+      launch_next(s, split_df_kernel, dim3(grid_for(n * m)), 256, x64, m, n, m, xs, X);
     }
     if (final_residual) {
       // the true residual of the returned solution
-      matvec(x64, 1, B, r64, nullptr, nullptr);
+      matvec(x64, 1, B, r64, nullptr, nullptr, nullptr);
       if (cudaMemsetAsync(rnorm, 0, sizeof(double), s) != cudaSuccess)
         return check_launch("ntg_chol_solve_tc memset");
       max_abs64_kernel<<<grid_for(n * m), 256, 0, s>>>(r64, n * m, rnorm);
-      note_launch(2);
+      note_launch();
       if (cudaMemcpyAsync(final_residual, rnorm, sizeof(double), cudaMemcpyDeviceToDevice, s) !=
           cudaSuccess)
         return check_launch("ntg_chol_solve_tc residual copy");
@@ -1366,13 +1465,13 @@ extern "C" int ntg_chol_solve_tc(void* stream, const float* A, const float* L, i
       rc = exact_residual(s, A, n, lambda, B, B64, x64, m, r32, rnorm, xsplit, it > 0);
       if (rc) return rc;
     } else {
-      split_df_kernel<<<grid_for(n * m), 256, 0, s>>>(x64, m, n, m, xsplit, nullptr);
+      launch_next(s, split_df_kernel, dim3(grid_for(n * m)), 256, x64, m, n, m, xsplit, nullptr);
       residual_df_kernel<<<dim3((unsigned)ceil_div(m, 64), (unsigned)ceil_div(n, 64)), 256, 0, s>>>(
           A, n, lambda, B, B64, x64, xsplit, m, r32, rnorm);
-      note_launch(2);
+      note_launch();
     }
     if (it == refine_iters) break;
-    rc = apply(r32, nullptr);
+    rc = inv_apply_many(s, f, ldl, n, r32, m, z, y);
     if (rc) return rc;
     accumulate_tc_kernel<<<grid_for(n * m), 256, 0, s>>>(x64, r32, X, n * m);
     note_launch();
@@ -1406,10 +1505,9 @@ extern "C" int ntg_gemm_df(void* stream, const float* A, int64_t lda, int64_t ro
       (reinterpret_cast<uintptr_t>(xs + n * mini(m, kSmallM)) + 255) & ~(uintptr_t)255);
   for (int64_t c0 = 0; c0 < m; c0 += kSmallM) {
     const int64_t mc = mini(kSmallM, m - c0);
-    split_df_kernel<<<grid_for(n * mc), 256, 0, s>>>(X + c0, m, n, mc, xs, nullptr);
+    launch_next(s, split_df_kernel, dim3(grid_for(n * mc)), 256, X + c0, m, n, mc, xs, nullptr);
     launch_matvec(s, A, lda, rows, n, nullptr, Y0 ? Y0 + c0 : nullptr, nullptr, nullptr, xs, mc,
-                  m, 2, Y64 ? Y64 + c0 : nullptr, Y ? Y + c0 : nullptr, dpart, nullptr);
-    note_launch(3);
+                  m, 2, Y64 ? Y64 + c0 : nullptr, Y ? Y + c0 : nullptr, dpart, nullptr, nullptr);
   }
   return check_launch("ntg_gemm_df");
 }

@@ -208,3 +208,26 @@ def test_many_right_hand_sides_at_tile_edges(nt, n, m):
     x = predict.CholeskySolver(_t(a), 0., True).solve(_t(b), refine_iters=1)
     want = np.linalg.solve(a.astype(np.float32).astype(np.float64), b.astype(np.float64))
     assert np.max(np.abs(x.cpu().numpy() - want)) < 1e-6 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize('n,m', [(1, 1), (15, 2), (16, 3), (17, 5), (129, 8), (300, 9), (513, 16),
+                                 (4865, 4)])
+def test_few_right_hand_sides_by_rows_and_columns(nt, n, m):
+    """Conjugate-gradient solves at the edges of the row-and-column layout (a power of two of
+    threads a row, 304 blocks): kappa <= 5 converges to the float32 rounding of the solution;
+    one column zero, which stays zero."""
+    from nt_gb300 import predict
+    rng = np.random.default_rng(n)
+    q = rng.standard_normal((n, min(n, 200)))
+    a = (np.eye(n) + q @ q.T / max(n, 200)).astype(np.float32)
+    b = rng.standard_normal((n, m)).astype(np.float32)
+    b[:, -1] *= float(m == 1)
+    solver = predict.CholeskySolver(_t(a), 0., True)
+    x = solver.solve(_t(b)).cpu().numpy()
+    want = np.linalg.solve(a.astype(np.float64), b.astype(np.float64))
+    assert np.max(np.abs(x - want)) < 1e-6 * np.max(np.abs(want))
+    assert m == 1 or np.max(np.abs(x[:, -1])) == 0.
+    r = b - a.astype(np.float64) @ x
+    # of the returned FP64 solution: below that of its float32 rounding, 2^-24 |A| |x|
+    assert float(solver.residual) <= np.max(np.abs(r)) + 2. ** -24 * np.max(
+        np.abs(a).astype(np.float64) @ np.abs(x))
