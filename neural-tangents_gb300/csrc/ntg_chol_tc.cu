@@ -2,15 +2,18 @@
 // the sm_103a tensor cores (neural_tangents/_src/predict.py:1224-1258 restated
 // for the GPU): A = K + lambda I = L L^T in FP32 with 128-wide panels.
 //
-// Per panel k:
+// Per panel k, on a chain of its own:
 //   diag_block_kernel   one CTA factors the 128 x 128 diagonal block (four
 //                       32-wide steps, each a warp-level Cholesky + inverse in
 //                       registers overlapped with the other warps' deferred
 //                       updates, then the sub-panel and the next column block as
 //                       register-tiled warp products in shared memory) and writes
 //                       the block's inverse L11^-1;
-//   gemm_tf32x3         the rows below: L21 = A21 L11^-T as a product with that
-//                       inverse (in place, one 128-wide column of tiles);
+//   next_tile_kernel    the first tile of the rows below, L21 = A21 L11^-T as a product with
+//                       that inverse, and its update of the next diagonal block;
+// beside it:
+//   gemm_tf32x3         the other rows of L21 (in place, one 128-wide column of tiles) and
+//                       of the next column block;
 //   gemm_tf32x3 lower   the trailing update A22 -= L21 L21^T on the tensor cores
 //                       (3xTF32 products, FP32 accumulation; tiles on or below the
 //                       diagonal only).
@@ -58,6 +61,39 @@ int grid_for(int64_t n) {
 // Set-up
 // ---------------------------------------------------------------------------
 
+// The kernels of a solve follow one another in a stream, most of them shorter than the gap
+// between two launches. Each lets the next one be set up while it runs and waits, before its
+// first access to memory, for the one before to have finished and its writes to be visible
+// (launch_next sets the launch attribute; without it both are no-ops). With the sums, splits
+// and checks of an iteration in the kernels next to them, 5000 points and ten right-hand sides
+// take 245 us an iteration (290 in twelve plain launches), an iteration after convergence,
+// eight kernels that return at once, 14 us (48).
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KA, typename... A>
+void launch_next_smem(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, size_t smem,
+                      A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
+  note_launch();
+}
+template <typename... KA, typename... A>
+void launch_next(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, A... args) {
+  launch_next_smem(s, kernel, grid, threads, 0, args...);
+}
+
 __global__ void trace_tc_kernel(const float* __restrict__ A, int64_t n, double* __restrict__ out) {
   double s = 0.0;
   for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += (double)A[i * n + i];
@@ -89,6 +125,92 @@ __global__ void init_factor_ld_kernel(const float* __restrict__ A, int64_t n, in
     else if (j == i) v = (float)((double)A[i * n + i] + lam);
     L[idx] = v;
   }
+}
+
+// ---------------------------------------------------------------------------
+// What the next diagonal block waits for
+// ---------------------------------------------------------------------------
+
+// d += A B^T of one m16n8k8 TF32 product (mma.sync, row-major A, B given as rows of k).
+__device__ __forceinline__ void mma_tf32_16x8(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
+                                              uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
+}
+
+// The first tile of panel k, L21 = A21 L11^-T (UPDATE false: rows k + 128 .., in place), then its
+// update of the diagonal block behind it, A22 -= L21 L21^T (UPDATE, lower part): all that the
+// next diagonal block waits for. Eight CTAs of 16 rows, each warp 16 columns, 3xTF32 on
+// mma.sync straight from L2: 128 x 128 x 128 is too short for the set-up of a tcgen05 pipeline
+// (10 - 13 us and a gap of 3 - 5 in gemm_tf32x3, 5 us here with the launches overlapped; both
+// products in one CTA 27 us), and without shared memory the CTAs fit beside those of the
+// trailing update. A panel of a 5000-point factorisation takes 50 - 58 us (66), bound from
+// there on by the trailing update and the inverse, which share the SMs.
+template <bool UPDATE>
+__global__ void __launch_bounds__(256)
+    next_tile_kernel(float* __restrict__ L, int64_t ldl, int64_t n, int64_t k, const float* linv) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nb = (int)mini(PB, n - k - PB);
+  const int r0 = blockIdx.x * 16, c0 = (threadIdx.x >> 5) * 16;
+  float* const a21 = L + (k + PB) * ldl + k;
+  const bool idle = UPDATE && c0 > r0 + 15;
+  // L11^-1 is lower triangular: its rows c0 .. c0 + 15 end at column c0 + 15
+  const int K = UPDATE ? PB : c0 + 16;
+  const float* const B = UPDATE ? a21 : linv;
+  const int64_t ldb = UPDATE ? ldl : PB;
+  const int nbr = UPDATE ? nb : PB;
+  after_previous();
+  if (idle) return;
+  float acc[2][4] = {};
+  // Thread t of four holds the words 4 t .. 4 t + 3 of 16 consecutive k and hands them to two
+  // products, (0, 1) as their k = t and t + 4, then (2, 3): the same order of k in A and B.
+#pragma unroll 4
+  for (int kb = 0; kb < K; kb += 16) {
+    float4 av[2], bv[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int ra = r0 + g + 8 * h, rb = c0 + g + 8 * h;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      av[h] = ra < nb ? *reinterpret_cast<const float4*>(a21 + ra * ldl + kb + 4 * t) : zero;
+      bv[h] = rb < nbr ? *reinterpret_cast<const float4*>(B + rb * ldb + kb + 4 * t) : zero;
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      uint32_t ah[4], al[4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        split_tf32(s ? av[h].z : av[h].x, ah[h], al[h]);
+        split_tf32(s ? av[h].w : av[h].y, ah[2 + h], al[2 + h]);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint32_t h0, l0, h1, l1;
+        split_tf32(s ? bv[j].z : bv[j].x, h0, l0);
+        split_tf32(s ? bv[j].w : bv[j].y, h1, l1);
+        mma_tf32_16x8(acc[j], al, h0, h1);
+        mma_tf32_16x8(acc[j], ah, l0, l1);
+        mma_tf32_16x8(acc[j], ah, h0, h1);
+      }
+    }
+  }
+  if (!UPDATE) __syncthreads();  // the rows are read by every warp before they are written
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = r0 + g + 8 * (e >> 1), c = c0 + 8 * j + 2 * t + (e & 1);
+      if (i >= nb) continue;
+      if (!UPDATE) a21[i * ldl + c] = acc[j][e];
+      else if (c <= i) a21[i * ldl + PB + c] -= acc[j][e];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -241,6 +363,7 @@ __global__ void __launch_bounds__(512, 1)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r0 = (lane >> 3) * 8, c0 = (lane & 7) * 4;
   const int nb = (int)mini(PB, n - k);
+  after_previous();
   if (nb == PB) {
     // full block (16-byte aligned: ldl % 4 == 0, k % 128 == 0): all eight 16-byte loads
     // of a thread in flight at once; entries above the diagonal are not read
@@ -543,33 +666,6 @@ struct PcgState {
   int all_done;
   int ticket;               // blocks of the running kernel that have finished
 };
-
-// The kernels of a solve follow one another in a stream, most of them shorter than the gap
-// between two launches. Each lets the next one be set up while it runs and waits, before its
-// first access to memory, for the one before to have finished and its writes to be visible
-// (launch_next sets the launch attribute; without it both are no-ops). With the sums, splits
-// and checks of an iteration in the kernels next to them, 5000 points and ten right-hand sides
-// take 245 us an iteration (290 in twelve plain launches), an iteration after convergence,
-// eight kernels that return at once, 14 us (48).
-__device__ __forceinline__ void after_previous() {
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... KA, typename... A>
-void launch_next(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
-  note_launch();
-}
 
 __device__ __forceinline__ void df_add(float& sh, float& sl, float bh, float bl) {
   const float s = sh + bh;
@@ -1088,14 +1184,15 @@ int attrs_once() {
   return rc;
 }
 
-// Per-device streams and events of the factorisation: the critical chain (diagonal
-// block, panel product, update of the next column block) on a high-priority stream,
-// the bulk of each trailing update on a second stream one panel behind it, and the
-// inverse factor L^-T, block by block as the panels become final, on a third.
+// Per-device streams and events of the factorisation: the critical chain (diagonal block,
+// next_tile_kernel) and, beside it, the rest of the panel and of the next column block on
+// high-priority streams, the bulk of each trailing update on a third stream one panel behind
+// them, and the inverse factor L^-T, block by block as the panels become final, on a fourth.
 struct SideStream {
-  cudaStream_t hi = nullptr, trail = nullptr, side = nullptr;
-  cudaEvent_t fork = nullptr, panel = nullptr, trail_done = nullptr;
-  cudaEvent_t join[3] = {nullptr, nullptr, nullptr};
+  cudaStream_t hi = nullptr, near = nullptr, trail = nullptr, side = nullptr;
+  cudaEvent_t fork = nullptr, diag = nullptr, next = nullptr, panel = nullptr, column = nullptr,
+              trail_done = nullptr;
+  cudaEvent_t join[4] = {nullptr, nullptr, nullptr, nullptr};
   // held while one factorisation enqueues its work: the events are re-recorded per panel,
   // and two host threads interleaving their records and waits would order each other's
   // launches (a wait, once enqueued, is not affected by a later record)
@@ -1114,10 +1211,11 @@ int side_stream(SideStream** out) {
     int least = 0, greatest = 0;
     bool ok = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess;
     ok = ok && cudaStreamCreateWithPriority(&ss.hi, cudaStreamNonBlocking, greatest) == cudaSuccess;
+    ok = ok && cudaStreamCreateWithPriority(&ss.near, cudaStreamNonBlocking, greatest) == cudaSuccess;
     ok = ok && cudaStreamCreateWithPriority(&ss.trail, cudaStreamNonBlocking, least) == cudaSuccess;
     ok = ok && cudaStreamCreateWithPriority(&ss.side, cudaStreamNonBlocking, least) == cudaSuccess;
-    cudaEvent_t* evs[6] = {&ss.fork, &ss.panel, &ss.trail_done, &ss.join[0], &ss.join[1],
-                           &ss.join[2]};
+    cudaEvent_t* evs[10] = {&ss.fork,       &ss.diag,    &ss.next,    &ss.panel,   &ss.column,
+                            &ss.trail_done, &ss.join[0], &ss.join[1], &ss.join[2], &ss.join[3]};
     for (cudaEvent_t* e : evs)
       ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
@@ -1273,61 +1371,63 @@ extern "C" int ntg_chol_factor_tc(void* stream, const float* A, int64_t n, doubl
     return cudaEventRecord(e, from) == cudaSuccess && cudaStreamWaitEvent(to, e, 0) == cudaSuccess;
   };
   if (!record_wait(ss->fork, s, ss->hi) || cudaStreamWaitEvent(ss->trail, ss->fork, 0) ||
-      cudaStreamWaitEvent(ss->side, ss->fork, 0))
+      cudaStreamWaitEvent(ss->side, ss->fork, 0) || cudaStreamWaitEvent(ss->near, ss->fork, 0))
     return check_launch("ntg_chol_factor_tc fork");
-  // every return after the fork joins the three streams back into s
+  // every return after the fork joins the four streams back into s
   auto join = [&]() -> int {
-    const cudaStream_t from[3] = {ss->hi, ss->trail, ss->side};
-    for (int i = 0; i < 3; ++i)
+    const cudaStream_t from[4] = {ss->hi, ss->near, ss->trail, ss->side};
+    for (int i = 0; i < 4; ++i)
       if (!record_wait(ss->join[i], from[i], s)) return check_launch("ntg_chol_factor_tc join");
     return NTG_OK;
   };
-  // Step b on the high-priority stream: diagonal block, L21 = A21 L11^-T, then (after the
-  // previous panel's trailing update, which also wrote it) the update of column block
-  // b + 1 only, so that block b + 1 can be factored at once; the trailing update of the
-  // columns beyond (rows and columns >= k + 2 PB) runs on the trailing stream meanwhile.
+  auto wait = [](cudaStream_t to, cudaEvent_t e) {
+    return cudaStreamWaitEvent(to, e, 0) == cudaSuccess;
+  };
+  // Step b. hi: diagonal block b, then the tile of L21 and the update (next_tile_kernel) that
+  // block b + 1 waits for. near: the rows of the panel and of column block b + 1 below these.
+  // trail: the columns beyond (rows and columns >= k + 2 PB). Column block b + 1 and block
+  // (b + 1, b + 1) come after the trailing update of panel b - 1, which also wrote them.
   const int64_t nblk = (n + PB - 1) / PB;
   for (int64_t b = 0; b < nblk; ++b) {
     const int64_t k = b * PB;
-    diag_block_kernel<<<1, 512, kDiagSmem, ss->hi>>>(L, ldl, n, k, info, f.linv + b * PB * PB);
-    note_launch();
-    const int64_t rest = n - k - PB;
-    float* l21 = L + (k + PB) * ldl + k;
+    float* const linv = f.linv + b * PB * PB;
+    const int64_t rest = n - k - PB, nb1 = mini(PB, rest), far = rest - nb1;
+    float* const l21 = L + (k + PB) * ldl + k;  // rows of the next block
+    float* const l31 = l21 + PB * ldl;          // rows beyond
+    bool ok = true;
+    launch_next_smem(ss->hi, diag_block_kernel, dim3(1), 512, kDiagSmem, L, ldl, n, k, info, linv);
     if (rest > 0) {
+      ok = record_wait(ss->diag, ss->hi, ss->near);
+      if (b > 0) ok = ok && wait(ss->hi, ss->column) && wait(ss->hi, ss->trail_done);
+      launch_next(ss->hi, next_tile_kernel<false>, dim3(PB / 16), 256, L, ldl, n, k, linv);
+      launch_next(ss->hi, next_tile_kernel<true>, dim3(PB / 16), 256, L, ldl, n, k, linv);
+    }
+    ok = ok && record_wait(ss->next, ss->hi, ss->side);
+    if (!ok) return join(), check_launch("ntg_chol_factor_tc events");
+    if (far > 0) {
       // in place (n = 128 columns: each tile row is read before it is written)
-      rc = gemm_tf32x3(ss->hi, l21, ldl, f.linv + b * PB * PB, PB, l21, ldl, rest, PB, PB, 1.f,
-                       0.f, 0);
+      rc = gemm_tf32x3(ss->near, l31, ldl, linv, PB, l31, ldl, far, PB, PB, 1.f, 0.f, 0);
       if (rc) return join(), rc;
-    }
-    if (!record_wait(ss->panel, ss->hi, ss->side) ||
-        cudaStreamWaitEvent(ss->trail, ss->panel, 0) != cudaSuccess)
-      return join(), check_launch("ntg_chol_factor_tc panel event");
-    {
-      const int64_t r0 = k, nb = mini(PB, n - r0), rows = r0 + nb;
-      rc = gemm_tf32x3(ss->side, f.uinv + r0, ldl, f.linv + b * PB * PB, PB, f.uinv + r0, ldl,
-                       rows, nb, nb, 1.f, 0.f, 0);
+      ok = record_wait(ss->panel, ss->near, ss->side) && wait(ss->trail, ss->panel) &&
+           wait(ss->near, ss->next) && (b == 0 || wait(ss->near, ss->trail_done));
+      if (!ok) return join(), check_launch("ntg_chol_factor_tc events");
+      rc = gemm_tf32x3(ss->near, l31, ldl, l21, ldl, L + (k + 2 * PB) * ldl + k + PB, ldl, far,
+                       nb1, PB, -1.f, 1.f, 0);
       if (rc) return join(), rc;
-      if (n - rows > 0) {
-        rc = gemm_tf32x3(ss->side, f.uinv + r0, ldl, L + rows * ldl + r0, ldl, f.uinv + rows,
-                         ldl, rows, n - rows, nb, -1.f, 1.f, 0);
-        if (rc) return join(), rc;
-      }
+      rc = gemm_tf32x3(ss->trail, l31, ldl, l31, ldl, L + (k + 2 * PB) * ldl + k + 2 * PB, ldl, far,
+                       far, PB, -1.f, 1.f, 1);
+      if (rc) return join(), rc;
+      if (cudaEventRecord(ss->column, ss->near) != cudaSuccess ||
+          cudaEventRecord(ss->trail_done, ss->trail) != cudaSuccess)
+        return join(), check_launch("ntg_chol_factor_tc events");
     }
-    if (rest > 0) {
-      const int64_t nb1 = mini(PB, rest), far = rest - nb1;
-      if (far > 0) {
-        float* l31 = l21 + nb1 * ldl;
-        rc = gemm_tf32x3(ss->trail, l31, ldl, l31, ldl, L + (k + PB + nb1) * ldl + k + PB + nb1,
-                         ldl, far, far, PB, -1.f, 1.f, 1);
-        if (rc) return join(), rc;
-      }
-      // column block b + 1 after the trailing update of panel b - 1 (recorded last step)
-      if (b > 0 && cudaStreamWaitEvent(ss->hi, ss->trail_done, 0) != cudaSuccess)
-        return join(), check_launch("ntg_chol_factor_tc trail event");
-      if (cudaEventRecord(ss->trail_done, ss->trail) != cudaSuccess)
-        return join(), check_launch("ntg_chol_factor_tc trail event");
-      rc = gemm_tf32x3(ss->hi, l21, ldl, l21, ldl, L + (k + PB) * ldl + k + PB, ldl, rest, nb1,
-                       PB, -1.f, 1.f, 0);
+    const int64_t nb = mini(PB, n - k), rows = k + nb;
+    rc = gemm_tf32x3(ss->side, f.uinv + k, ldl, linv, PB, f.uinv + k, ldl, rows, nb, nb, 1.f, 0.f,
+                     0);
+    if (rc) return join(), rc;
+    if (n - rows > 0) {
+      rc = gemm_tf32x3(ss->side, f.uinv + k, ldl, L + rows * ldl + k, ldl, f.uinv + rows, ldl, rows,
+                       n - rows, nb, -1.f, 1.f, 0);
       if (rc) return join(), rc;
     }
   }

@@ -231,3 +231,17 @@ def test_few_right_hand_sides_by_rows_and_columns(nt, n, m):
     # of the returned FP64 solution: below that of its float32 rounding, 2^-24 |A| |x|
     assert float(solver.residual) <= np.max(np.abs(r)) + 2. ** -24 * np.max(
         np.abs(a).astype(np.float64) @ np.abs(x))
+
+
+@pytest.mark.parametrize('n', [128, 129, 143, 255, 256, 257, 385, 512, 900])
+def test_factor_around_the_next_block(nt, n):
+    """One to eight panels with remainders of 1 to 128 rows: the factor itself, |L L^T - A|
+    within n products of 3xTF32 (2^-21) of the largest entry."""
+    from nt_gb300 import predict
+    rng = np.random.default_rng(n)
+    q = rng.standard_normal((n, n))
+    a = (np.eye(n) + q @ q.T / n).astype(np.float32)
+    solver = predict.CholeskySolver(_t(a), 0., True)
+    assert solver.info == 0
+    l = np.tril(solver.L.cpu().numpy().astype(np.float64))
+    assert np.max(np.abs(l @ l.T - a)) < n ** .5 * 2. ** -21 * np.max(np.abs(a))
