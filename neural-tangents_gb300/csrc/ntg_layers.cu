@@ -3,6 +3,7 @@
 // rule and the ABRelu/Erf epilogue fused in), elementwise Dense/activation,
 // pooling and the Flatten / GlobalAvgPool readouts.
 #include <cstdio>
+#include <climits>
 #include <string>
 
 #include "ntg_common.cuh"
@@ -69,28 +70,40 @@ __global__ void __launch_bounds__(256) gemm_nn_kernel(const float* __restrict__ 
 
 // ---------------------------------------------------------------------------
 // Full-spatial input covariance: out[b, a, a', c, c'] = sum_k x1[a,c,k] x2[a',c',k] / K
-// One CTA per (b, a) row; loops over a'.
+// One CTA per (b, a) row. A thread keeps its (c, c') for all planes a', so that an entry costs
+// its products, one store and no index arithmetic: bound by the stores (456 pairs of 28 x 28
+// images and the 43 samples with themselves, 1.2 GB: 383 us; 1490 with the indices taken apart
+// by 64-bit divisions for every entry).
 // ---------------------------------------------------------------------------
-__global__ void input_fs_kernel(const float* __restrict__ x1, const float* __restrict__ x2,
-                                int64_t batch, int64_t n2, int64_t A, int64_t C, int64_t K,
-                                float inv_k, float* __restrict__ out) {
-  int64_t blk = blockIdx.x;
-  int64_t b = blk / A, a = blk - b * A;
+__global__ void __launch_bounds__(256)
+    input_fs_kernel(const float* __restrict__ x1, const float* __restrict__ x2, int64_t batch,
+                    int64_t n2, int64_t A, int C, int64_t K, float inv_k,
+                    float* __restrict__ out) {
+  const int64_t b = blockIdx.x / A, a = blockIdx.x - b * A;
   if (b >= batch) return;
   int64_t i1, i2;
   pair_of(b, n2, i1, i2);
-  const float* r1 = x1 + ((i1 * A + a) * C) * K;
+  const float* r1 = x1 + (i1 * A + a) * C * K;
   const float* img2 = x2 + i2 * A * C * K;
-  float* o = out + ((b * A + a) * A) * C * C;
-  int64_t plane = C * C;
-  for (int64_t idx = threadIdx.x; idx < A * plane; idx += blockDim.x) {
-    int64_t ap = idx / plane, rem = idx - ap * plane;
-    int64_t c = rem / C, cp = rem - c * C;
+  const int64_t plane = (int64_t)C * C;
+  float* o = out + (b * A + a) * A * plane;
+  for (int64_t e = threadIdx.x; e < plane; e += 256) {
+    const int64_t c = plane <= INT_MAX ? (int)e / C : e / C;
     const float* p1 = r1 + c * K;
-    const float* p2 = img2 + (ap * C + cp) * K;
-    float s = 0.f;
-    for (int64_t k = 0; k < K; ++k) s = fmaf(__ldg(p1 + k), __ldg(p2 + k), s);
-    o[idx] = s * inv_k;
+    const float* p2 = img2 + (e - c * C) * K;
+    float x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = k < K ? __ldg(p1 + k) : 0.f;
+#pragma unroll 4
+    for (int64_t ap = 0; ap < A; ++ap) {
+      const float* y = p2 + ap * C * K;
+      float s = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < K) s = fmaf(x[k], __ldg(y + k), s);
+      for (int64_t k = 4; k < K; ++k) s = fmaf(__ldg(p1 + k), __ldg(y + k), s);
+      o[ap * plane + e] = s * inv_k;
+    }
   }
 }
 
@@ -201,6 +214,119 @@ __global__ void conv_fs_general_kernel(const float* __restrict__ in_q,
     }
     out_q[idx] = q;
     if (out_t) out_t[idx] = t;
+  }
+}
+
+// The same rule plane by plane, for any geometry whose planes fit: G consecutive output planes
+// (b, i, i') per CTA (1, or as many as 256 entries hold), first the sums over the A offsets into
+// shared memory (coalesced reads of whole input planes), then those over the C offsets, the
+// affine rule and the activation. fh + fw reads an entry instead of fh fw, and indices of one
+// plane in 32 bits. Bound by the two barriers a plane and, in the activation, by issue: a
+// network of two 5 x 5 layers on 28 x 28 maps, a pooling and a 5 x 5 layer on 14 x 14 maps takes
+// 6.7 ms for 456 pairs (53.5 entry by entry), one of 3 x 3 layers on 13 x 13 maps 1.26 ms for
+// 1600 (3.89). 3 x 3 windows on maps whose rows are whole 16-byte words go by lines instead (below):
+// 4.7 ps an entry and layer at 28 x 28, 13 here at 13 x 13.
+// F: the window where it is F x F with zero padding (unrolled, its loads in flight together).
+struct PlaneAt {
+  int64_t in, i1, i2;  // entry 0 of the first plane that the window sees; samples
+  int i, ip, lo, hi;   // output position; offsets [lo, hi) of the window on the map
+};
+
+template <int F>
+__global__ void __launch_bounds__(kThreads)
+    conv_fs_plane_kernel(const float* __restrict__ in_q, const float* __restrict__ in_t,
+                         float* __restrict__ out_q, float* __restrict__ out_t, ConvGeom g, int G,
+                         ntg_affine_t aff, ntg_act_t act, ntg_var_t var1, ntg_var_t var2) {
+  extern __shared__ __align__(16) float2 sums[];  // [G][C][C]
+  const int A = (int)g.A, C = (int)g.C, Ao = (int)g.Ao, Co = (int)g.Co;
+  const int P = C * C, Po = Co * Co;
+  PlaneAt* at = reinterpret_cast<PlaneAt*>(sums + G * P);  // [G]
+  const int64_t planes = g.batch * Ao * Ao, diag = (int64_t)(A + 1) * P;
+  const float inv = 1.f / (float)(g.fh * g.fw);
+  const ActC ac = act_consts(act);
+  // x / Co for x < Co^2, Co <= 1024
+  const uint32_t magic = Co > 1 ? 0xffffffffu / (uint32_t)Co + 1u : 0u;
+  const bool circular = F == 0 && g.circular;
+  for (int64_t p0 = (int64_t)blockIdx.x * G; p0 < planes; p0 += (int64_t)gridDim.x * G) {
+    const int n = (int)(planes - p0 < G ? planes - p0 : G);
+    for (int u = threadIdx.x; u < n; u += kThreads) {
+      const int64_t b = (p0 + u) / (Ao * Ao);
+      const int r = (int)(p0 + u - b * (Ao * Ao));
+      PlaneAt v;
+      pair_of(b, g.n2, v.i1, v.i2);
+      v.i = r / Ao;
+      v.ip = r - v.i * Ao;
+      const int ia = v.i * g.sh - g.ph, iap = v.ip * g.sh - g.ph;
+      const int mn = ia < iap ? ia : iap, mx = ia < iap ? iap : ia;
+      v.lo = circular || mn > 0 ? 0 : -mn;
+      v.hi = circular || g.fh < A - mx ? g.fh : A - mx;
+      v.in = b * A * A * P + (circular ? 0 : ((int64_t)ia * A + iap) * P);
+      at[u] = v;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < n * P; e += kThreads) {
+      const int u = G == 1 ? 0 : e / P;
+      const int64_t off = at[u].in + e - u * P;
+      const int lo = at[u].lo, hi = at[u].hi;
+      float sq = 0.f, st = 0.f;
+      if (circular) {
+        for (int d = 0; d < g.fh; ++d) {
+          int64_t ia = (int64_t)at[u].i * g.sh + d - g.ph, iap = (int64_t)at[u].ip * g.sh + d - g.ph;
+          wrap_index(ia, A, 1);
+          wrap_index(iap, A, 1);
+          const int64_t o = off + (ia * A + iap) * P;
+          sq += __ldg(in_q + o);
+          if (in_t) st += __ldg(in_t + o);
+        }
+      } else if (F) {
+        float q[F ? F : 1], t[F ? F : 1];
+#pragma unroll
+        for (int d = 0; d < F; ++d) {
+          const bool in = d >= lo && d < hi;
+          q[d] = in ? __ldg(in_q + off + d * diag) : 0.f;
+          t[d] = in && in_t ? __ldg(in_t + off + d * diag) : 0.f;
+        }
+#pragma unroll
+        for (int d = 0; d < F; ++d) sq += q[d], st += t[d];
+      } else {
+        for (int d = lo; d < hi; ++d) {
+          sq += __ldg(in_q + off + d * diag);
+          if (in_t) st += __ldg(in_t + off + d * diag);
+        }
+      }
+      sums[e] = make_float2(sq, st);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < n * Po; e += kThreads) {
+      const int u = G == 1 ? 0 : e / Po;
+      const int r = e - u * Po, j = Co > 1 ? (int)__umulhi((uint32_t)r, magic) : r, jp = r - j * Co;
+      const int jc = j * g.sw - g.pw, jcp = jp * g.sw - g.pw;
+      const float2* T = sums + u * P;
+      P2 s = p2s(0.f);
+      if (circular) {
+        for (int w = 0; w < g.fw; ++w) {
+          int64_t c1 = jc + w, c2 = jcp + w;
+          wrap_index(c1, C, 1);
+          wrap_index(c2, C, 1);
+          s = add2(s, p2ld(reinterpret_cast<const float*>(T + (int)c1 * C + (int)c2)));
+        }
+      } else {
+        const int mn = jc < jcp ? jc : jcp, mx = jc < jcp ? jcp : jc;
+        const int fw = F ? F : g.fw;
+#pragma unroll
+        for (int w = 0; w < fw; ++w)
+          if (mn + w >= 0 && mx + w < C)
+            s = add2(s, p2ld(reinterpret_cast<const float*>(T + jc * C + jcp + w * (C + 1))));
+      }
+      float sq, st, q, t = 0.f;
+      p2u(s, sq, st);
+      apply_affine(aff, sq, st, out_t != nullptr, q, t, inv);
+      if (act.kind != NTG_ACT_NONE)
+        act_apply(ac, q, t, var_at(var1, at[u].i1, at[u].i, j), var_at(var2, at[u].i2, at[u].ip, jp));
+      out_q[p0 * Po + e] = q;
+      if (out_t) out_t[p0 * Po + e] = t;
+    }
+    __syncthreads();
   }
 }
 
@@ -1334,19 +1460,22 @@ __global__ void conv_ds_kernel(const float* __restrict__ in_q, const float* __re
 }
 
 // ---------------------------------------------------------------------------
-// Elementwise affine + activation on [B, M].
+// Elementwise affine + activation on [B, M]. I: 32-bit entries where they fit, as taking an
+// index apart by 64-bit divisions costs more than the rule (4096 x 4096 entries: 43 us
+// instead of 55).
 // ---------------------------------------------------------------------------
+template <typename I>
 __global__ void affine_act_kernel(const float* __restrict__ in_q, const float* __restrict__ in_t,
                                   float* __restrict__ out_q, float* __restrict__ out_t,
-                                  int64_t batch, int64_t n2, int64_t A, int64_t C, int diag,
+                                  I batch, I n2, I A, I C, int diag,
                                   int has_affine, ntg_affine_t aff, ntg_act_t act,
                                   ntg_var_t var1, ntg_var_t var2) {
-  const int64_t M = diag ? A * C : A * A * C * C;
-  const int64_t total = batch * M;
+  const I M = diag ? A * C : A * A * C * C;
+  const I total = batch * M;
   const ActC ac = act_consts(act);
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int64_t b = idx / M, m = idx - b * M;
+  for (I idx = (I)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (I)gridDim.x * blockDim.x) {
+    const I b = idx / M, m = idx - b * M;
     float q = in_q[idx];
     float t = in_t ? in_t[idx] : 0.f;
     if (has_affine) {
@@ -1356,19 +1485,18 @@ __global__ void affine_act_kernel(const float* __restrict__ in_q, const float* _
       t = t2;
     }
     if (act.kind != NTG_ACT_NONE) {
-      int64_t a1, a2, c1, c2;
+      I a1, a2, c1, c2;
       if (diag) {
         a1 = a2 = m / C;
         c1 = c2 = m - a1 * C;
       } else {
-        int64_t r = m;
+        I r = m;
         c2 = r % C; r /= C;
         c1 = r % C; r /= C;
         a2 = r % A;
         a1 = r / A;
       }
-      int64_t i1, i2;
-      pair_of(b, n2, i1, i2);
+      const I i1 = n2 > 0 ? b / n2 : b, i2 = n2 > 0 ? b - i1 * n2 : b;
       act_apply(ac, q, t, var_at(var1, i1, a1, c1), var_at(var2, i2, a2, c2));
     }
     out_q[idx] = q;
@@ -1652,7 +1780,7 @@ extern "C" int ntg_input_fs(void* stream, const float* x1, const float* x2, int6
   NTG_REQUIRE(!pairs || (x2 && n2 > 0), "ntg_input_fs: pairs mode needs x2 and n2 > 0");
   const float* xb = pairs ? x2 : x1;
   int64_t blocks = batch * a;
-  NTG_REQUIRE(blocks < (1ll << 31), "ntg_input_fs: grid too large");
+  NTG_REQUIRE(blocks < (1ll << 31) && c <= INT_MAX, "ntg_input_fs: grid too large");
   const size_t vec_sm = sizeof(float) * 4 * (c + a * c);
   if (c >= 4 && c <= 32 && (c & (c - 1)) == 0 && k <= 4 && vec_sm <= 48 * 1024 &&
       (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
@@ -1660,7 +1788,7 @@ extern "C" int ntg_input_fs(void* stream, const float* x1, const float* x2, int6
         x1, xb, batch, pairs ? n2 : 0, (int)a, (int)c, (int)k, 1.f / (float)k, out);
   } else {
     input_fs_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
-        x1, xb, batch, pairs ? n2 : 0, a, c, k, 1.f / (float)k, out);
+        x1, xb, batch, pairs ? n2 : 0, a, (int)c, k, 1.f / (float)k, out);
   }
   note_launch();
   return check_launch("ntg_input_fs");
@@ -1828,6 +1956,24 @@ extern "C" int ntg_conv_fs(void* stream, const float* in_q, const float* in_t, f
   } else {
     ConvGeom g{batch, n2, a, c, ao, co, fh, fw, sh, sw, ph, pw, pad_mode == NTG_PAD_CIRCULAR};
     int64_t total = batch * ao * ao * co * co;
+    // planes of up to 110 x 110 entries (two CTAs per SM) by the plane, larger ones by the entry
+    const int64_t G = c * c >= 256 ? 1 : 256 / (c * c);
+    const size_t sm = (size_t)G * (c * c * sizeof(float2) + sizeof(PlaneAt));
+    if (c <= 110 && a <= 32768 && ao <= 32768 && co <= 1024) {
+      const int f = fh == fw && pad_mode == NTG_PAD_ZERO ? fh : 0;
+      auto kernel = f == 3   ? conv_fs_plane_kernel<3>
+                    : f == 5 ? conv_fs_plane_kernel<5>
+                             : conv_fs_plane_kernel<0>;
+      const cudaError_t e = cudaFuncSetAttribute(
+          kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if (e != cudaSuccess)
+        return fail(NTG_ERR_CUDA, std::string("ntg_conv_fs: ") + cudaGetErrorString(e));
+      const int64_t blocks = ceil_div(batch * ao * ao, G);
+      kernel<<<(unsigned)(blocks < 152 * 64 ? blocks : 152 * 64), kThreads, sm, s>>>(
+          in_q, in_t, out_q, out_t, g, (int)G, aff, act, var1, var2);
+      note_launch();
+      return check_launch("ntg_conv_fs");
+    }
     conv_fs_general_kernel<<<grid_for(total), kThreads, 0, s>>>(in_q, in_t, out_q, out_t, g, aff,
                                                                  act, var1, var2);
   }
@@ -2060,9 +2206,15 @@ extern "C" int ntg_affine_act(void* stream, const float* in_q, const float* in_t
       affine_act_fs_kernel<0><<<grid, kThreads, 0, as_stream(stream)>>>(
         in_q, in_t, out_q, out_t, batch, n2, (int)a, (int)c, has_affine, aff, act, var1, var2);
   } else {
-    affine_act_kernel<<<grid_for(batch * m), kThreads, 0, as_stream(stream)>>>(
-        in_q, in_t, out_q, out_t, batch, n2, a, c, diag_spatial, has_affine, aff, act, var1,
-        var2);
+    const int grid = grid_for(batch * m);
+    if (batch * m < (1ll << 31) && n2 >= 0 && n2 < (1ll << 31))
+      affine_act_kernel<uint32_t><<<grid, kThreads, 0, as_stream(stream)>>>(
+          in_q, in_t, out_q, out_t, (uint32_t)batch, (uint32_t)n2, (uint32_t)a, (uint32_t)c,
+          diag_spatial, has_affine, aff, act, var1, var2);
+    else
+      affine_act_kernel<int64_t><<<grid, kThreads, 0, as_stream(stream)>>>(
+          in_q, in_t, out_q, out_t, batch, n2, a, c, diag_spatial, has_affine, aff, act, var1,
+          var2);
   }
   note_launch();
   return check_launch("ntg_affine_act");

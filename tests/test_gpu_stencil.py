@@ -8,6 +8,7 @@ only changes the launch, so results for different depths are bit-identical.
 """
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -182,3 +183,67 @@ def test_pool_transpose_block_matches_general(nt):
 
     fast, slow = run(0), run(1)
     assert torch.equal(fast, slow)
+
+
+@pytest.mark.parametrize('a,c,filt,strides,pad,circular', [
+    (14, 14, (3, 3), (1, 1), (1, 1), False), (7, 7, (5, 5), (1, 1), (2, 2), False),
+    (9, 5, (3, 2), (1, 1), (1, 0), False), (6, 17, (3, 3), (2, 3), (1, 1), False),
+    (5, 6, (3, 5), (1, 1), (1, 2), True), (8, 1, (3, 1), (1, 1), (1, 0), False),
+    (4, 1, (1, 1), (1, 1), (0, 0), False), (3, 110, (3, 3), (1, 1), (1, 1), False),
+    (2, 111, (3, 3), (1, 1), (1, 1), False), (28, 28, (5, 5), (1, 1), (0, 0), False)])
+@pytest.mark.parametrize('has_t', [True, False])
+def test_conv_planes_match_float64(nt, a, c, filt, strides, pad, circular, has_t):
+    """The conv rule by planes (up to 110 x 110 entries, groups of small ones) and by entries
+    against sums in float64: (fh + fw) roundings of at most 2^-24 of the sum of magnitudes each,
+    and those of the affine rule (4)."""
+    from nt_gb300 import _ops as O
+    (fh, fw), (sh, sw), (ph, pw) = filt, strides, pad
+    B = 3 if a * c < 400 else 1
+    ao, co = [(n if circular else (n + 2 * p - f) // s + 1)
+              for n, f, s, p in ((a, fh, sh, ph), (c, fw, sw, pw))]
+    g = torch.Generator(device='cuda').manual_seed(a * 100 + c)
+    q, t = (torch.randn((B, a, a, c, c), generator=g, device='cuda') for _ in range(2))
+    w2, b2 = 1.7, 0.3
+    aff = O.affine(w2, b2, w2)
+    outs = O.conv_fs(q, t if has_t else None, B, 1, a, c, fh, fw, sh, sw, ph, pw, ao, co, circular,
+                     aff, O.NO_ACT, O.NO_VAR, O.NO_VAR, True, (B,))
+
+    def window(x):
+        x = x.double()
+        for dim, (f, s, p, n, o) in ((1, (fh, sh, ph, a, ao)), (3, (fw, sw, pw, c, co))):
+            total = 0.
+            for d in range(f):
+                at = torch.arange(o, device='cuda') * s + d - p
+                ok = torch.ones(o, device='cuda', dtype=torch.bool) if circular else \
+                    (at >= 0) & (at < n)
+                part = x.index_select(dim, at % n).index_select(dim + 1, at % n)
+                m = (ok[:, None] & ok[None, :]).double()
+                total = total + part * m.reshape(m.shape + (1,) * (x.ndim - dim - 2))
+            x = total
+        return x / (fh * fw)
+
+    wq = w2 * window(q) + b2
+    wt = w2 * (window(t) if has_t else 0.) + wq
+    size = w2 * (window(q.abs()) + window(t.abs())) + b2
+    for got, want in zip(outs, (wq, wt)):
+        err = (got.double() - want).abs() / size
+        assert float(err.max()) < (fh + fw + 4) * 2. ** -24
+
+
+@pytest.mark.parametrize('shape', [(14, 14, 1), (9, 7, 3), (28, 28, 1), (5, 12, 6)])
+@pytest.mark.parametrize('filt', [3, 5])
+def test_full_spatial_networks_of_any_size(nt, shape, filt):
+    """Pooled conv networks with a mean over the positions, layer by layer, against the oracle
+    (1e-5 of the largest entry, the bound of the other network tests)."""
+    from oracle import nt_oracle as o
+    net = lambda m: [m.Conv(1, (filt, filt), padding='SAME', W_std=1.4, b_std=.1), m.Relu(),
+                     m.Conv(1, (filt, filt), padding='SAME', W_std=1.3), m.Erf(),
+                     m.AvgPool((2, 2), (2, 2)), m.Conv(1, (3, 3), padding='SAME', W_std=1.2),
+                     m.Relu(), m.GlobalAvgPool(), m.Dense(1, 1.1, .1)]
+    rng = np.random.default_rng(shape[0])
+    x1, x2 = (rng.standard_normal((n,) + shape).astype(np.float32) for n in (2, 3))
+    x2[1] = x1[0]
+    kf, ko = nt.stax.serial(*net(nt.stax))[2], o.serial(*net(o))
+    for b in (x2, None):
+        for got, want in zip(kf(x1, b, ('nngp', 'ntk')), ko(x1, b, ('nngp', 'ntk'))):
+            assert np.max(np.abs(got.cpu().numpy() - want)) < 1e-5 * np.max(np.abs(want))
