@@ -110,20 +110,30 @@ __global__ void trace_tc_kernel(const float* __restrict__ A, int64_t n, double* 
 }
 
 // L[i, j] = A[i, j] (j < i), A[i, i] + lambda (j == i), 0 above the diagonal and in the
-// padding columns n <= j < ldl.
-__global__ void init_factor_ld_kernel(const float* __restrict__ A, int64_t n, int64_t ldl,
-                                      double reg, int absolute, const double* __restrict__ trace,
-                                      float* __restrict__ L, double* __restrict__ lambda) {
-  const double lam = absolute ? reg : reg * trace[0] / (double)n;
-  if (blockIdx.x == 0 && threadIdx.x == 0) lambda[0] = lam;
-  const int64_t total = n * ldl;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = idx / ldl, j = idx - i * ldl;
-    float v = 0.f;
-    if (j < i) v = A[i * n + j];
-    else if (j == i) v = (float)((double)A[i * n + i] + lam);
-    L[idx] = v;
+// padding columns n <= j < ldl; Z = I, padded alike. A row per blockIdx.y: bound by the two arrays that it writes (n 5000: 41 us; two kernels over entries
+// 96).
+__global__ void __launch_bounds__(256)
+    init_factor_ld_kernel(const float* __restrict__ A, int64_t n, int64_t ldl, double reg,
+                          int absolute, const double* __restrict__ trace, float* __restrict__ L,
+                          float* __restrict__ Z, double* __restrict__ lambda) {
+  // FP64 is slow here: a division by every thread takes longer than the kernel
+  auto lam = [&] { return absolute ? reg : reg * trace[0] / (double)n; };
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) lambda[0] = lam();
+  const int64_t i = blockIdx.y, j0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
+  const float* a = A + i * n;
+  float v[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int64_t j = j0 + 256 * u;
+    v[u] = j <= i ? __ldg(a + j) : 0.f;
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int64_t j = j0 + 256 * u;
+    if (j >= ldl) break;
+    L[i * ldl + j] = v[u];
+    Z[i * ldl + j] = j == i ? 1.f : 0.f;
+    if (j == i) L[i * ldl + j] = (float)((double)v[u] + lam());
   }
 }
 
@@ -486,30 +496,27 @@ __global__ void __launch_bounds__(512, 1)
 constexpr size_t kDiagSmem = (size_t)(PB * PBS + 32 * XP + PB * XP + 32 * XP + 4 * 32 * 33) *
                              sizeof(float);
 
-// out[j, i] = in[i, j] for an [rows, cols] block (row pitches ld_in, ld_out).
-__global__ void transpose_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ out,
-                                 int64_t ld_out, int64_t rows, int64_t cols) {
+// out[j, i] = in[i, j] for an [rows, cols] block (row pitches ld_in, ld_out); upper: in is zero
+// below its diagonal, and the tiles there are not read (n 5000: 36 us instead of 63).
+__global__ void __launch_bounds__(256)
+    transpose_kernel(const float* __restrict__ in, int64_t ld_in, float* __restrict__ out,
+                     int64_t ld_out, int64_t rows, int64_t cols, bool upper) {
   __shared__ float tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  for (int i = ty; i < 32; i += 8) {
+  const bool zero = upper && c0 + 31 < r0;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int i = ty + 8 * u;
     const int64_t r = r0 + i, c = c0 + tx;
-    tile[i][tx] = (r < rows && c < cols) ? in[r * ld_in + c] : 0.f;
+    tile[i][tx] = (r < rows && c < cols && !zero) ? in[r * ld_in + c] : 0.f;
   }
   __syncthreads();
-  for (int i = ty; i < 32; i += 8) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int i = ty + 8 * u;
     const int64_t c = c0 + i, r = r0 + tx;
     if (c < cols && r < rows) out[c * ld_out + r] = tile[tx][i];
-  }
-}
-
-// I [n, ld]: ones on the diagonal, zeros elsewhere (padding columns included).
-__global__ void identity_kernel(float* __restrict__ Z, int64_t n, int64_t ld) {
-  const int64_t total = n * ld;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = idx / ld, j = idx - i * ld;
-    Z[idx] = (i == j) ? 1.f : 0.f;
   }
 }
 
@@ -1309,7 +1316,7 @@ int inv_apply_many(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, fl
                    float* z, float* y) {
   {
     dim3 g((unsigned)ceil_div(m, 32), (unsigned)ceil_div(n, 32));
-    transpose_kernel<<<g, 256, 0, s>>>(X, m, z, ldl, n, m);
+    transpose_kernel<<<g, 256, 0, s>>>(X, m, z, ldl, n, m, false);
     note_launch();
   }
   // y[c, j] = sum_i z[c, i] L^-1[j, i]: NT with B = L^-1 (row-major)
@@ -1320,7 +1327,7 @@ int inv_apply_many(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, fl
   if (rc) return rc;
   {
     dim3 g((unsigned)ceil_div(n, 32), (unsigned)ceil_div(m, 32));
-    transpose_kernel<<<g, 256, 0, s>>>(z, ldl, X, m, m, n);
+    transpose_kernel<<<g, 256, 0, s>>>(z, ldl, X, m, m, n, false);
     note_launch();
   }
   return check_launch("ntg_chol_solve_tc apply");
@@ -1354,8 +1361,8 @@ extern "C" int ntg_chol_factor_tc(void* stream, const float* A, int64_t n, doubl
   if (cudaMemsetAsync(info, 0, sizeof(int), s) != cudaSuccess)
     return check_launch("ntg_chol_factor_tc memset");
   trace_tc_kernel<<<1, 1024, 0, s>>>(A, n, lambda + 1);
-  init_factor_ld_kernel<<<grid_for(n * ldl), 256, 0, s>>>(A, n, ldl, diag_reg, absolute,
-                                                          lambda + 1, L, lambda);
+  init_factor_ld_kernel<<<dim3((unsigned)ceil_div(ldl, 1024), (unsigned)n), 256, 0, s>>>(
+      A, n, ldl, diag_reg, absolute, lambda + 1, L, f.uinv, lambda);
   note_launch(2);
   SideStream* ss = nullptr;
   rc = side_stream(&ss);
@@ -1365,8 +1372,6 @@ extern "C" int ntg_chol_factor_tc(void* stream, const float* A, int64_t n, doubl
   // block b, Z[:, b] <- Z[:, b] Linv_b^T, then Z[:, >b] -= Z[:, b] L[>b, b]^T, where only
   // the rows [0, r0 + nb) of Z[:, b] are non-zero (Z is upper triangular). Step b reads
   // panel b and Linv_b only, which no later panel changes.
-  identity_kernel<<<grid_for(n * ldl), 256, 0, s>>>(f.uinv, n, ldl);
-  note_launch();
   auto record_wait = [](cudaEvent_t e, cudaStream_t from, cudaStream_t to) {
     return cudaEventRecord(e, from) == cudaSuccess && cudaStreamWaitEvent(to, e, 0) == cudaSuccess;
   };
@@ -1434,7 +1439,7 @@ extern "C" int ntg_chol_factor_tc(void* stream, const float* A, int64_t n, doubl
   rc = join();
   if (rc) return rc;
   dim3 g((unsigned)ceil_div(n, 32), (unsigned)ceil_div(n, 32));
-  transpose_kernel<<<g, 256, 0, s>>>(f.uinv, ldl, f.linvf, ldl, n, n);
+  transpose_kernel<<<g, 256, 0, s>>>(f.uinv, ldl, f.linvf, ldl, n, n, true);
   note_launch();
   return check_launch("ntg_chol_factor_tc");
 }
