@@ -1311,7 +1311,7 @@ int inv_apply_small(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, f
 // X = (L L^T)^-1 X for many right-hand sides on the tensor cores, through the transposed
 // right-hand sides z = X^T [m, ldl]: y = z L^-T (= (L^-1 X)^T), z = y L^-1 (= X'^T). Each
 // tile's sum runs over the triangle only (4096 right-hand sides, n 4096: 907 -> 470 us a
-// product).
+// product, 393 since the split has eight warps).
 int inv_apply_many(cudaStream_t s, const FactorWs& f, int64_t ldl, int64_t n, float* X, int64_t m,
                    float* z, float* y) {
   {

@@ -6,7 +6,7 @@
 //
 // One CTA per 128 x 128 tile of C. TMA brings 128 x 32 float32 tiles of A and B
 // (one 128-byte swizzled row per matrix row) into a 3-stage shared-memory ring;
-// four converter warps split each tile in place (hi) and into a second buffer
+// eight converter warps split each tile in place (hi) and into a second buffer
 // (lo) and hand the stage to the MMA thread, which issues 12 MMAs per stage and
 // frees it with tcgen05.commit; the converter warps then drain the accumulator
 // with tcgen05.ld into the idle ring, from which all warps write C row by row
@@ -15,6 +15,11 @@
 // symmetric rank-k update of a Cholesky factorisation). Every wait is bounded:
 // one that runs out raises the device error word, lets the copies and MMAs in
 // flight land (bounded), frees the tensor memory and returns.
+//
+// Bound by shared memory: a stage is written by TMA, read and written twice over by the
+// split and read three times by the MMAs, 224 KB for 768 clocks of products. Four splitting
+// warps left the split itself on the critical path: 4096 x 4096 triangular by 4096 470 us,
+// with eight 393, with sixteen 388; a rank-128 update of 741 tiles 81, 69 and 68 us.
 #include <mutex>
 #include <string>
 
@@ -62,7 +67,8 @@ constexpr int GSTAGES = 3;
 constexpr int GTILE = GM * GK * 4;             // 16 KB per operand tile
 constexpr int GSTAGE = 4 * GTILE;              // A (hi in place), A lo, B (hi in place), B lo
 constexpr int GSMEM = GSTAGES * GSTAGE + 1024 + 256;
-constexpr int GTHREADS = 192;                  // warp 0 TMA, warp 1 MMA, warps 2-5 split + epilogue
+constexpr int GSPLIT = 8;                      // splitting warps
+constexpr int GTHREADS = 64 + 32 * GSPLIT;     // warp 0 TMA, warp 1 MMA, the others split + epilogue
 constexpr uint32_t GTMEM_COLS = 128;
 constexpr uint64_t GWAIT = 1ull << 21;
 constexpr uint32_t GIDESC = tc::idesc(2, GM, GN);  // kind::tf32
@@ -90,11 +96,11 @@ __device__ __forceinline__ float tf32_rn(float x) {
 }
 
 // hi = tf32(x) in place, lo = tf32(x - hi) into lo_buf at the same offset, for the
-// 16-byte chunks tid, tid + 128, ... of one operand tile (same swizzled layout).
+// 16-byte chunks tid, tid + 32 GSPLIT, ... of one operand tile (same swizzled layout).
 __device__ __forceinline__ void split_tile(uint8_t* tile, uint8_t* lo_buf, int tid) {
 #pragma unroll
-  for (int i = 0; i < GTILE / 16 / 128; ++i) {
-    const int off = (tid + 128 * i) * 16;
+  for (int i = 0; i < GTILE / 16 / (32 * GSPLIT); ++i) {
+    const int off = (tid + 32 * GSPLIT * i) * 16;
     float4 v = *reinterpret_cast<float4*>(tile + off);
     float4 h, l;
     h.x = tf32_rn(v.x); l.x = tf32_rn(v.x - h.x);
@@ -142,7 +148,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < GSTAGES; ++s) {
       tc::mbar_init(tc::smem_u32(&bars[s]), 1);
-      tc::mbar_init(tc::smem_u32(&bars[GSTAGES + s]), 4);
+      tc::mbar_init(tc::smem_u32(&bars[GSTAGES + s]), GSPLIT);
       tc::mbar_init(tc::smem_u32(&bars[2 * GSTAGES + s]), 1);
     }
     tc::mbar_init(tc::smem_u32(&bars[3 * GSTAGES]), 1);
@@ -210,7 +216,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
       }
     }
   } else {
-    // split warps (2..5): each stage's A and B tiles, then the epilogue
+    // split warps: each stage's A and B tiles, then the epilogue
     const int tid = threadIdx.x - 64;
     bool ok = true;
     for (int kc = 0; kc < nk; ++kc) {
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
   }
 
   // Epilogue through shared memory: the split warps move the accumulator from TMEM into
-  // the (now idle) stage buffers, then all six warps write C row by row, coalesced.
+  // the (now idle) stage buffers, then all warps write C row by row, coalesced.
   tc::fence_before();
   __syncthreads();
   const bool acc_ok = !s_fail;
@@ -248,7 +254,7 @@ __global__ void __launch_bounds__(GTHREADS, 1)
     tc::fence_after();
     const int q = warp & 3;
 #pragma unroll 1
-    for (int c0 = 0; c0 < GN; c0 += 32) {
+    for (int c0 = (warp - 2) / 4 * 32; c0 < GN; c0 += GSPLIT * 8) {
       uint32_t v[32];
       tc::tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
       float* dst = stile + (q * 32 + lane) * SP + c0;
