@@ -61,39 +61,6 @@ int grid_for(int64_t n) {
 // Set-up
 // ---------------------------------------------------------------------------
 
-// The kernels of a solve follow one another in a stream, most of them shorter than the gap
-// between two launches. Each lets the next one be set up while it runs and waits, before its
-// first access to memory, for the one before to have finished and its writes to be visible
-// (launch_next sets the launch attribute; without it both are no-ops). With the sums, splits
-// and checks of an iteration in the kernels next to them, 5000 points and ten right-hand sides
-// take 245 us an iteration (290 in twelve plain launches), an iteration after convergence,
-// eight kernels that return at once, 14 us (48).
-__device__ __forceinline__ void after_previous() {
-  asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... KA, typename... A>
-void launch_next_smem(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, size_t smem,
-                      A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.dynamicSmemBytes = smem;
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
-  note_launch();
-}
-template <typename... KA, typename... A>
-void launch_next(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, A... args) {
-  launch_next_smem(s, kernel, grid, threads, 0, args...);
-}
-
 __global__ void trace_tc_kernel(const float* __restrict__ A, int64_t n, double* __restrict__ out) {
   double s = 0.0;
   for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += (double)A[i * n + i];
@@ -1029,6 +996,11 @@ __device__ __forceinline__ void block_max(double* slot, double v) {
   atomicMax(reinterpret_cast<unsigned long long*>(slot),
             (unsigned long long)__double_as_longlong(fabs(v)));
 }
+
+// With the sums, splits and checks of an iteration in the kernels next to them and every launch
+// set up under the one before (launch_next), 5000 points and ten right-hand sides take 245 us
+// an iteration (290 in twelve plain launches), an iteration after convergence, eight kernels
+// that return at once, 14 us (48).
 
 // Set-up: p = z and its split; bnorm, r0norm, rho[0] = r.z (from part), every column active.
 // bpart, rpart: the blocks' maxima.

@@ -44,6 +44,38 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 constexpr float kPi = 3.14159265358979323846f;
 
 // ---------------------------------------------------------------------------
+// Chains of short kernels in one stream, most of them shorter than the gap between two
+// launches. Each lets the next one be set up while it runs and waits, before its first access
+// to memory, for the one before to have finished and its writes to be visible (launch_next
+// sets the launch attribute; without it both are no-ops).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KA, typename... A>
+void launch_next_smem(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, size_t smem,
+                      A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
+  note_launch();
+}
+template <typename... KA, typename... A>
+void launch_next(cudaStream_t s, void (*kernel)(KA...), dim3 grid, int threads, A... args) {
+  launch_next_smem(s, kernel, grid, threads, 0, args...);
+}
+
+// ---------------------------------------------------------------------------
 // Bulk-copy rings: shared-memory addresses and bounded mbarrier waits. A wait
 // that runs out returns false; the kernel then raises its device error word.
 // ---------------------------------------------------------------------------

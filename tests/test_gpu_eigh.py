@@ -61,3 +61,23 @@ def test_spectral_weights(nt, kind):
         w = [np.expm1(-e), np.expm1(-e) / np.abs(l64), pos * np.exp(-2 * e), np.exp(-e),
              -np.expm1(-2 * e) / np.abs(l64), -np.expm1(-e), -np.expm1(-e) / np.abs(l64)][kind]
         np.testing.assert_allclose(got[:, j, :], w * x, rtol=1e-6, atol=1e-30)
+
+
+@pytest.mark.parametrize('n', [65, 96, 128, 129, 320])
+def test_eigh_of_coupled_blocks(nt, n):
+    """Two to ten blocks of 32, where the couplings inside a block are rotated once a sweep: a
+    matrix whose couplings lie inside the blocks only, one whose couplings lie between them
+    only, and both; the bounds of test_eigh_matches_float64."""
+    from nt_gb300 import predict
+    rng = np.random.default_rng(n)
+    g = rng.standard_normal((n, n))
+    g = (g + g.T) / 2
+    inside = (np.arange(n)[:, None] // 32) == (np.arange(n)[None] // 32)
+    for mask in (inside, ~inside | np.eye(n, dtype=bool), np.ones((n, n))):
+        a = (g * mask).astype(np.float32)
+        evals, evecs = predict._eigh(torch.from_numpy(a).cuda(), 0.)
+        w, v = evals.double().cpu().numpy(), evecs.double().cpu().numpy()
+        scale = np.linalg.norm(a.astype(np.float64), 2)
+        assert np.max(np.abs(a @ v - v * w[None])) / scale < 2e-5
+        assert np.max(np.abs(v.T @ v - np.eye(n))) < 2e-5
+        assert np.max(np.abs(np.sort(w) - np.linalg.eigvalsh(a.astype(np.float64)))) < 1e-5 * scale
