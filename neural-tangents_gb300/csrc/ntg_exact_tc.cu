@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
 }
 
 // A's digits, 2.5 times its size, are made for a band of at most 512 MiB of rows at a time (one
-// tile at least; one band up to n = 7168) and X's for all columns: 12 bytes an entry where the
+// tile at least; one band up to n = 7296) and X's for all columns: 12 bytes an entry where the
 // double-float split takes 8.
 struct ExactWs {
   int64_t kpad, arows, xcols;  // arows: of a band

@@ -176,7 +176,7 @@ def test_exact_residual(nt, n, m):
 
 
 def test_exact_residual_in_bands(nt):
-    """A's digits are made 7168 rows at a time from there on: the largest residual once more,
+    """A's digits are made 7296 rows at a time from there on: the largest residual once more,
     under the same bound, at two bands and a remainder of columns."""
     from nt_gb300 import predict
     n, m = 7300, 70
