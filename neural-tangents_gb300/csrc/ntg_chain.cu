@@ -157,7 +157,7 @@ int launch_chain(const char* who, const ntg_chain_t* prog, ChainArgs a, void* wo
   else if (pg.nseg == 3 && n0 == 3 && c1 == 3 && c2 == 3)
     e = launch_chain_myrtle10(relu_only, pg, a);
   else
-    e = launch_chain_any(pg, a);
+    e = relu_only ? launch_chain_relu(pg, a) : launch_chain_any(pg, a);
   note_launch();
   if (e == cudaSuccess && a.parts.n > 1) {
     chain_reduce_kernel<<<(unsigned)ceil_div(g.total, 64), 64, 0, a.stream>>>(
@@ -203,8 +203,7 @@ extern "C" int ntg_chain_vars(void* stream, const ntg_chain_t* prog, const float
   rules_of(*prog, nl, relu_only, rare);
   const VarArgs a{as_stream(stream), x1, n1, var1, x2, n2, var2, static_cast<float*>(workspace)};
   const cudaError_t e = rare ? launch_var_rare(*prog, a)
-                        : relu_only && prog->channels == 3 ? launch_var_relu(*prog, a)
-                                                           : launch_var_any(*prog, a);
+                        : relu_only ? launch_var_relu(*prog, a) : launch_var_any(*prog, a);
   if (e != cudaSuccess) return fail(NTG_ERR_CUDA, w + ": " + cudaGetErrorString(e));
   note_launch();
   return check_launch("ntg_chain_vars");

@@ -95,6 +95,7 @@ struct VarArgs {
 cudaError_t launch_chain_myrtle5(bool relu_only, const ntg_chain_t& pg, const ChainArgs& a);
 cudaError_t launch_chain_myrtle7(bool relu_only, const ntg_chain_t& pg, const ChainArgs& a);
 cudaError_t launch_chain_myrtle10(bool relu_only, const ntg_chain_t& pg, const ChainArgs& a);
+cudaError_t launch_chain_relu(const ntg_chain_t& pg, const ChainArgs& a);
 cudaError_t launch_chain_any(const ntg_chain_t& pg, const ChainArgs& a);
 cudaError_t launch_chain_rare(const ntg_chain_t& pg, const ChainArgs& a);
 cudaError_t launch_var_relu(const ntg_chain_t& pg, const VarArgs& a);
@@ -143,9 +144,11 @@ __device__ __forceinline__ void put(float* p, const float (&v)[1]) { *p = v[0]; 
 // column left ([row][j] = [row][j + 1]), so that the sample-2 entries of a pair are one
 // aligned 8-byte load on odd rows too, and an address per sample serves every plane of it.
 // RO: what is compiled in: 1: an ABRelu in every layer, NTK parameterisation, 0: ABRelu, Erf
-// or no activation, 2: every rule (Sin / Rbf / Gelu as well). COMP: see abrelu2.
+// or no activation, 2: every rule (Sin / Rbf / Gelu as well). ROOTS: see abrelu2_v; always with
+// RO 0 and 2. COMP: see abrelu2.
 // KC > 0: channel count. NTK = false: the nngp only (the ntk's slots are left alone).
-template <int S, int NC, bool FIRST, bool LAST, int RO, int COMP, int KC, bool NTK = true>
+template <int S, int NC, bool FIRST, bool LAST, int RO, bool ROOTS, int COMP, int KC,
+          bool NTK = true>
 __device__ __forceinline__ void chain_line(ChainCtx& cx, const ntg_chain_t& pg, int lbase,
                                            const float* sec, const float* in_slots,
                                            float* out_slots, int delta) {
@@ -317,7 +320,7 @@ __device__ __forceinline__ void chain_line(ChainCtx& cx, const ntg_chain_t& pg, 
           if (RO == 1 || ac.kind != NTG_ACT_NONE) {
             const P2 v1 = p2ld(a1 + vo + 2 * u), v2 = p2ld(a2[u] + vo);
             if (RO == 1 || (ac.kind == NTG_ACT_ABRELU && ac.stab <= 0.f)) {
-              abrelu2_v<COMP>(ac, q, t, v1, v2);
+              abrelu2_v<COMP, ROOTS>(ac, q, t, v1, v2);
             } else {
               float qa, qb, ta, tb, va, vb, wa, wb;
               p2u(q, qa, qb);
@@ -381,10 +384,11 @@ __device__ __forceinline__ void chain_line(ChainCtx& cx, const ntg_chain_t& pg, 
   };
 
   // planes with every level inside the line, by threes (the period of the (A, B, new) plane
-  // ring, so that its rotation is a renaming of registers); the others one by one
+  // ring, so that its rotation is a renaming of registers); the others one by one, and all in the
+  // ROOTS lines beside RO 1's others, which few pairs take
   int s = lo;
   while (s < hi + NC) {
-    if (S == S0 && s >= lo + NC && s + 2 < hi) {
+    if (S == S0 && (RO != 1 || !ROOTS) && s >= lo + NC && s + 2 < hi) {
       step(s, std::true_type());
       step(s + 1, std::true_type());
       step(s + 2, std::true_type());
@@ -397,19 +401,23 @@ __device__ __forceinline__ void chain_line(ChainCtx& cx, const ntg_chain_t& pg, 
 }
 
 // NCT >= 0: the segment's conv count is known at compile time (one instantiation).
-template <int S, bool LAST, int NCT, int RO, int COMP, bool NTK = true>
+template <int S, bool LAST, int NCT, int RO, bool ROOTS, int COMP, bool NTK = true>
 __device__ __forceinline__ void pooled_line(ChainCtx& cx, const ntg_chain_t& pg, int ncv,
                                             int lbase, const float* sec, const float* in_slots,
                                             float* out_slots, int m) {
+  auto line = [&](auto nc) {
+    chain_line<S, decltype(nc)::value, false, LAST, RO, ROOTS, COMP, 0, NTK>(
+        cx, pg, lbase, sec, in_slots, out_slots, m);
+  };
   if constexpr (NCT >= 0) {
-    chain_line<S, NCT, false, LAST, RO, COMP, 0, NTK>(cx, pg, lbase, sec, in_slots, out_slots, m);
+    line(std::integral_constant<int, NCT>());
     return;
   }
   switch (ncv) {
-    case 0: chain_line<S, 0, false, LAST, RO, COMP, 0, NTK>(cx, pg, lbase, sec, in_slots, out_slots, m); break;
-    case 1: chain_line<S, 1, false, LAST, RO, COMP, 0, NTK>(cx, pg, lbase, sec, in_slots, out_slots, m); break;
-    case 2: chain_line<S, 2, false, LAST, RO, COMP, 0, NTK>(cx, pg, lbase, sec, in_slots, out_slots, m); break;
-    default: chain_line<S, 3, false, LAST, RO, COMP, 0, NTK>(cx, pg, lbase, sec, in_slots, out_slots, m); break;
+    case 0: line(std::integral_constant<int, 0>()); break;
+    case 1: line(std::integral_constant<int, 1>()); break;
+    case 2: line(std::integral_constant<int, 2>()); break;
+    default: line(std::integral_constant<int, 3>()); break;
   }
 }
 
@@ -428,10 +436,12 @@ __device__ __forceinline__ void tri_pair(int64_t p, int64_t n, int64_t& i, int64
 }
 
 // One sample pair's images (as channel planes) and variance maps into the sections that
-// chain_line reads, segment by segment; returns the first float after them.
+// chain_line reads, segment by segment; returns the first float after them. one_root: whether
+// the variances that this thread loaded are all one_root_var.
 __device__ __forceinline__ float* load_pair(ChainCtx& cx, const ntg_chain_t& pg, int nseg,
                                             const float* im1, const float* im2, const float* g1,
-                                            const float* g2, float* smem, float* (&sec)[3]) {
+                                            const float* g2, float* smem, float* (&sec)[3],
+                                            bool& one_root) {
   const int K = pg.channels;
   float* p = smem;
   int l = 0;
@@ -455,9 +465,11 @@ __device__ __forceinline__ float* load_pair(ChainCtx& cx, const ntg_chain_t& pg,
       const float* b = g2 + pg.var_off[l];
       for (int e = threadIdx.x; e < n; e += NT) {
         const int es = (e & ~(S - 1)) | ((e + 1) & (S - 1));
-        v[e] = __ldg(a + e);
-        v[D + e] = __ldg(b + e);
+        const float va = __ldg(a + e), vb = __ldg(b + e);
+        v[e] = va;
+        v[D + e] = vb;
         v[2 * D + e] = __ldg(b + es);
+        one_root = one_root && one_root_var(va) && one_root_var(vb);
       }
     }
     p += 3 * D;
@@ -476,7 +488,7 @@ __device__ __forceinline__ float* load_pair(ChainCtx& cx, const ntg_chain_t& pg,
 // the line after that, which overwrites the slots just read, starts behind a barrier.
 // NSEG > 0: segment count and conv counts N1, N2 fixed at compile time (the common
 // Myrtle shapes), so that only the code this network runs is in the kernel.
-template <int N0, int NSEG, int N1, int N2, int RO, int COMP, int KC>
+template <int N0, int NSEG, int N1, int N2, int RO, bool ROOTS, int COMP, int KC>
 __device__ __forceinline__ void chain_lines(ChainCtx& cx, const ntg_chain_t& pg, int nseg,
                                             float* const (&sec)[3], float* slots, int first,
                                             int last) {
@@ -493,26 +505,26 @@ __device__ __forceinline__ void chain_lines(ChainCtx& cx, const ntg_chain_t& pg,
   const int l0 = nseg > 1 ? min(2 * l1 + 1, S0 - 1) : last;
   for (int d0 = f0; d0 <= l0; ++d0) {
     if (nseg == 1) {
-      chain_line<S0, N0, true, true, RO, COMP, KC>(cx, pg, 0, sec[0], nullptr, nullptr, d0);
+      chain_line<S0, N0, true, true, RO, ROOTS, COMP, KC>(cx, pg, 0, sec[0], nullptr, nullptr, d0);
       continue;
     }
-    chain_line<S0, N0, true, false, RO, COMP, KC>(cx, pg, 0, sec[0], nullptr, slots, d0);
+    chain_line<S0, N0, true, false, RO, ROOTS, COMP, KC>(cx, pg, 0, sec[0], nullptr, slots, d0);
     __syncthreads();
     const int m1 = (d0 - 1) / 2;
     if (!(d0 & 1) || m1 < f1) continue;
     if (nseg == 2) {
-      pooled_line<S1, true, NSEG == 2 ? N1 : -1, RO, COMP>(cx, pg, nc1, N0, sec[1], slots, nullptr,
-                                                           m1);
+      pooled_line<S1, true, NSEG == 2 ? N1 : -1, RO, ROOTS, COMP>(cx, pg, nc1, N0, sec[1], slots,
+                                                                  nullptr, m1);
       continue;
     }
-    pooled_line<S1, false, NSEG == 3 ? N1 : -1, RO, COMP>(cx, pg, nc1, N0, sec[1], slots, slots2,
-                                                          m1);
+    pooled_line<S1, false, NSEG == 3 ? N1 : -1, RO, ROOTS, COMP>(cx, pg, nc1, N0, sec[1], slots,
+                                                                 slots2, m1);
     const int m2 = (m1 - 1) / 2;
     if (!(m1 & 1) || m2 < first) continue;
     if (threadIdx.x < 8 * S1) {  // the threads of segment 1: its three lines are in
       asm volatile("bar.sync 1, %0;" ::"n"(8 * S1) : "memory");
-      pooled_line<S2, true, NSEG == 3 ? N2 : -1, RO, COMP>(cx, pg, nc2, N0 + nc1, sec[2], slots2,
-                                                           nullptr, m2);
+      pooled_line<S2, true, NSEG == 3 ? N2 : -1, RO, ROOTS, COMP>(cx, pg, nc2, N0 + nc1, sec[2],
+                                                                  slots2, nullptr, m2);
     }
   }
 }
@@ -560,10 +572,20 @@ __device__ __forceinline__ void chain_pair(const ntg_chain_t& pg, const float* _
   const int64_t im = (int64_t)S0 * S0 * pg.channels;
   ChainCtx cx;
   float* sec[3] = {nullptr, nullptr, nullptr};
+  bool one_root = true;
   float* red = load_pair(cx, pg, nseg, x1 + gi * im, x2 + gj * im, var1 + gi * pg.var_stride,
-                         var2 + gj * pg.var_stride, smem, sec);  // 2 * NT / 32 floats
-  __syncthreads();
-  chain_lines<N0, NSEG, N1, N2, RO, COMP, KC>(cx, pg, nseg, sec, slots, first, last);
+                         var2 + gj * pg.var_stride, smem, sec, one_root);  // 2 * NT / 32 floats
+  one_root = __syncthreads_and(one_root);
+  auto lines = [&](auto two_roots) {
+    chain_lines<N0, NSEG, N1, N2, RO, decltype(two_roots)::value, COMP, KC>(cx, pg, nseg, sec,
+                                                                            slots, first, last);
+  };
+  if constexpr (RO == 1) {
+    if (one_root) lines(std::false_type());
+    else lines(std::true_type());
+  } else {
+    lines(std::true_type());
+  }
 
   // block reduction of the readout sums
   float aq = cx.acc_q, at = cx.acc_t;
@@ -626,10 +648,11 @@ __global__ void __launch_bounds__(NT, kChainCtasPerSm)
 // scratch. A self pair's diagonal only couples to itself under the conv rule, and the entries
 // are evaluated exactly as chain_line evaluates row 0 of line 0, so that the pair (i, i) has
 // var1 var2 - q^2 == 0 there. Each layer's pre-activation variances go to the segment's
-// sections and to `out`.
+// sections and to `out`; one_root: see load_pair.
 template <int RO>
 __device__ __forceinline__ void diag_layers(const ntg_chain_t& pg, int S, int nc, int lbase,
-                                            float* sec, int K, float* d, float* tmp, float* out) {
+                                            float* sec, int K, float* d, float* tmp, float* out,
+                                            bool& one_root) {
   const int n = S * S, D = (K + nc) * n;
   for (int k = 0; k < nc; ++k) {
     const ntg_affine_t& af = pg.aff[lbase + k];
@@ -646,6 +669,7 @@ __device__ __forceinline__ void diag_layers(const ntg_chain_t& pg, int S, int nc
       v[e] = v[D + e] = q;
       v[2 * D + (e & ~(S - 1)) + ((w + S - 1) & (S - 1))] = q;
       out[pg.var_off[lbase + k] + e] = q;
+      one_root = one_root && one_root_var(q);
       if (ac.kind != NTG_ACT_NONE) {
         float t = 0.f;
         const float vi = q, sv = sqrt_var(q);
@@ -701,7 +725,6 @@ __global__ void __launch_bounds__(NT, kChainCtasPerSm)
       d[e] = g * cx.inv_k;
     }
     __syncthreads();
-    diag_layers<RO>(pg, S0, N0, 0, sec[0], K, d, tmp, out);
     // the spatial diagonal of pooled line 0 of a segment of size S: row 0 and its side row
     auto pooled_diag = [&](const float* slot, int S) {
       const int plane = (S + S / 2) * S;
@@ -711,22 +734,39 @@ __global__ void __launch_bounds__(NT, kChainCtasPerSm)
       }
       __syncthreads();
     };
+    bool one_root = true;
+    diag_layers<RO>(pg, S0, N0, 0, sec[0], K, d, tmp, out, one_root);
     // lines -1 .. 1 of segment 0 for segment 1's maps, then -3 .. 3 with segment 1 as well
     // for segment 2's
-    for (int stage = 1; stage < nseg; ++stage) {
-      const int w = stage == 1 ? 1 : 3;
-      for (int d0 = -w; d0 <= w; ++d0) {
-        chain_line<S0, N0, true, false, RO, -1, KC, false>(cx, pg, 0, sec[0], nullptr, mine, d0);
-        __syncthreads();
-        if (stage == 2 && (d0 & 1) && d0 > -3)
-          pooled_line<S1, false, -1, RO, -1, false>(cx, pg, nc1, N0, sec[1], mine, mine + kSlots1,
-                                                    (d0 - 1) / 2);
+    auto segments = [&](auto two_roots) {
+      constexpr bool ROOTS = decltype(two_roots)::value;
+      for (int stage = 1; stage < nseg; ++stage) {
+        const int w = stage == 1 ? 1 : 3;
+        for (int d0 = -w; d0 <= w; ++d0) {
+          chain_line<S0, N0, true, false, RO, ROOTS, -1, KC, false>(cx, pg, 0, sec[0], nullptr,
+                                                                    mine, d0);
+          __syncthreads();
+          if (stage == 2 && (d0 & 1) && d0 > -3)
+            pooled_line<S1, false, -1, RO, ROOTS, -1, false>(cx, pg, nc1, N0, sec[1], mine,
+                                                             mine + kSlots1, (d0 - 1) / 2);
+        }
+        if (stage == 2) __syncthreads();
+        pooled_diag(stage == 1 ? mine : mine + kSlots1, S0 >> stage);
+        diag_layers<RO>(pg, S0 >> stage, stage == 1 ? nc1 : nc2, stage == 1 ? N0 : N0 + nc1,
+                        sec[stage], 0, d, tmp, out, one_root);
       }
-      if (stage == 2) __syncthreads();
-      pooled_diag(stage == 1 ? mine : mine + kSlots1, S0 >> stage);
-      diag_layers<RO>(pg, S0 >> stage, stage == 1 ? nc1 : nc2, stage == 1 ? N0 : N0 + nc1,
-                      sec[stage], 0, d, tmp, out);
+    };
+    // By the rule of a pair of this sample (chain_pair), which goes by all maps, or
+    // var1 var2 - q^2 would not be 0 in the pair: the pooled variances are sums over entries that
+    // the two forms round differently.
+    bool roots = RO != 1 || !__syncthreads_and(one_root);
+    if constexpr (RO == 1) {
+      if (!roots) {
+        segments(std::false_type());
+        roots = !__syncthreads_and(one_root);
+      }
     }
+    if (roots) segments(std::true_type());
   }
 }
 
@@ -759,7 +799,8 @@ cudaError_t launch_chain_k(const ntg_chain_t& pg, const ChainArgs& a) {
 // ReLU family also to their precision (all layers share the precision of one call).
 template <int N0, int N1, int N2>
 cudaError_t launch_myrtle(bool relu_only, const ntg_chain_t& pg, const ChainArgs& a) {
-  if (!relu_only || pg.channels != 3) return launch_chain_k<N0, 3, N1, N2, 0>(pg, a);
+  if (!relu_only) return launch_chain_k<N0, 3, N1, N2, 0>(pg, a);
+  if (pg.channels != 3) return launch_chain_relu(pg, a);
   bool comp = false;
   for (int l = 0; l < NTG_CHAIN_MAX_LAYERS; ++l) comp = comp || pg.act[l].compensated != 0;
   return comp ? launch_chain_k<N0, 3, N1, N2, 1, 1, 3>(pg, a)

@@ -16,7 +16,7 @@ cudaError_t by_convs(const ntg_chain_t& pg, const VarArgs& a) {
 }  // namespace
 
 cudaError_t launch_var_relu(const ntg_chain_t& pg, const VarArgs& a) {
-  return by_convs<1, 3>(pg, a);
+  return pg.channels == 3 ? by_convs<1, 3>(pg, a) : by_convs<1>(pg, a);
 }
 cudaError_t launch_var_any(const ntg_chain_t& pg, const VarArgs& a) { return by_convs<0>(pg, a); }
 cudaError_t launch_var_rare(const ntg_chain_t& pg, const VarArgs& a) { return by_convs<2>(pg, a); }

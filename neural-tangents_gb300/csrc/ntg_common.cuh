@@ -324,9 +324,11 @@ __device__ __forceinline__ void act_apply(const ActC& c, float& q, float& t, flo
 // The ABRelu branch of act_apply (do_stabilize off) on a packed pair, with
 // the same operation sequence per lane. COMP: -1 reads c.comp, 0 / 1 fix the
 // plain / compensated var1 var2 - q^2 at compile time. ROOTS: n = sqrt(v1) sqrt(v2) is given;
-// else it is sqrt(v1 v2 + 2^-126), which has no zero to look out for: where both variances
-// and q vanish the angle counts as 0 instead of pi / 2, which only ntk' = ntk dot would see,
-// so this form is for kernels whose ntk vanishes with the variances.
+// else it is sqrt(v1 v2 + 2^-126), one root instead of two and no zero to look out for, which is
+// right to rounding while v1 v2 is 2^-64 or more. It may be 0 as well where the ntk vanishes
+// with the variances: with q = 0 the angle then counts as 0 instead of pi / 2, which only
+// ntk' = ntk dot would see. (In the standard parameterization with a bias of 0 the ntk is 1
+// there.)
 template <int COMP, bool ROOTS>
 __device__ __forceinline__ void abrelu2_n(const ActC& c, P2& q, P2& t, P2 v1, P2 v2, P2 n) {
   const P2 pr = mul2(v1, v2), qq = mul2(q, q);
@@ -379,14 +381,29 @@ __device__ __forceinline__ void abrelu2(const ActC& c, P2& q, P2& t, P2 v1, P2 v
   abrelu2_n<COMP, true>(c, q, t, v1, v2, mul2(sv1, sv2));
 }
 
-template <int COMP = -1>
-__device__ __forceinline__ void abrelu2_v(const ActC& c, P2& q, P2& t, P2 v1, P2 v2) {
-  abrelu2_n<COMP, false>(c, q, t, v1, v2, v1);
-}
-
 // sqrt(var) as every kernel of the library evaluates it (one approximate
 // square root), so that the fused and the materialised paths round alike.
 __device__ __forceinline__ float sqrt_var(float v) { return sqrt_approx(fmaxf(v, 0.f)); }
+
+// abrelu2 from the variances alone, for kernels without root maps. ROOTS false: abrelu2_n's form
+// with one root, for variances that are all one_root_var and an ntk that vanishes with them: the
+// ReLU networks of the fused chain, where the second root is 9 % of the time (60 images through
+// Myrtle-5 in the standard parameterization 9.8 -> 10.8 ms); diagonal-spatial networks take two
+// roots (2 %: 100 x 90 pairs of three layers 298 -> 303 us a call).
+template <int COMP, bool ROOTS>
+__device__ __forceinline__ void abrelu2_v(const ActC& c, P2& q, P2& t, P2 v1, P2 v2) {
+  if (ROOTS) {
+    float a, b, d, e;
+    p2u(v1, a, b);
+    p2u(v2, d, e);
+    abrelu2<COMP>(c, q, t, v1, v2, p2(sqrt_var(a), sqrt_var(b)), p2(sqrt_var(d), sqrt_var(e)));
+  } else {
+    abrelu2_n<COMP, false>(c, q, t, v1, v2, v1);
+  }
+}
+__device__ __forceinline__ bool one_root_var(float v) {
+  return (v >= 0x1p-32f && v <= 0x1p63f) || v == 0.f;
+}
 
 __device__ __forceinline__ void act_apply(const ActC& c, float& q, float& t, float v1, float v2) {
   act_apply<true>(c, q, t, v1, v2, sqrt_var(v1), sqrt_var(v2));

@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kDsThreads)
               }
               if (RELU) {
                 P2 qq = p2(q[0], q[1]), tt = p2(t[0], t[1]);
-                abrelu2_v(ac, qq, tt, p2(v1[0], v1[1]), p2(v2[0], v2[1]));
+                abrelu2_v<-1, true>(ac, qq, tt, p2(v1[0], v1[1]), p2(v2[0], v2[1]));
                 p2u(qq, q[0], q[1]);
                 p2u(tt, t[0], t[1]);
               } else {
