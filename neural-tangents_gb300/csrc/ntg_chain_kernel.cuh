@@ -384,11 +384,13 @@ __device__ __forceinline__ void chain_line(ChainCtx& cx, const ntg_chain_t& pg, 
   };
 
   // planes with every level inside the line, by threes (the period of the (A, B, new) plane
-  // ring, so that its rotation is a renaming of registers); the others one by one, and all in the
-  // ROOTS lines beside RO 1's others, which few pairs take
+  // ring, so that its rotation is a renaming of registers); the others one by one. With more than
+  // the ReLU rule compiled in (RO 0 and 2, always ROOTS) four copies of a step are more code than
+  // the SM's instruction cache holds: 60 images through Myrtle-5 with Erf 19.1 ms so and 14.2 one
+  // by one, Gelu 45.3 and 35.2, Sin 27.4 and 18.7, Myrtle-10 with Erf 44.0 and 26.1.
   int s = lo;
   while (s < hi + NC) {
-    if (S == S0 && (RO != 1 || !ROOTS) && s >= lo + NC && s + 2 < hi) {
+    if (S == S0 && !ROOTS && s >= lo + NC && s + 2 < hi) {
       step(s, std::true_type());
       step(s + 1, std::true_type());
       step(s + 2, std::true_type());
