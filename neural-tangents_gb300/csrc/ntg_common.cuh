@@ -124,9 +124,14 @@ __device__ __forceinline__ float prod_minus_sq(float v1, float v2, float q, int 
   return d;
 }
 
-// One special-function instruction; inputs below 2^-126 count as zero (handling them took
-// three more instructions per root).
 __device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// One special-function instruction, three less: inputs below 2^-126 count as zero.
+__device__ __forceinline__ float sqrt_ftz(float x) {
   float r;
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
@@ -344,10 +349,14 @@ __device__ __forceinline__ void abrelu2_n(const ActC& c, P2& q, P2& t, P2 v1, P2
   p2u(q, q0, q1);
   p2u(n, n0, n1);
   if (!ROOTS) {
-    n0 = sqrt_approx(n0);
-    n1 = sqrt_approx(n1);
+    n0 = sqrt_ftz(n0);
+    n1 = sqrt_ftz(n1);
   }
-  const float s0 = sqrt_approx(fmaxf(d0, 0.f)), s1 = sqrt_approx(fmaxf(d1, 0.f));
+  d0 = fmaxf(d0, 0.f);
+  d1 = fmaxf(d1, 0.f);
+  // with one root, what is below 2^-126 is nothing beside v1 v2
+  const float s0 = ROOTS ? sqrt_approx(d0) : sqrt_ftz(d0);
+  const float s1 = ROOTS ? sqrt_approx(d1) : sqrt_ftz(d1);
   const float den0 = n0 + fabsf(q0), den1 = n1 + fabsf(q1);
   const P2 sp = p2(s0, s1);
   const P2 r = mul2(sp, p2(rcp_approx(den0), rcp_approx(den1)));

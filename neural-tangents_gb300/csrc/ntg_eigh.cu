@@ -63,7 +63,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // back to c^2 + s^2 = 1 by one Newton step, so that thousands of rotations do not drift.
 __device__ __forceinline__ void sym_schur2(float app, float aqq, float apq, float& c, float& s) {
   const float h = 0.5f * (aqq - app);
-  const float r = sqrt_approx(fmaf(h, h, apq * apq));
+  const float r = sqrt_ftz(fmaf(h, h, apq * apq));
   const float t = apq * rcp_approx(h + copysignf(r, h));
   c = rsqrt_approx(fmaf(t, t, 1.f));
   s = t * c;

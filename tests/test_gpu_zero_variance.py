@@ -54,3 +54,31 @@ def test_empty_regions(nt, name, par, b, e1, e2):
     for y in (x2, None):
         for g, w in zip(kf(x1, y, ('nngp', 'ntk')), ko(x1, y, ('nngp', 'ntk'))):
             assert np.max(np.abs(g.cpu().numpy() - w)) <= 1e-5 * np.max(np.abs(w))
+
+
+# powers of two, so that float32 scales the images exactly; networks without a bias are homogeneous
+@pytest.mark.parametrize('e1,e2', [(-12, -12), (-20, -20), (-27, -27), (-30, -30), (-32, -32),
+                                   (-60, 0), (30, 30)])
+@pytest.mark.parametrize('name', ['diagonal', 'band', 'chain5', 'chain1', 'layers'])
+def test_scaled_images(nt, name, e1, e2):
+    """Images far from unit size, against the same network on the unscaled images: one layer's
+    v1 v2 - q^2 keeps 20 bits at 2^-128, the smallest product here (2^-149 is float32's step),
+    and the angle is as good as its root; 1e-5 as for images of unit size. A variance's own
+    covariances, products of 2^-240 at (-60, 0), are float32 zeros where poolings or layer rules
+    take them from a whole per-sample kernel."""
+    if e1 == -60 and name not in ('diagonal', 'chain1'):
+        pytest.skip('the per-sample kernels underflow')
+    shape = {'layers': (6, 6, 2)}.get(name, SHAPES.get(name))
+    if name == 'layers':
+        net = lambda m: [m.Conv(1, (3, 3), padding='SAME', W_std=1.3), m.Relu(),
+                         m.Conv(1, (3, 3), padding='SAME', W_std=1.3), m.Relu(), m.GlobalAvgPool()]
+    else:
+        net = lambda m: _net(m, name, None, 'ntk')
+    x1, x2 = _images(2, shape, 1, None), _images(2, shape, 2, None)
+    kf, ko = nt.stax.serial(*net(nt.stax))[2], o.serial(*net(o))
+    for precision in ('fp32', 'mixed'):
+        got = kf(x1 * np.float32(2.) ** e1, x2 * np.float32(2.) ** e2, ('nngp', 'ntk'),
+                 precision=precision)
+        for g, w in zip(got, ko(x1, x2, ('nngp', 'ntk'))):
+            g = g.cpu().numpy().astype(np.float64) * 2. ** -(e1 + e2)
+            assert np.max(np.abs(g - w)) <= 1e-5 * np.max(np.abs(w))
