@@ -3,25 +3,29 @@
 // transformations of matrix multiplication by using fast routines of matrix multiplication
 // and its applications", Numer. Algorithms 59 (2012)).
 //
-// A row of A + lambda I (a column of X) is scaled by a power of two and written in balanced
-// base-256 digits, |d| <= 128, which bf16 holds exactly: A = 2^(E_i - 7) sum_p 2^-8p a_p with
-// five digits (40 bits below the row's largest entry), X = 2^(F_j - 7) sum_q 2^-8q x_q with six
-// (48 bits). The products a_p x_q with p + q <= 5 are tcgen05.mma kind::f16, those of one level
-// p + q summed in one FP32 accumulator in tensor memory: at most five products of at most 2^14
-// per k, so 192 k stay below 2^24 and every sum is an exact integer. Every 192 k the six
+// The products of the diagonal, (A_ii + lambda) x_i, are taken in FP64: a ridge small beside A_ii
+// keeps its bits. For the others A' = A D and X' = D^-1 X, D = 2^-s with 2^2s near the diagonal,
+// so that rows and columns of different scale weigh alike (|a_ij| <= sqrt(a_ii a_jj)). A row of A'
+// (a column of X') is scaled by a power of two and written in balanced base-256 digits,
+// |d| <= 128, which bf16 holds exactly: A' = 2^(E_i - 7) sum_p 2^-8p a_p, X' likewise with F_j,
+// six digits each (48 bits below the largest entry, so float32 entries down to 2^-23 of it are
+// exact). The products a_p x_q with p + q <= 5 are tcgen05.mma kind::f16, those of one level
+// p + q summed in one FP32 accumulator in tensor memory: at most six products of at most 2^14
+// per k, so 160 k stay below 2^24 and every sum is an exact integer. Every 160 k the six
 // accumulators are drained: levels 0 - 2 into a 64-bit integer per entry, levels 3 - 5, the last
-// 24 of 48 bits, into a float. What is dropped or rounded is near 2^-48 of the largest product:
-// as close to the true residual as the double-float sums (44 bits, 11 FP32 operations a
-// product) that smaller problems take. Fewer digits are not: with four and five (14 products
-// instead of 20) small entries beside large ones cost a solution 1.6e-6 at a condition of 2.5e4.
+// 24 of 48 bits, into a float. What is dropped or rounded is near 2^-48 of the largest entry of
+// the row of A' times that of the column of X': no more than the double-float sums lose (44 bits,
+// 11 FP32 operations a product) that smaller problems take. Fewer digits do: with four and five
+// small entries beside large ones cost a solution 1.6e-6 at a condition of 2.5e4; with five for A,
+// its diagonal among them and no D, scales that span 1e5 cost 1e-6, and kernels that decay to
+// nothing 2e-10 instead of 1e-12 after two steps.
 //
-// One CTA per 128 x 64 tile: TMA brings the eleven digit tiles of 32 k into a 3-stage ring
-// (64 KB a stage), one thread issues the 20 x 2 MMAs of a stage, eight warps drain. Every
+// One CTA per 128 x 64 tile: TMA brings the twelve digit tiles of 32 k into a 3-stage ring
+// (72 KB a stage), one thread issues the 21 x 2 MMAs of a stage, eight warps drain. Every
 // wait is bounded: one that runs out raises the device error word, lets the copies and MMAs
 // in flight land, frees the tensor memory and returns. Bound by the MMAs and the drain that
-// follows each 192 k of them: 4096 x 4096 times 4096 x 4096 takes 3.1 ms (0.88 PFLOP/s of
-// digit products) and 0.3 ms for the digits, against 24.4 ms in double-floats; the whole
-// solve with its gradient goes from 37.3 to 15.8 ms.
+// follows each 160 k of them: 4096 x 4096 times 4096 x 4096 takes 3.4 ms (0.84 PFLOP/s of
+// digit products) and 0.3 ms for the digits, against 24.4 ms in double-floats.
 #include <cuda_bf16.h>
 
 #include <mutex>
@@ -34,8 +38,8 @@ namespace ntg {
 namespace {
 
 constexpr int XM = 128, XN = 64, XK = 32;
-constexpr int PA = 5, PX = 6, LV = 6;   // digits of A, of X; levels
-constexpr int XSTAGES = 3, XCHUNK = 6;  // ring stages; stages per drain (192 k)
+constexpr int PA = 6, PX = 6, LV = 6;   // digits of A, of X; levels
+constexpr int XSTAGES = 3, XCHUNK = 5;  // ring stages; stages per drain (160 k)
 constexpr int XA = XM * XK * 2, XB = XN * XK * 2;  // bytes of a digit tile
 constexpr int XSTAGE = PA * XA + PX * XB;
 constexpr int XSMEM = XSTAGES * XSTAGE + 1024 + 256;
@@ -68,6 +72,21 @@ __device__ __forceinline__ long long fixed_point(double v, int e, int bits) {
   return raw < 0 ? -m : m;
 }
 
+// v = h + l: h its first 24 bits, l the others rounded to 24, from the bits where h and l are
+// normal numbers.
+__device__ __forceinline__ void split_bits(double v, float& h, float& l) {
+  const int hi = __double2hiint(v), ex = (hi >> 20) & 0x7ff;
+  const unsigned lo = __double2loint(v), sign = (unsigned)hi & 0x80000000u;
+  if ((unsigned)(ex - 950) < 200u) {
+    h = __uint_as_float(sign | (unsigned)(ex - 896) << 23 | (unsigned)(hi & 0xfffff) << 3 |
+                        lo >> 29);
+    l = __uint2float_rn(lo & 0x1fffffffu) * __uint_as_float(sign | (unsigned)(ex - 948) << 23);
+  } else {
+    h = (float)v;
+    l = isfinite(h) ? (float)(v - (double)h) : 0.f;
+  }
+}
+
 // Balanced base-256 digits of v, most significant first; |v| <= 2^(8 D - 1).
 template <int D>
 __device__ __forceinline__ void digits_of(long long v, int (&d)[D]) {
@@ -93,27 +112,35 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
       "l"(a), "l"(b), "r"(XIDESC), "r"(acc));
 }
 
-// Digits of rows i0 .. i0 + rows of A + lambda I [n, n] -> as [PA][rows][kpad], exponents
-// rowE[rows] (a row below 2^E). One CTA per row; rows past n and k past n are zero.
+// diag[k] = A_kk + lambda, S[k] = s with 2^2s near it (0 where it is no positive number).
 __global__ void __launch_bounds__(256)
-    digits_rows_kernel(const float* __restrict__ A, const double* __restrict__ lambda, int64_t n,
+    scales_kernel(const float* __restrict__ A, const double* __restrict__ lambda, int64_t n,
+                  double* __restrict__ diag, int* __restrict__ S) {
+  const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (k >= n) return;
+  const double d = (double)__ldg(A + k * n + k) + lambda[0];
+  diag[k] = d;
+  const int e = exponent_of(d);
+  S[k] = d > 0.0 && e != kBad ? e >> 1 : 0;
+}
+
+// Digits of rows i0 .. i0 + rows of A D without its diagonal, A [n, n] -> as [PA][rows][kpad],
+// exponents rowE[rows] (a row below 2^E). One CTA per row; rows past n and k past n are zero.
+__global__ void __launch_bounds__(256)
+    digits_rows_kernel(const float* __restrict__ A, const int* __restrict__ S, int64_t n,
                        int64_t i0, int64_t rows, int64_t kpad, __nv_bfloat16* __restrict__ as,
                        int* __restrict__ rowE) {
   __shared__ int red[8];
   const int64_t at = blockIdx.x, i = i0 + at;
   const float* a = A + i * n;
   int e = kNone;
-  double diag = 0.0;
   if (i < n) {
-    diag = (double)__ldg(a + i) + lambda[0];
-    float mx = 0.f;
-    bool bad = false;
     for (int64_t k = threadIdx.x; k < n; k += 256) {
-      const float v = k == i ? 0.f : fabsf(__ldg(a + k));
-      bad = bad || !isfinite(v);
-      mx = fmaxf(mx, v);
+      const uint32_t v = __float_as_uint(__ldg(a + k)) & 0x7fffffffu;
+      if (k == i || v == 0) continue;
+      // a subnormal counts as the largest
+      e = max(e, v >= 0x7f800000u ? kBad : (int)(v >> 23) - 126 - __ldg(S + k));
     }
-    e = bad ? kBad : max(exponent_of((double)mx), exponent_of(diag));
   }
   e = __reduce_max_sync(0xffffffffu, e);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
@@ -124,10 +151,8 @@ __global__ void __launch_bounds__(256)
   const bool some = e != kBad && e != kNone;
   for (int64_t k = threadIdx.x; k < kpad; k += 256) {
     int d[PA] = {};
-    if (some && k == i) {
-      digits_of<PA>(fixed_point(diag, e, 8 * PA - 1), d);
-    } else if (some && k < n) {
-      float t = scalbnf(__ldg(a + k), 7 - e);
+    if (some && k < n && k != i) {
+      float t = scalbnf(__ldg(a + k), 7 - e - __ldg(S + k));
 #pragma unroll
       for (int p = 0; p < PA; ++p) {
         const float r = rintf(t);
@@ -140,22 +165,24 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// colF[j] = the exponent of column j of X [n, m], preset to kNone.
+// colF[j] = the exponent of column j of D^-1 X, X [n, m], preset to kNone.
 __global__ void __launch_bounds__(256)
-    exponents_kernel(const double* __restrict__ X, int64_t n, int64_t m, int* __restrict__ colF) {
+    exponents_kernel(const double* __restrict__ X, const int* __restrict__ S, int64_t n, int64_t m,
+                     int* __restrict__ colF) {
   const int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (j >= m) return;
   const int64_t k0 = (int64_t)blockIdx.y * 64, k1 = k0 + 64 < n ? k0 + 64 : n;
   int e = kNone;
 #pragma unroll 8
-  for (int64_t k = k0; k < k1; ++k) e = max(e, exponent_of(X[k * m + j]));
-  if (e != kNone) atomicMax(&colF[j], e);
+  for (int64_t k = k0; k < k1; ++k) e = max(e, exponent_of(X[k * m + j]) + __ldg(S + k));
+  // S is far smaller than what kNone and kBad are from an exponent
+  if (e > kNone / 2) atomicMax(&colF[j], e < kBad / 2 ? e : kBad);
 }
 
-// Digits of the columns of X [n, m] -> xs [PX][cols][kpad] (transposed); 32 x 32 blocks.
+// Digits of the columns of D^-1 X, X [n, m] -> xs [PX][cols][kpad] (transposed); 32 x 32 blocks.
 __global__ void __launch_bounds__(256)
-    digits_cols_kernel(const double* __restrict__ X, int64_t n, int64_t m, int64_t cols,
-                       int64_t kpad, const int* __restrict__ colF,
+    digits_cols_kernel(const double* __restrict__ X, const int* __restrict__ S, int64_t n,
+                       int64_t m, int64_t cols, int64_t kpad, const int* __restrict__ colF,
                        __nv_bfloat16* __restrict__ xs) {
   __shared__ long long q[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -164,7 +191,9 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int r = ty; r < 32; r += 8) {
     const int64_t k = k0 + r, j = j0 + tx;
-    q[r][tx] = k < n && f != kNone && f != kBad ? fixed_point(X[k * m + j], f, 8 * PX - 1) : 0;
+    q[r][tx] = k < n && f != kNone && f != kBad
+                   ? fixed_point(X[k * m + j], f - __ldg(S + k), 8 * PX - 1)
+                   : 0;
   }
   __syncthreads();
 #pragma unroll
@@ -183,6 +212,7 @@ struct ExactArgs {
   int64_t k;                     // length of the sums
   int64_t arows, xcols, ni, nj;  // digit rows of a slice, tiles
   const int *rowE, *colF;
+  const double *diag, *X;  // of the band
   const float* B;
   const double* B64;
   float* R;
@@ -345,8 +375,9 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     __syncthreads();
   } else {
     // the products to shared memory as sums of three floats (24 + 24 bits of levels 0 - 2,
-    // levels 3 - 5), then the residuals row by row, coalesced. b and the first float cancel
-    // exactly where they cancel; FP64 would take as long as the products.
+    // levels 3 - 5), then the residuals row by row, coalesced. b less the diagonal's product
+    // and the first float cancel exactly where they cancel. One FP64 operation an entry: six,
+    // with the conversions, took 12 us a tile.
     float* tile = reinterpret_cast<float*>(smem);
     if (warp >= 2) {
       const int row = (warp & 3) * 32 + lane;
@@ -379,14 +410,12 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       if (i >= g.n || j >= g.m) continue;
       const int64_t at = i * g.m + j;
       const float* t = tile + (idx / XN) * XP + idx % XN;
-      float bh, bl = 0.f;
-      if (g.B64) {
-        bh = (float)g.B64[at];
-        bl = (float)(g.B64[at] - (double)bh);
-      } else {
-        bh = g.B[at];
-      }
-      const float r = ((bh - t[0]) + (bl - t[XM * XP])) - t[2 * XM * XP];
+      float dh, dl;
+      split_bits(fma(-__ldg(g.diag + i), __ldg(g.X + at), g.B64 ? g.B64[at] : 0.0), dh, dl);
+      const float b = g.B64 ? 0.f : g.B[at];
+      const float s = __fadd_rn(b, dh), z = __fsub_rn(s, b);
+      const float e = __fadd_rn(__fsub_rn(b, __fsub_rn(s, z)), __fsub_rn(dh, z));  // b + dh - s
+      const float r = ((s - t[0]) + ((e + dl) - t[XM * XP])) - t[2 * XM * XP];
       g.R[at] = r;
       mx = fmaxf(mx, fabsf(r));
     }
@@ -403,13 +432,14 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(XTMEM));
 }
 
-// A's digits, 2.5 times its size, are made for a band of at most 512 MiB of rows at a time (one
-// tile at least; one band up to n = 7296) and X's for all columns: 12 bytes an entry where the
+// A's digits, 3 times its size, are made for a band of at most 512 MiB of rows at a time (one
+// tile at least; one band up to n = 6656) and X's for all columns: 12 bytes an entry where the
 // double-float split takes 8.
 struct ExactWs {
   int64_t kpad, arows, xcols;  // arows: of a band
   __nv_bfloat16 *as, *xs;
-  int *rowE, *colF;
+  int *rowE, *colF, *S;
+  double* diag;
   size_t bytes;
 };
 
@@ -421,13 +451,15 @@ ExactWs exact_ws(void* ws, int64_t n, int64_t m) {
   w.xcols = ceil_div(m, XN) * XN;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t a = up((size_t)PA * w.arows * w.kpad * 2), x = up((size_t)PX * w.xcols * w.kpad * 2);
-  const size_t e = up((size_t)w.arows * 4), f = up((size_t)w.xcols * 4);
+  const size_t e = up((size_t)w.arows * 4), f = up((size_t)w.xcols * 4), d = up((size_t)n * 8);
   char* p = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
   w.as = reinterpret_cast<__nv_bfloat16*>(p);
   w.xs = reinterpret_cast<__nv_bfloat16*>(p + a);
   w.rowE = reinterpret_cast<int*>(p + a + x);
   w.colF = reinterpret_cast<int*>(p + a + x + e);
-  w.bytes = a + x + e + f + 256;
+  w.diag = reinterpret_cast<double*>(p + a + x + e + f);
+  w.S = reinterpret_cast<int*>(p + a + x + e + f + d);
+  w.bytes = a + x + e + f + d + up((size_t)n * 4) + 256;
   return w;
 }
 
@@ -460,23 +492,27 @@ int exact_residual(cudaStream_t s, const float* A, int64_t n, const double* lamb
   const cudaError_t e = cudaFuncSetAttribute(
       exact_residual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, XSMEM);
   if (e != cudaSuccess) return fail(NTG_ERR_CUDA, std::string("exact residual: ") + cudaGetErrorString(e));
+  if (!same_a) {
+    scales_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(A, lambda, n, w.diag, w.S);
+    note_launch();
+  }
   fill_int_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, s>>>(w.colF, m, kNone);
   exponents_kernel<<<dim3((unsigned)ceil_div(m, 256), (unsigned)ceil_div(n, 64)), 256, 0, s>>>(
-      X, n, m, w.colF);
+      X, w.S, n, m, w.colF);
   digits_cols_kernel<<<dim3((unsigned)ceil_div(w.kpad, 32), (unsigned)ceil_div(w.xcols, 32)), 256,
-                       0, s>>>(X, n, m, w.xcols, w.kpad, w.colF, w.xs);
+                       0, s>>>(X, w.S, n, m, w.xcols, w.kpad, w.colF, w.xs);
   note_launch(3);
   for (int64_t i0 = 0; i0 < n; i0 += w.arows) {
     if (!same_a || n > w.arows) {
-      digits_rows_kernel<<<(unsigned)w.arows, 256, 0, s>>>(A, lambda, n, i0, w.arows, w.kpad, w.as,
+      digits_rows_kernel<<<(unsigned)w.arows, 256, 0, s>>>(A, w.S, n, i0, w.arows, w.kpad, w.as,
                                                            w.rowE);
       note_launch();
     }
     const int64_t rows = n - i0 < w.arows ? n - i0 : w.arows;
     const int64_t ni = ceil_div(rows, XM), nj = w.xcols / XN;
-    const ExactArgs g{rows, m, n, w.arows, w.xcols, ni, nj, w.rowE, w.colF,
-                      B ? B + i0 * m : nullptr, B64 ? B64 + i0 * m : nullptr, R + i0 * m, rnorm,
-                      err};
+    const ExactArgs g{rows, m, n, w.arows, w.xcols, ni, nj, w.rowE, w.colF, w.diag + i0,
+                      X + i0 * m, B ? B + i0 * m : nullptr, B64 ? B64 + i0 * m : nullptr,
+                      R + i0 * m, rnorm, err};
     exact_residual_kernel<<<(unsigned)(ni * nj), XTHREADS, XSMEM, s>>>(ma, mx, g);
     note_launch();
   }

@@ -7,9 +7,9 @@
 
 namespace ntg {
 
-// Whether n x n times n x m products are worth the digits, from 2^26 on: there the five
-// launches take 58 us (n 512, m 256) and 85 us (n 1024, m 64) against 158 and 302 us of the
-// double-float kernel, at 2^30 96 - 296 us against 513 - 1330. Below, the digits and the
+// Whether n x n times n x m products are worth the digits, from 2^26 on: there the six
+// launches take 71 us (n 512, m 256) and 103 us (n 1024, m 64) against 158 and 302 us of the
+// double-float kernel, at 2^30 113 - 358 us against 513 - 1330. Below, the digits and the
 // launches take more and more of the time.
 bool exact_residual_pays(int64_t n, int64_t m);
 size_t exact_residual_bytes(int64_t n, int64_t m);

@@ -196,6 +196,35 @@ def test_exact_residual_in_bands(nt):
         assert abs(float(solver.residual) - float(r.abs().max())) < n ** .5 * 2. ** -38 * float(size)
 
 
+@pytest.mark.parametrize('n,m', [(1024, 65), (777, 500), (1500, 130)])
+@pytest.mark.parametrize('kind', ['scales', 'decay'])
+def test_exact_residual_of_wide_ranges(nt, kind, n, m):
+    """Kernels whose samples differ in scale by 1e5, and kernels that decay to nothing: two
+    refinement steps leave what the residual itself loses, 2^-46 of the largest products of the
+    matrix scaled to a unit diagonal (twice 2^-48 for either operand and as much for the sums),
+    times the root of their number and that matrix's condition."""
+    from nt_gb300 import predict
+    g = torch.Generator(device='cuda').manual_seed(n)
+    r = lambda *s: torch.rand(s, generator=g, device='cuda', dtype=torch.float64)
+    if kind == 'scales':
+        x = torch.randn((n, 32), generator=g, device='cuda', dtype=torch.float64)
+        x = x / x.norm(dim=1, keepdim=True)
+        s = torch.exp(r(n, 1) * np.log(1e5))
+        k = ((1. + x @ x.t()) ** 3 / 8 + 1e-2 * torch.eye(n, device='cuda')) * s * s.t()
+    else:
+        x = 30. * r(n, 2)
+        k = torch.exp(-torch.cdist(x, x) ** 2) + 1e-2 * torch.eye(n, device='cuda')
+    k = k.float()
+    b = torch.randn((n, m), generator=g, device='cuda')
+    _, x64 = predict.CholeskySolver(k, 0., True).solve(b, refine_iters=2, want_x64=True)
+    a = k.double()
+    root = a.diagonal().sqrt()[:, None]
+    unit = torch.linalg.eigvalsh(a / root / root.t())
+    want = torch.linalg.solve(a / root / root.t(), b.double() / root)
+    err = float((x64 * root - want).norm() / want.norm())
+    assert err < n ** .5 * 2. ** -46 * float(unit[-1] / unit[0])
+
+
 @pytest.mark.parametrize('n,m', [(1, 17), (127, 17), (128, 130), (129, 40), (257, 17), (390, 300)])
 def test_many_right_hand_sides_at_tile_edges(nt, n, m):
     """Products with the triangular inverses stop at the triangle, tile by tile: kappa <= 5, so
