@@ -405,7 +405,8 @@ _NOT_GAUSSIAN = ('The input to the activation function must be Gaussian, i.e. a 
 def _flat_run(k: Kernel, specs, i: int) -> int:
     """End of the run of Dense / activation layers from specs[i] that _flat_rules takes on k:
     flat kernels, no do_stabilize (it rescales by the pre-activation maximum). An activation
-    right on the scalar-zero NTK of an input kernel stays with _act_rule, which keeps it."""
+    right on the scalar-zero NTK of an input kernel stays with _act_rule, which keeps it, and
+    affine rules on a Kernel without the variances, which they do not read, with _dense_rule."""
     first = next((s.kind for s in specs[i:] if s.kind != 'identity'), None)
     if k.nngp.ndim != 2 or first is None or (first == 'act' and _zero_ntk(k)):
         return i
@@ -413,6 +414,9 @@ def _flat_run(k: Kernel, specs, i: int) -> int:
     while end < len(specs) and (specs[end].kind in ('dense', 'identity') or (
             specs[end].kind == 'act' and not specs[end].params.get('do_stabilize'))):
         end += 1
+    if k.cov1 is None or (k.cov2 is None and k.nngp.shape[1] > k.nngp.shape[0]
+                          and all(s.kind != 'act' for s in specs[i:end])):
+        return i
     return end if any(s.kind != 'identity' for s in specs[i:end]) else i
 
 

@@ -103,3 +103,14 @@ def test_small_products(nt, m, n, k):
     L.call('ntg_gemm_ex', L.stream(), L.ptr(a), L.ptr(b), L.ptr(c), m, n, k, 0, -2., 1)
     assert bool(((c.double() - (1. - 2. * want)).abs() <= 2 * bound + 2. ** -22
                  * (1. + 2. * want.abs())).all())
+
+
+def test_dense_on_kernels_without_variances(nt):
+    s = nt.stax
+    k = s.Identity()[2](_data(5, 12, 8), _data(7, 12, 9))
+    kf = s.serial(s.Dense(1, 1.3, .2), s.Dense(1, 1.1))[2]
+    want = kf(k)
+    for part in (k.replace(cov1=None, cov2=None), k.replace(cov2=None)):
+        got = kf(part)
+        assert torch.equal(got.nngp, want.nngp) and torch.equal(got.ntk, want.ntk)
+        assert got.cov2 is None

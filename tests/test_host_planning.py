@@ -161,3 +161,19 @@ def test_diagonal_requirement_algebra():
             if D is stax.Diagonal:
                 assert c << (b << a) == (c << b) << a == (a >> b) >> c
                 assert (a & b) == (b & a) and (a & b) & c == a & (b & c) and (a & a) == a
+
+
+def test_flat_runs_leave_kernels_without_variances_to_the_layer_rules():
+    """Affine rules read no variances, so a Kernel without them goes through Dense."""
+    from nt_gb300 import stax
+    from nt_gb300.kernel import Kernel
+    k = Kernel(nngp=torch.zeros(2, 3), ntk=None, cov1=torch.zeros(2), cov2=torch.zeros(3),
+               x1_is_x2=False, is_gaussian=True, is_reversed=False, is_input=False,
+               diagonal_batch=True, diagonal_spatial=False, shape1=(2, 4), shape2=(3, 4))
+    dense = stax.serial(stax.Dense(1), stax.Dense(1, 1.2, .1))[2].specs
+    net = stax.serial(stax.Dense(1), stax.Relu())[2].specs
+    assert stax._flat_run(k, dense, 0) == stax._flat_run(k, net, 0) == 2
+    assert stax._flat_run(k.replace(cov1=None), dense, 0) == 0
+    assert stax._flat_run(k.replace(cov2=None), dense, 0) == 0
+    # refused there: the activation reads a variance per row and column
+    assert stax._flat_run(k.replace(cov2=None), net, 0) == 2
