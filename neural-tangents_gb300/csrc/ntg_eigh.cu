@@ -543,10 +543,14 @@ __global__ void refine_e_kernel(const double* __restrict__ S, const double* __re
     if (i != j) {
       // separated: the gap is `sep` times the coupling or more (what a correction leaves over
       // is its square) and above the resolution of the float32 eigenvalues (1e-6 of the
-      // largest); closer pairs are a cluster
+      // largest); closer pairs are a cluster. By the larger of (i, j)'s and (j, i)'s coupling,
+      // so that both are taken alike: half a rotation would leave the pair 1 / sep from
+      // orthogonal.
       const double num = S[idx] + lam[j] * r;
+      const double other = S[j * n + i] + lam[i] * R[j * n + i];
       const double gap = lam[j] - lam[i];
-      if (fabs(gap) > sep * fabs(num) && fabs(gap) > 1e-6 * lam[n]) e = num / gap;
+      if (fabs(gap) > sep * fmax(fabs(num), fabs(other)) && fabs(gap) > 1e-6 * lam[n])
+        e = num / gap;
     }
     E[idx] = (float)e;
   }

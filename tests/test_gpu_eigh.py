@@ -81,3 +81,19 @@ def test_eigh_of_coupled_blocks(nt, n):
         assert np.max(np.abs(a @ v - v * w[None])) / scale < 2e-5
         assert np.max(np.abs(v.T @ v - np.eye(n))) < 2e-5
         assert np.max(np.abs(np.sort(w) - np.linalg.eigvalsh(a.astype(np.float64)))) < 1e-5 * scale
+
+
+@pytest.mark.parametrize('n', [64, 100, 333])
+def test_eigh_of_a_cluster(nt, n):
+    """Half the spectrum at one eigenvalue, half 1e-5 apart: what the refinement cannot separate
+    stays orthogonal; the bounds of test_eigh_matches_float64."""
+    from nt_gb300 import predict
+    g = torch.Generator(device='cuda').manual_seed(n)
+    q = torch.linalg.qr(torch.randn((n, n), generator=g, device='cuda', dtype=torch.float64))[0]
+    e = torch.ones(n, device='cuda', dtype=torch.float64)
+    e[n // 2:] += 1e-5 * torch.arange(n - n // 2, device='cuda')
+    a = ((q * e) @ q.t()).float()
+    evals, evecs = predict._eigh(a, 0.)
+    a, w, v = a.double(), evals.double(), evecs.double()
+    assert float((a @ v - v * w).abs().max()) < 2e-5
+    assert float((v.t() @ v - torch.eye(n, device='cuda')).abs().max()) < 2e-5
