@@ -107,9 +107,8 @@ __device__ __forceinline__ int col_slot(int pos) { return (pos & 1) * (JP / 2) +
 template <bool CROSS>
 __global__ void __launch_bounds__(kInnerThreads)
     jacobi_inner_kernel(const float* __restrict__ A, int64_t lda, int nblk, int round,
-                        int inner_sweeps, float* __restrict__ Uout, const int* done) {
+                        int inner_sweeps, float* __restrict__ Uout) {
   after_previous();
-  if (*done) return;
   __shared__ float ism[2 * JP * JP];  // two copies of S
   __shared__ unsigned s_max;
   constexpr int N = JP * JP;
@@ -275,9 +274,8 @@ __device__ __forceinline__ void mm64(float (&acc)[4][4], const float (*X)[JPV],
 // consecutive rows. Both only wait for the rotations, so one launch takes them.
 __global__ void __launch_bounds__(256)
     jacobi_apply_kernel(float* __restrict__ A, float* __restrict__ V, int64_t ld, int nblk,
-                        int round, const float* __restrict__ Uall, const int* done) {
+                        int round, const float* __restrict__ Uall) {
   after_previous();
-  if (*done) return;
   extern __shared__ __align__(16) float asm_[];
   float(*T)[JPV] = reinterpret_cast<float(*)[JPV]>(asm_);
   float(*Uj)[JPV] = T + JP;
@@ -573,7 +571,6 @@ struct EighWs {
   float* v;
   float* u;
   double* norms;
-  int* done;
 };
 
 EighWs eigh_ws(void* ws, int64_t npad) {
@@ -585,7 +582,6 @@ EighWs eigh_ws(void* ws, int64_t npad) {
   e.u = e.v + npad * npad;
   const int64_t npairs = npad / JP;
   e.norms = reinterpret_cast<double*>(e.u + npairs * JP * JP);
-  e.done = reinterpret_cast<int*>(e.norms + 2);
   return e;
 }
 
@@ -603,7 +599,7 @@ extern "C" size_t ntg_eigh_workspace_bytes(int64_t n) {
   if (n <= 0 || n > 32768) return SIZE_MAX;
   const int64_t npad = (n + JP - 1) / JP * JP;
   return (size_t)(2 * npad * npad + (npad / JP) * JP * JP) * sizeof(float) + 2 * sizeof(double) +
-         sizeof(int) + 512 + refine_bytes(n);
+         512 + refine_bytes(n);
 }
 
 extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, float* evals,
@@ -625,21 +621,19 @@ extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, f
     return check_launch("ntg_eigh");
   eigh_init_kernel<<<egrid(npad * npad), 256, 0, s>>>(A, n, shift, e.w, e.v, npad);
   note_launch();
-  if (cudaMemsetAsync(e.done, 0, sizeof(int), s) != cudaSuccess) return check_launch("ntg_eigh");
   int sweeps = 0;
   double off2 = INFINITY;
   for (int sw = 0; sw < max_sweeps; ++sw) {
     for (int r = 0; r < nblk - 1; ++r) {
       // one inner sweep per pair and round: an inner problem driven further is undone by the
-      // next rounds (n = 500: nine outer sweeps with one inner sweep or two, 7.4 against 12.0
-      // ms). A single pair is the whole matrix: to convergence.
-      // The couplings inside a block are rotated in the first round of a sweep only, which pairs
-      // every block once: the same ten sweeps to convergence at half the rotations, 8.0 -> 4.9
-      // ms for the predictions of 500 points, with the launches overlapped.
+      // next rounds. A single pair is the whole matrix: to convergence. The couplings inside a
+      // block are rotated in the first round of a sweep only, which pairs every block once.
+      // n = 500, eigenpairs alone: 4.5 ms in ten sweeps, which an inner sweep over all couplings
+      // in each round, or two, needs as well.
       launch_next(s, r == 0 ? jacobi_inner_kernel<false> : jacobi_inner_kernel<true>, dim3(npairs),
-                  kInnerThreads, e.w, npad, nblk, r, npairs == 1 ? 8 : 1, e.u, e.done);
+                  kInnerThreads, e.w, npad, nblk, r, npairs == 1 ? 8 : 1, e.u);
       launch_next_smem(s, jacobi_apply_kernel, dim3(npairs, (unsigned)(npairs + npad / JP)), 256,
-                       kApplySmem, e.w, e.v, npad, nblk, r, e.u, e.done);
+                       kApplySmem, e.w, e.v, npad, nblk, r, e.u);
     }
     ++sweeps;
     if (cudaMemsetAsync(e.norms, 0, 2 * sizeof(double), s) != cudaSuccess)
@@ -659,7 +653,7 @@ extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, f
   note_launch();
   if (refine_steps > 0) {
     char* rp = reinterpret_cast<char*>(
-        (reinterpret_cast<uintptr_t>(e.done + 1) + 255) & ~(uintptr_t)255);
+        (reinterpret_cast<uintptr_t>(e.norms + 2) + 255) & ~(uintptr_t)255);
     double* S = reinterpret_cast<double*>(rp);
     double* R = S + n * n;
     double* lam = R + n * n;
