@@ -73,6 +73,10 @@ __device__ __forceinline__ void sym_schur2(float app, float aqq, float apq, floa
 }
 
 constexpr int kInnerThreads = 512;
+// Shared memory that a CTA of the inner kernel asks for beyond its own 32 KB: half an SM's, so that
+// two of them never share one. They are placed while the launch before drains, onto whichever SMs
+// come free, and two on an SM take turns: 15 to 34 us a round, as it happened (n = 1500).
+constexpr size_t kInnerAlone = 84 * 1024;
 
 // The tournament as a fixed permutation of positions (Brent & Luk): pair k sits at positions
 // 2k, 2k + 1; after a round the player at position i moves to round_move(i), position 0 stays,
@@ -616,8 +620,10 @@ extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, f
   const int nblk = (int)(npad / JB);  // even
   const int npairs = nblk / 2;
   const EighWs e = eigh_ws(workspace, npad);
-  if (cudaFuncSetAttribute(jacobi_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kApplySmem) != cudaSuccess)
+  const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if (cudaFuncSetAttribute(jacobi_apply_kernel, smem, (int)kApplySmem) != cudaSuccess ||
+      cudaFuncSetAttribute(jacobi_inner_kernel<false>, smem, (int)kInnerAlone) != cudaSuccess ||
+      cudaFuncSetAttribute(jacobi_inner_kernel<true>, smem, (int)kInnerAlone) != cudaSuccess)
     return check_launch("ntg_eigh");
   eigh_init_kernel<<<egrid(npad * npad), 256, 0, s>>>(A, n, shift, e.w, e.v, npad);
   note_launch();
@@ -630,8 +636,9 @@ extern "C" int ntg_eigh(void* stream, const float* A, int64_t n, double shift, f
       // block are rotated in the first round of a sweep only, which pairs every block once.
       // n = 500, eigenpairs alone: 4.5 ms in ten sweeps, which an inner sweep over all couplings
       // in each round, or two, needs as well.
-      launch_next(s, r == 0 ? jacobi_inner_kernel<false> : jacobi_inner_kernel<true>, dim3(npairs),
-                  kInnerThreads, e.w, npad, nblk, r, npairs == 1 ? 8 : 1, e.u);
+      launch_next_smem(s, r == 0 ? jacobi_inner_kernel<false> : jacobi_inner_kernel<true>,
+                       dim3(npairs), kInnerThreads, kInnerAlone, e.w, npad, nblk, r,
+                       npairs == 1 ? 8 : 1, e.u);
       launch_next_smem(s, jacobi_apply_kernel, dim3(npairs, (unsigned)(npairs + npad / JP)), 256,
                        kApplySmem, e.w, e.v, npad, nblk, r, e.u);
     }
