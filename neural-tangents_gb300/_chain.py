@@ -17,6 +17,7 @@ layer-by-layer path.
 from __future__ import annotations
 
 import dataclasses
+import math
 from typing import Optional
 
 import torch
@@ -232,10 +233,21 @@ DS_MAX_SMEM = 100 * 1024  # two CTAs per SM; larger images go layer by layer
 # from 1 to 256 pairs of 8 x 8 to 32 x 32 images, against 1.1 - 2.9 ms by the layer rules or the
 # whole-kernel chain; 225 (three poolings): 1.3 - 1.9 ms against 1.3 - 1.4 ms up to 32 pairs.
 BAND_MAX_PLANES = 49
+# Many pairs of small images fill the GPU either way. A plane then takes the band 4 - 6 ns
+# whatever its size, an entry of a whole pair the layer rules 14 - 58 ps, and a call by these no
+# less than 0.8 ms. So the band is for pairs of 128 entries a plane, or for as many planes as it
+# takes in that time. 10^4 pairs, two 2 x 2 poolings, band and layer rules: 4 x 4 images 3.1 and
+# 0.9 ms, 8 x 8 3.2 and 2.4, 12 x 12 3.4 and 5.6; one pooling: 4 x 4 0.54 and 0.83, 8 x 8 0.54
+# and 2.4. Past 2^29 entries, 8 GB in the layer rules' tensors, it is the band again, which holds
+# none of them.
+BAND_ENTRIES_PER_PLANE = 128
+BAND_SMALL_CALL = 1 << 17
+BAND_LARGE_CALL = 1 << 29
 
 
-def _narrow_band(specs, size) -> bool:
-    """Whether the poolings leave a Flatten no more than BAND_MAX_PLANES offsets to see."""
+def _narrow_band(specs, size, pairs: int) -> bool:
+    """Whether the poolings leave a Flatten no more than BAND_MAX_PLANES offsets to see, and few
+    enough for `pairs` pairs of images of that size."""
     d = [0] * len(size)
     pools = [s.params for s in specs if s.kind == 'pool']
     for p in reversed(pools):
@@ -245,22 +257,27 @@ def _narrow_band(specs, size) -> bool:
     planes = 1
     for x, m in zip(d, size):
         planes *= 2 * min(x, m - 1) + 1
-    return bool(pools) and planes <= BAND_MAX_PLANES
+    if not pools or planes > BAND_MAX_PLANES:
+        return False
+    entries = math.prod(size) ** 2
+    return (BAND_ENTRIES_PER_PLANE * planes <= entries or pairs * planes <= BAND_SMALL_CALL
+            or pairs * entries > BAND_LARGE_CALL)
 
 
-def plan_ds(specs, x_shape, ctx: _Ctx, pools: bool = False):
+def plan_ds(specs, x_shape, ctx: _Ctx, pools: bool = False, pairs: int = 1):
     """(program, layers after the readout, is_gaussian) of a serial network whose layers up to a
     Flatten / GlobalAvgPool / GlobalSumPool readout are stride-1 zero-padded Conv, Dense and
     activations, on [N, A, K] or [N, A, C, K] inputs; None for another network. pools: a network
     with AvgPool / SumPool layers among these, their windows inside the maps, and a Flatten
-    readout, which sees a band around the spatial diagonal."""
+    readout, which sees a band around the spatial diagonal; pairs: of the call."""
     if len(x_shape) not in (3, 4):
         return None
     specs = [s for s in specs if s.kind != 'identity']
     ridx = next((i for i, s in enumerate(specs) if s.kind in ('gpool', 'flatten')), None)
     if not ridx or ridx > 3 * L.DS_MAX_LAYERS or specs[0].kind == 'act':
         return None
-    if pools and (specs[ridx].kind != 'flatten' or not _narrow_band(specs[:ridx], x_shape[1:-1])):
+    if pools and (specs[ridx].kind != 'flatten' or not _narrow_band(
+            specs[:ridx], x_shape[1:-1], pairs)):
         return None
     a, c = x_shape[1], x_shape[2] if len(x_shape) == 4 else 1
     pg = L.DsChain()
@@ -341,7 +358,9 @@ def try_ds(kfn, x1: torch.Tensor, x2: Optional[torch.Tensor], compute_ntk: bool,
     around them; whole: see try_fused."""
     if x2 is not None and x2.shape[1:] != x1.shape[1:]:
         return None
-    plan = plan_ds(kfn.specs, tuple(x1.shape), ctx, pools)
+    n = x1.shape[0]
+    pairs = n * (n + 1) // 2 if x2 is None else n * x2.shape[0]
+    plan = plan_ds(kfn.specs, tuple(x1.shape), ctx, pools, pairs)
     if plan is None:
         return None
     pg, spatial, post, gaussian = plan

@@ -177,3 +177,22 @@ def test_flat_runs_leave_kernels_without_variances_to_the_layer_rules():
     assert stax._flat_run(k.replace(cov2=None), dense, 0) == 0
     # refused there: the activation reads a variance per row and column
     assert stax._flat_run(k.replace(cov2=None), net, 0) == 2
+
+
+def test_bands_of_many_small_pairs_go_layer_by_layer():
+    """128 entries of a pair's kernel per plane of its band, or a call of at most 2^17 planes or
+    of more entries than the layer rules should hold."""
+    from nt_gb300 import _chain, stax
+    conv = lambda: stax.Conv(1, (3, 3), padding='SAME')
+    pool = lambda: stax.AvgPool((2, 2), (2, 2))
+    one = stax.serial(conv(), stax.Relu(), pool(), stax.Flatten())[2].specs              # 9 planes
+    two = stax.serial(conv(), stax.Relu(), pool(), conv(), pool(), stax.Flatten())[2].specs  # 49
+    ctx = stax._Ctx('fp32')
+    band = lambda specs, size, pairs: _chain.plan_ds(specs, (2, size, size, 1), ctx, True,
+                                                     pairs) is not None
+    for specs, planes, size in ((one, 9, 4), (two, 49, 4), (two, 49, 8)):
+        assert band(specs, size, 1) and band(specs, size, (1 << 17) // planes)
+        assert not band(specs, size, (1 << 17) // planes + 1)
+        assert not band(specs, size, (1 << 29) // size ** 4)
+        assert band(specs, size, (1 << 29) // size ** 4 + 1)
+    assert band(one, 6, 10 ** 6) and band(two, 12, 10 ** 6) and band(two, 28, 10 ** 6)
