@@ -73,8 +73,11 @@ __global__ void __launch_bounds__(256) gemm_nn_kernel(const float* __restrict__ 
 // One CTA per (b, a) row. A thread keeps its (c, c') for all planes a', so that an entry costs
 // its products, one store and no index arithmetic: bound by the stores (456 pairs of 28 x 28
 // images and the 43 samples with themselves, 1.2 GB: 383 us; 1490 with the indices taken apart
-// by 64-bit divisions for every entry).
+// by 64-bit divisions for every entry). Planes of fewer than 64 entries (SMALL; 1-D inputs: one)
+// would leave that most threads idle: entry by entry over the planes instead, as long as a row's
+// fit 32 bits (4 x 4 pairs of 1000 positions 83 us against 887).
 // ---------------------------------------------------------------------------
+template <bool SMALL>
 __global__ void __launch_bounds__(256)
     input_fs_kernel(const float* __restrict__ x1, const float* __restrict__ x2, int64_t batch,
                     int64_t n2, int64_t A, int C, int64_t K, float inv_k,
@@ -87,6 +90,18 @@ __global__ void __launch_bounds__(256)
   const float* img2 = x2 + i2 * A * C * K;
   const int64_t plane = (int64_t)C * C;
   float* o = out + (b * A + a) * A * plane;
+  if (SMALL) {
+    const uint32_t P = (uint32_t)plane, n = (uint32_t)A * P;
+    for (uint32_t e = threadIdx.x; e < n; e += 256) {
+      const uint32_t ap = e / P, r = e - ap * P, c = r / (uint32_t)C;
+      const float* p1 = r1 + c * K;
+      const float* y = img2 + ((int64_t)ap * C + (r - c * C)) * K;
+      float s = 0.f;
+      for (int64_t k = 0; k < K; ++k) s = fmaf(__ldg(p1 + k), __ldg(y + k), s);
+      o[e] = s * inv_k;
+    }
+    return;
+  }
   for (int64_t e = threadIdx.x; e < plane; e += 256) {
     const int64_t c = plane <= INT_MAX ? (int)e / C : e / C;
     const float* p1 = r1 + c * K;
@@ -1787,8 +1802,9 @@ extern "C" int ntg_input_fs(void* stream, const float* x1, const float* x2, int6
     input_fs_vec_kernel<<<(unsigned)blocks, 256, vec_sm, as_stream(stream)>>>(
         x1, xb, batch, pairs ? n2 : 0, (int)a, (int)c, (int)k, 1.f / (float)k, out);
   } else {
-    input_fs_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
-        x1, xb, batch, pairs ? n2 : 0, a, (int)c, k, 1.f / (float)k, out);
+    auto kernel = c < 8 && a * c * c < (1ll << 31) ? input_fs_kernel<true> : input_fs_kernel<false>;
+    kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(x1, xb, batch, pairs ? n2 : 0, a, (int)c,
+                                                            k, 1.f / (float)k, out);
   }
   note_launch();
   return check_launch("ntg_input_fs");

@@ -247,3 +247,19 @@ def test_full_spatial_networks_of_any_size(nt, shape, filt):
     for b in (x2, None):
         for got, want in zip(kf(x1, b, ('nngp', 'ntk')), ko(x1, b, ('nngp', 'ntk'))):
             assert np.max(np.abs(got.cpu().numpy() - want)) < 1e-5 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize('a,c,k', [(1, 1, 1), (300, 1, 3), (257, 1, 64), (40, 2, 4), (33, 5, 5),
+                                   (19, 7, 3), (12, 8, 1), (9, 13, 65)])
+def test_input_covariances_of_narrow_maps(nt, a, c, k):
+    """Either side of the rule at eight columns, one CTA's 256 threads and four channels: a chain of
+    k products and the division against float64."""
+    from nt_gb300 import _ops as O
+    g = torch.Generator(device='cuda').manual_seed(a + k)
+    x, y = (torch.randn((n, a, c, k), generator=g, device='cuda') for n in (2, 3))
+    for got, u, v, eq in ((O.input_fs(x, y), x, y, 'nacd,mbed->nmabce'),
+                          (O.input_fs(x, None), x, x, 'nacd,nbed->nabce')):
+        u, v = u.double(), v.double()
+        want = torch.einsum(eq, u, v) / k
+        bound = (k + 2) * 2. ** -24 * torch.einsum(eq, u.abs(), v.abs()) / k
+        assert bool(((got.double().reshape(want.shape) - want).abs() <= bound).all())
