@@ -65,7 +65,7 @@ BYTES_PER_ENTRY = (10 * 32 ** 4 + 8 * 16 ** 4 + 8 * 8 ** 4) * 4
 FLOPS_PER_ELEM_LAYER = 4 * 2 + 4 * 2 + 4 + 40
 # Warp instructions one pair costs in the Myrtle-5 fused kernel: smsp__inst_executed.sum of
 # chain_fwd_kernel<2, 3, 1, 1, 1, 0, 3> over a 32 x 32 tile (ncu), divided by its 1024 pairs.
-WARP_INSTR_PER_PAIR = 2.70e6
+WARP_INSTR_PER_PAIR = 2.76e6
 # Instruction issue peak: 152 SMs x 4 warp schedulers, one instruction per cycle each.
 ISSUE_SLOTS_PER_CYCLE = 152 * 4
 

@@ -222,9 +222,10 @@ def check_device(where: str) -> None:
     """Raises NtgError when a bounded wait of a device kernel ran out since the last check.
 
     The streamed, adjoint and tensor-core kernels bound every pipeline wait; one that runs
-    out sets a device error word and the kernel winds down with its results incomplete.
+    out sets the device's error word and the kernel winds down with its results incomplete.
     The current stream is synchronised first, so that every kernel it carries has finished,
-    then ntg_device_status reads and clears the words (one 4-byte read per word)."""
+    then ntg_device_status waits for the legacy stream and reads and clears the word, which is
+    in host memory mapped into the device."""
     if not torch.cuda.is_available():
         return  # nothing of this library can have run
     torch.cuda.current_stream().synchronize()
@@ -237,7 +238,7 @@ def check_device(where: str) -> None:
 @contextlib.contextmanager
 def boundary(where: str):
     """A public call of the package: on its normal exit, and only at the outermost level
-    (calls nest, e.g. nt.batch calls kernel_fn per tile), the device error words are
+    (calls nest, e.g. nt.batch calls kernel_fn per tile), the device error word is
     checked with check_device."""
     d = getattr(_depth, 'n', 0)
     _depth.n = d + 1

@@ -228,13 +228,15 @@ def _assemble(rows, names, single):
 
 
 class CapturedBatch:
-    """``batch(kernel_fn, batch_size)(x1, x2, get)`` for fixed input shapes, captured
+    """``batch(kernel_fn)(x1, x2, get)`` for fixed input shapes, captured
     once as a CUDA graph and replayed: for serving, where the same shapes come back
     and the host-side work of a call (per-sample chains, launches, allocations)
     would otherwise be repeated. Only networks on the fused chain path (whose
     forward has no host synchronisation) can be captured. A call copies the inputs
     into the graph's static buffers, replays, and returns the graph's static
     output tensors, which the next call overwrites (clone them to keep them).
+    ``batch_size`` has no effect (the whole grid is one launch, whose working set does not
+    grow with it); it is taken for the signature of ``batch``.
     Not in the reference (XLA compiles, it does not capture)."""
 
     def __init__(self, kernel_fn, x1_shape, x2_shape=None, get=('nngp', 'ntk'),

@@ -24,8 +24,8 @@
 // lines (64 KB) in L2, where nothing waits for them (red.add, read one plane
 // ahead), and no square roots of the variances. K(x, x) of 120 images through Myrtle-5
 // (7260 pairs): 41.0 ms with one CTA of 512 threads, two columns a thread and the pooled
-// lines in shared memory (4.56 M warp instructions a pair, 65 % of the issue slots), 24.8 ms
-// so (2.68 M, 64 %). Three CTAs an SM (80 registers, spills): 27.1 ms; the layers of a step
+// lines in shared memory (4.56 M warp instructions a pair, 65 % of the issue slots), 25.1 ms
+// so (2.7 M, 64 %). Three CTAs an SM (80 registers, spills): 27.1 ms; the layers of a step
 // made independent of one another (each on the plane of the step before, 128 registers):
 // 27.0 ms.
 #pragma once

@@ -8,10 +8,11 @@
 // memory, so that one 8-byte access and one packed add serve both in the window sums, which
 // run along the columns, then along the rows; a thread owns two neighbouring columns, so that
 // the activation rule runs on packed pairs. The variances (elementwise on the diagonal) come
-// from the same code on every sample with itself, in a launch before. Bound by issue (70 % of
-// the slots; FP32 and shared memory about even): 100 x 90 pairs of 32 x 32 x 3 images through
-// three 3 x 3 convs take 144 us (194 us with the window sizes read at run time), against 815
-// us in 27 launches for the layer rules, which move every layer's tensors through HBM.
+// from the same code on every sample with itself, in a launch before. Bound by issue (76 % of
+// the active slots; FP32 and shared memory about even): 100 x 90 pairs of 32 x 32 x 3 images
+// through three 3 x 3 convs take 158 us (a third more with the window sizes read at run time),
+// against 815 us in 27 launches for the layer rules, which move every layer's tensors through
+// HBM.
 //
 // A network with poolings before its Flatten needs more than the diagonal, but not the whole
 // (a c)^2 kernel: an entry of the readout sees the offsets (h' - h, w' - w) within k - 1 of the
@@ -20,7 +21,7 @@
 // most a x c entries, so the kernel walks the planes of the band one after another, the
 // diagonal first (it gives a sample's variances), and adds each into the pooled planes of the
 // next level in shared memory. One 2 x 2 pooling behind two convs on 28 x 28 images: 9 planes,
-// 456 pairs in 54 us and the 43 samples' variances in 34 (a serial walk, few CTAs), against 5.8
+// 456 pairs in 57 us and the 43 samples' variances in 36 (a serial walk, few CTAs), against 5.8
 // ms in 28 launches for the layer rules on 28^4 entries a pair.
 #include <string>
 

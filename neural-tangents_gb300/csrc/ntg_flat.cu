@@ -523,7 +523,9 @@ __global__ void __launch_bounds__(256)
 bool gemm_small(cudaStream_t s, const float* a, const float* b, float* c, int64_t m, int64_t n,
                 int64_t k, bool trans_a, float alpha, bool accumulate) {
   // below one 64 x 64 tile per SM: the eigenvectors of 500 points times 60 columns take 16 us
-  // (57 us on eight 64 x 64 tiles)
+  // (57 us on eight 64 x 64 tiles); whole calls on 64 x 64 tiles and here, plain and with A
+  // transposed: 200^3 38, 48 and 28, 27 us, 500^3 64, 85 and 43, 44, 640^3 77, 104 and 61, 62,
+  // 768^3 (144 tiles) 86, 121 and 81, 82, 768 x 768 x 4096 368, 554 and 334, 347
   if (ceil_div(m, 64) * ceil_div(n, 64) >= 152 || ceil_div(m, 32) > 65535) return false;
   const dim3 grid((unsigned)ceil_div(n, 32), (unsigned)ceil_div(m, 32));
   if (trans_a)
@@ -543,7 +545,9 @@ int gram_fp32(cudaStream_t s, const float* x1, const float* x2, int64_t n1, int6
     return sym ? a * (a + 1) / 2 : a * b;
   };
   // The largest tile that still gives every SM one: a tile costs the same whatever else
-  // runs, and a smaller one reads more of its operands per output.
+  // runs, and a smaller one reads more of its operands per output. Calls on 128-wide tiles and
+  // on the ones taken here: 300^2 x 784 120 and 32 us, 700^2 121 and 53 (32 wide), 1000^2 121 and
+  // 73, 1200 x 1100 x 3072 417 and 305 (64 wide); at 1500^2 (144 tiles of 128) 122 and 120.
   if (tiles(128) >= 152) {
     const float inv = 1.f / (float)d;
     const int64_t nb1 = ceil_div(n1, 128);
